@@ -30,15 +30,16 @@ def build_port():
 
 def reference_root():
     """Where the reference's sources are: $FSPH_REFERENCE, else a checkout
-    named `reference` beside this repository; None when neither exists."""
+    named `reference` beside this repository; None when neither holds them
+    (an empty folder counts as absent)."""
     cand = os.environ.get("FSPH_REFERENCE") or os.path.join(
         os.path.dirname(os.path.dirname(HERE)), "reference")
-    return cand if os.path.isdir(cand) else None
+    return cand if os.path.isdir(os.path.join(cand, "include", "physics")) else None
 
 
 def build_ref(ref_root=None):
     ref_root = ref_root or reference_root()
-    if not ref_root or not os.path.isdir(ref_root):
+    if not ref_root or not os.path.isdir(os.path.join(ref_root, "include", "physics")):
         return False
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={ref_root}"], check=True)
     return True
