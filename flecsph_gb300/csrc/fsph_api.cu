@@ -256,6 +256,13 @@ bool params_supported(const fsph_params * p, std::string * why) {
   return true;
 }
 
+// positions, velocities, thermodynamics or h changed: no derived record of
+// the state is current any more
+void records_stale(fsph_ctx * c) {
+  c->ahyd_ok = c->fv_ok = c->fdv_ok = c->vel_ok = false;
+  c->prho2_ok = c->pair64_ok = false;
+}
+
 fsph_status set_device(fsph_ctx * c) {
   CK(cudaSetDevice(c->device));
   return FSPH_OK;
@@ -525,9 +532,24 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   ok &= dalloc(c, &c->d_time, 1) == cudaSuccess;
   ok &= dalloc(c, &c->d_status, 1) == cudaSuccess;
   ok &= dalloc(c, &c->d_cons, 8 * (1 + CONS_BLOCKS)) == cudaSuccess;
+  if(!c->mixed)
+    ok &= dalloc(c, &c->prho2, N) == cudaSuccess;
   if(!ok) {
     cudaGetLastError();
     return fail(FSPH_ERR_OOM);
+  }
+  if(!c->mixed) {
+    // The pair terms (16 B per list slot) only save the energy passes a second
+    // evaluation: taken where they leave at least three quarters of the free
+    // memory to everything else (4 KB a particle at the default capacity)
+    const size_t slots = Npad * (size_t)c->Ls.maxnb;
+    size_t mfree = 0, mtotal = 0;
+    if(cudaMemGetInfo(&mfree, &mtotal) == cudaSuccess &&
+       slots <= mfree / 4 / sizeof(double2) &&
+       dalloc(c, &c->pair64, slots) != cudaSuccess) {
+      c->pair64 = nullptr;
+      cudaGetLastError();
+    }
   }
   if(cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess)
     return fail(FSPH_ERR_CUDA);
@@ -574,8 +596,7 @@ static fsph_status upload_impl(fsph_ctx * c, const fsph_soa_view * v,
   if(!c || !v || v->n < 2 || v->n > c->cap || !v->x || !v->y ||
      (c->p.dimension == 3 && !v->z) || !v->m || !v->h || !v->id)
     return FSPH_ERR_ARG;
-  c->ahyd_ok = false;
-  c->fv_ok = c->fdv_ok = c->vel_ok = false;
+  records_stale(c);
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -635,8 +656,7 @@ static fsph_status upload_fields_impl(fsph_ctx * c, const fsph_soa_view * v,
   cudaMemcpyKind kind) {
   if(!c || !v || !c->uploaded || v->n != c->n)
     return FSPH_ERR_ARG;
-  c->ahyd_ok = false;
-  c->fv_ok = c->fdv_ok = c->vel_ok = false;
+  records_stale(c);
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -813,8 +833,7 @@ static bool wendland(int k);
 fsph_status fsph_update_iteration(fsph_ctx * c) {
   if(!c || !c->uploaded)
     return FSPH_ERR_STATE;
-  c->ahyd_ok = false;
-  c->fv_ok = c->fdv_ok = c->vel_ok = false;
+  records_stale(c);
   c->grav_nodes_ok = false;
   fsph_status s = set_device(c);
   if(s)
@@ -905,7 +924,7 @@ fsph_status fsph_compute_alpha(fsph_ctx * c) {
     c->last_error = "compute_alpha needs sph_viscosity = visc_cullen";
     return FSPH_ERR_STATE;
   }
-  c->ahyd_ok = false;
+  c->ahyd_ok = c->pair64_ok = false;
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -921,7 +940,7 @@ fsph_status fsph_compute_alpha(fsph_ctx * c) {
 static fsph_status density_impl(fsph_ctx * c, bool with_vsig) {
   if(!c || !c->tree_ok)
     return FSPH_ERR_STATE;
-  c->ahyd_ok = false;
+  c->ahyd_ok = c->pair64_ok = c->prho2_ok = false;
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -940,10 +959,14 @@ static fsph_status density_impl(fsph_ctx * c, bool with_vsig) {
   else {
     {
       Phase ph(c, FSPH_TIMER_DENSITY);
-      CK(launch_density_fp64(L, c->P, c->pp, c->Ls, c->cs_new, c->d_status, c->d_time));
+      CK(launch_density_fp64(L, c->P, c->pp, c->Ls, c->cs_new, c->prho2, c->d_status,
+        c->d_time));
+      c->prho2_ok = true;
     }
-    Phase ph(c, FSPH_TIMER_VSIG);
-    CK(launch_vsig_fp64(L, c->P, c->pp, c->Ls, c->cs_new));
+    if(with_vsig) {
+      Phase ph(c, FSPH_TIMER_VSIG);
+      CK(launch_vsig_fp64(L, c->P, c->pp, c->Ls, c->cs_new));
+    }
   }
   // the new sound speed becomes the particle's sound speed
   double * t = c->P.f[F_CS];
@@ -965,6 +988,17 @@ static bool wendland(int k) {
          k == FSPH_KERNEL_WENDLAND_C6;
 }
 
+// FP64 path: P / rho^2 as the state has it now
+static fsph_status prho2_current(fsph_ctx * c) {
+  if(!c->prho2_ok)
+    CK(launch_prho2(c->L(), c->P, c->prho2));
+  c->prho2_ok = true;
+  return FSPH_OK;
+}
+
+// fused_vsig: the signal speed rides in the pass (the FP64 one reads the
+// previous sound speed from cs_new, where the density pass left it, and takes
+// v_half for v: the caller says they are equal)
 static fsph_status accel_impl(fsph_ctx * c, int kick, int fused_vsig = 0) {
   if(!c || !c->tree_ok)
     return FSPH_ERR_STATE;
@@ -976,8 +1010,14 @@ static fsph_status accel_impl(fsph_ctx * c, int kick, int fused_vsig = 0) {
   if(c->mixed)
     CK(launch_accel_mixed(L, c->P, c->pp, c->Ls, c->K, kick, c->d_time, fused_vsig,
       c->fv_ok ? 1 : 0));
-  else
-    CK(launch_accel_fp64(L, c->P, c->pp, c->Ls, kick, c->d_time));
+  else {
+    fsph_status ps = prho2_current(c);
+    if(ps)
+      return ps;
+    CK(launch_accel_fp64(L, c->P, c->pp, c->Ls, kick, c->d_time, c->prho2,
+      fused_vsig ? c->cs_new : nullptr, c->pair64));
+    c->pair64_ok = c->pair64 != nullptr;
+  }
   // the float-float pass (Wendland kernels) leaves the pressure-only
   // acceleration in K.ahyd for the de/dt pass, and with the kick the
   // {v - v_half, m} records of the kicked velocities
@@ -1000,8 +1040,13 @@ fsph_status fsph_dudt(fsph_ctx * c) {
   if(c->mixed)
     CK(launch_dudt_mixed(L, c->P, c->pp, c->Ls, c->K, c->d_time, 0, c->fv_ok ? 1 : 0,
       c->fdv_ok ? 1 : 0));
-  else
-    CK(launch_dudt_fp64(L, c->P, c->pp, c->Ls, c->d_time));
+  else {
+    fsph_status ps = prho2_current(c);
+    if(ps)
+      return ps;
+    CK(launch_dudt_fp64(L, c->P, c->pp, c->Ls, c->d_time, c->prho2,
+      c->pair64_ok ? c->pair64 : nullptr));
+  }
   return FSPH_OK;
 }
 
@@ -1016,8 +1061,13 @@ fsph_status fsph_dedt(fsph_ctx * c) {
   if(c->mixed)
     CK(launch_dedt_mixed(L, c->P, c->pp, c->Ls, c->K, 0, c->d_time, c->d_status,
       c->ahyd_ok ? 1 : 0, c->fdv_ok ? 1 : 0));
-  else
-    CK(launch_dedt_fp64(L, c->P, c->pp, c->Ls));
+  else {
+    fsph_status ps = prho2_current(c);
+    if(ps)
+      return ps;
+    CK(launch_dedt_fp64(L, c->P, c->pp, c->Ls, c->prho2,
+      c->pair64_ok ? c->pair64 : nullptr));
+  }
   return FSPH_OK;
 }
 
@@ -1082,7 +1132,7 @@ static fsph_status elem(fsph_ctx * c, int op, int phase) {
   if(op != OP_KICK_V && op != OP_KICK_E && op != OP_KICK_U &&
      op != OP_SET_TOTAL_ENERGY && op != OP_DRAG_ACC && op != OP_DRAG_DEDT &&
      op != OP_DRAG_DUDT && op != OP_CHECK_NANS && op != OP_CHECK_NEGATIVITY)
-    c->ahyd_ok = c->fv_ok = c->fdv_ok = c->vel_ok = false;
+    records_stale(c);
   if(op == OP_KICK_V)
     c->fdv_ok = c->vel_ok = false;
   fsph_status s = set_device(c);
@@ -1440,12 +1490,12 @@ fsph_status fsph_step(fsph_ctx * c) {
       TRY(fsph_set_total_energy(c));
     if(cullen)
       TRY(fsph_initialize_alpha(c));
-    // mixed: the signal speed rides in the acceleration loop
-    TRY(density_impl(c, !c->mixed));
+    // the signal speed rides in the acceleration loop
+    TRY(density_impl(c, false));
     TRY(fsph_save_velocityhalf(c));
     if(cullen)
       TRY(fsph_compute_alpha(c));
-    TRY(accel_impl(c, 0, c->mixed));
+    TRY(accel_impl(c, 0, 1));
     if(relax) {
       TRY(fsph_add_drag_acceleration(c));
       TRY(fsph_add_short_range_repulsion(c));
@@ -1503,25 +1553,25 @@ fsph_status fsph_step(fsph_ctx * c) {
     c->permute_skip = 0;
     TRY(us);
     TRY(io_stage(c, IO_UPDATE));
-    TRY(density_impl(c, !c->mixed));
+    TRY(density_impl(c, false));
     if(cullen)
       TRY(fsph_compute_alpha(c));
     TRY(io_stage(c, IO_DENSITY));
     if(grav) {
       // newtonian/main_driver.cc:217-227: gravity between the hydro
       // acceleration and the velocity kick
-      TRY(accel_impl(c, 0, c->mixed));
+      TRY(accel_impl(c, 0, 1));
       TRY(fsph_gravitation(c));
       TRY(fsph_leapfrog_kick_v(c));
     }
     else if(relax) {
-      TRY(accel_impl(c, 0, c->mixed));
+      TRY(accel_impl(c, 0, 1));
       TRY(fsph_add_drag_acceleration(c));
       TRY(fsph_add_short_range_repulsion(c));
       TRY(fsph_leapfrog_kick_v(c));
     }
     else
-      TRY(accel_impl(c, 1, c->mixed));
+      TRY(accel_impl(c, 1, 1));
     TRY(io_stage(c, IO_ACCEL));
     if(evolve) {
       for(int m = 1; m <= p.pressure_updates_number; ++m) {

@@ -66,6 +66,14 @@ struct fsph_ctx {
   // K.vel holds v and c_s of the current state (written by the permute of
   // update_iteration on the mixed path)
   bool vel_ok = false;
+  // FP64 path: P / rho^2 per particle (written by the density pass; prho2_ok
+  // while P and rho are unchanged since) and the pair terms the acceleration
+  // pass leaves for the energy passes (pair64_ok while positions, h, v_half,
+  // rho, c_s and alpha are; pair64 is null where memory is short)
+  double * prho2 = nullptr;
+  double2 * pair64 = nullptr;
+  bool prho2_ok = false;
+  bool pair64_ok = false;
   bool uploaded = false;
   long long launches = 0;
   // timers

@@ -8,18 +8,33 @@
 // where libm and CUDA's pow/cbrt differ in the last bit.
 #include <cuda_runtime.h>
 
+#include "fsph_pair64.cuh"
 #include "fsph_sphmath.cuh"
 
 namespace fsph {
 
-#define PAIR_THREADS 256
+// Blocks of 64: the passes are bound by the FP64 pipe (two FMAs a clock and
+// SM), which two warps already fill, so what counts is an even share of warps
+// per SM.  Blocks of 256 left 121 of 152 SMs idle at 8k particles and a third
+// of the last wave at 91k.
+#define PAIR_THREADS 64
+
+// The loops below read a list's slots four at a time; the slots past its end
+// hold the particle itself, at distance zero.
+__device__ __forceinline__ int slot4(const int4 & q, int u) {
+  return u == 0 ? q.x : u == 1 ? q.y : u == 2 ? q.z : q.w;
+}
 
 // compute_density + recover_internal_energy + eos (default_physics.h:193-228,
-// 126-145, 309-316).  The new sound speed goes to cs_new: the signal speed
-// pass still needs the old one (see k_vsig).
-template<int D, int K>
+// 126-145, 309-316), and with visc_cullen compute_divv (:273-299) from the same
+// traversal.  The new sound speed goes to cs_new: the signal speed still needs
+// the old one (see k_vsig).  prho2 receives P / rho^2, which every pair of the
+// force and energy passes reads of its neighbour (a division per particle
+// instead of one per pair).
+template<int D, int K, bool CULL>
 __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
-  PhysParams pp, Lists Ls, double * cs_new, DevStatus * st, const DevTime * tm) {
+  PhysParams pp, Lists Ls, double * cs_new, double * prho2, DevStatus * st,
+  const DevTime * tm) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -30,22 +45,40 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
   const double * M = P.f[F_M];
   const double pa0 = X[a], pa1 = Y[a], pa2 = D == 3 ? Z[a] : 0.0;
   const double h_a = H[a];
+  double va[3] = {0.0, 0.0, 0.0};
+  if(CULL)
+    for(int d = 0; d < D; ++d)
+      va[d] = P.f[F_VX + d][a];
   const int cnt = Ls.cnt[a];
-  double rho_a = 0.0;
-  for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-    double r = 0;
-    double d0 = pa0 - X[b];
-    r += d0 * d0;
-    double d1 = pa1 - Y[b];
-    r += d1 * d1;
-    if(D == 3) {
-      double d2 = pa2 - Z[b];
-      r += d2 * d2;
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  double rho_a = 0.0, div_v = 0.0;
+  PairH<D, K> ph;
+  ph.init();
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int b = slot4(q4, u);
+      const double d0 = pa0 - X[b], d1 = pa1 - Y[b];
+      double r2 = d0 * d0 + d1 * d1, d2 = 0.0;
+      if(D == 3) {
+        d2 = pa2 - Z[b];
+        r2 += d2 * d2;
+      }
+      const PairR r = pair_r(r2);
+      ph.template set<true, CULL>(h_a, H[b], pp);
+      const double mb = M[b];
+      const double w = mb * pair_w<D, K>(r.r, ph, pp);
+      if(j0 + u < cnt)
+        rho_a += w;
+      if(CULL) {
+        const double f = pair_g<D, K>(r, ph, pp);
+        double dot = va[0] * (d0 * f) + va[1] * (d1 * f);
+        if(D == 3)
+          dot += va[2] * (d2 * f);
+        div_v += mb * dot;  // the padding slots' terms are zero
+      }
     }
-    r = sqrt(r);
-    double Wab = kfun<D, K>(r, .5 * (h_a + H[b]), pp);
-    rho_a += M[b] * Wab;
   }
   if(!(rho_a > 0))
     raise_status(st, FSPH_ERR_NEG_DENSITY, a);
@@ -68,26 +101,22 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
     cs);
   P.f[F_P][a] = Pa;
   cs_new[a] = cs;
-  if(pp.cullen) {
-    // compute_divv (default_physics.h:273-299), same traversal
-    double va[3] = {P.f[F_VX][a], P.f[F_VY][a], D == 3 ? P.f[F_VZ][a] : 0.0};
-    double pa[3] = {pa0, pa1, pa2};
-    double div_v = 0.0;
-    for(int j = 0; j < cnt; ++j) {
-      const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-      double pos_ab[3] = {pa[0] - X[b], pa[1] - Y[b], D == 3 ? pa[2] - Z[b] : 0.0};
-      const double h_ab = .5 * (h_a + H[b]);
-      double DiWab[3];
-      kgrad<D, K>(pos_ab, h_ab, DiWab, pp);
-      double dot = 0.0;
-      for(int d = 0; d < D; ++d)
-        dot += va[d] * DiWab[d];
-      div_v += M[b] * dot;
-    }
+  prho2[a] = Pa / (rho_a * rho_a);
+  if(CULL) {
     div_v /= rho_a;
     const double div_v_p = P.f[F_DIVV][a];
     P.f[F_DDIVVDT][a] = (div_v - div_v_p) / tm->dt;
     P.f[F_DIVV][a] = div_v;
+  }
+}
+
+// P / rho^2 of every particle where the density pass's is out of date (a
+// caller changed P or rho in between).
+__global__ void __launch_bounds__(256) k_prho2(Particles P, double * prho2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i < P.n) {
+    const double rho = P.f[F_RHO][i];
+    prho2[i] = P.f[F_P][i] / (rho * rho);
   }
 }
 
@@ -122,36 +151,38 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_alpha_cullen(Particles P,
   double gradV[D * D];
   for(int k = 0; k < D * D; ++k)
     gradV[k] = 0.0;
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  PairH<D, K> ph;
+  ph.init();
   for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
+    const int b = lp[slot_off(j)];
     const double pb[3] = {X[b], Y[b], D == 3 ? Z[b] : 0.0};
     double pos_ab[3] = {0, 0, 0}, vab[3] = {0, 0, 0};
-    double dist = 0.0;
+    double dist2 = 0.0;
     for(int d = 0; d < D; ++d) {
       pos_ab[d] = pa[d] - pb[d];
       vab[d] = va[d] - V[d][b];
-      dist += pos_ab[d] * pos_ab[d];
+      dist2 += pos_ab[d] * pos_ab[d];
     }
-    dist = sqrt(dist);
+    const PairR r = pair_r(dist2);
     // vsig = max(vsig, max(c_a, c_b) - min(v_ab . n_ab, 0)); the self pair
     // (0/0) is a NaN that std::max drops
-    double vn = 0.0;
-    for(int d = 0; d < D; ++d)
-      vn += vab[d] * (pos_ab[d] / dist);
-    const double cmax = c_a < CS[b] ? CS[b] : c_a;
-    const double mn = 0.0 < vn ? 0.0 : vn;   // std::min(vn, 0.0)
-    const double cand = cmax - mn;
-    vsig = vsig < cand ? cand : vsig;        // std::max(vsig, cand)
-    const double h_ab = .5 * (h_a + H[b]);
-    double DiWa[3];
-    kgrad<D, K>(pos_ab, h_ab, DiWa, pp);
-    const double Wab = kfun<D, K>(dist, h_ab, pp);
+    if(nonzero(dist2)) {
+      const double cmax = c_a < CS[b] ? CS[b] : c_a;
+      const double cand = cmax - approach<D>(vab, pos_ab, r);
+      vsig = vsig < cand ? cand : vsig;      // std::max(vsig, cand)
+    }
+    ph.template set<true, true>(h_a, H[b], pp);
+    const double f = pair_g<D, K>(r, ph, pp);
+    const double Wab = pair_w<D, K>(r.r, ph, pp);
     const double dvb = DV[b];
     const double sgn = dvb > 0.0 ? 1.0 : (dvb < 0.0 ? -1.0 : dvb);
     R_a += sgn * M[b] * Wab;
-    for(int i = 0; i < D; ++i)
-      for(int k = 0; k < D; ++k)
-        gradV[D * i + k] += M[b] * (-vab[i]) * DiWa[k];
+    for(int k = 0; k < D; ++k) {
+      const double DiW = pos_ab[k] * f;
+      for(int i = 0; i < D; ++i)
+        gradV[D * i + k] += M[b] * (-vab[i]) * DiW;
+    }
   }
   R_a /= rho_a;
   for(int k = 0; k < D * D; ++k)
@@ -208,26 +239,22 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_vsig(Particles P, Lists Ls,
   const double pa0 = X[a], pa1 = Y[a], pa2 = D == 3 ? Z[a] : 0.0;
   const double va0 = VX[a], va1 = VY[a], va2 = D == 3 ? VZ[a] : 0.0;
   const double c_a = cs_new[a];
+  const double va[3] = {va0, va1, va2};
   const int cnt = Ls.cnt[a];
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
   double vsig = 0.0;
   for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-    double q0 = pa0 - X[b], q1 = pa1 - Y[b], q2 = D == 3 ? pa2 - Z[b] : 0.0;
-    double dist = 0;
-    dist += q0 * q0;
-    dist += q1 * q1;
+    const int b = lp[slot_off(j)];
+    const double x[3] = {pa0 - X[b], pa1 - Y[b], D == 3 ? pa2 - Z[b] : 0.0};
+    double dist2 = x[0] * x[0] + x[1] * x[1];
     if(D == 3)
-      dist += q2 * q2;
-    dist = sqrt(dist);
-    double dotv = 0;
-    dotv += (va0 - VX[b]) * (q0 / dist);
-    dotv += (va1 - VY[b]) * (q1 / dist);
-    if(D == 3)
-      dotv += (va2 - VZ[b]) * (q2 / dist);
+      dist2 += x[2] * x[2];
+    if(!nonzero(dist2))
+      continue;  // the self pair's 0/0 drops out of the reference's maximum
+    double v[3] = {va[0] - VX[b], va[1] - VY[b], D == 3 ? va[2] - VZ[b] : 0.0};
     const double c_b = b >= a ? cs_new[b] : CS[b];
     const double cab = c_a < c_b ? c_b : c_a;
-    const double mn = 0.0 < dotv ? 0.0 : dotv;
-    const double cand = cab - mn;
+    const double cand = cab - approach<D>(v, x, pair_r(dist2));
     vsig = vsig < cand ? cand : vsig;
   }
   P.f[F_VSIG][a] = vsig;
@@ -236,9 +263,25 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_vsig(Particles P, Lists Ls,
 // compute_acceleration (default_physics.h:348-408); optionally followed by
 // leapfrog_kick_v (integration.h:65-70) for the same particle: the pass
 // reads only v_half of neighbours, never v.
-template<int D, int K>
+//
+// With VSIG the signal speed of k_vsig rides along: the caller says that v
+// equals v_half everywhere (true in a driver iteration, where both are saved
+// together), so the pair's velocity difference, distance and its reciprocal
+// are at hand; cs_old is the sound speed before the density pass.
+//
+// The pass leaves {grad W factor, Pi} of every pair in `pair` (16 bytes, slot
+// j of particle a at [a >> 5][j][a & 31]) for the energy pass, which needs the
+// same two values: read back from HBM they cost a fraction of the ~60 FP64
+// operations that recompute them.
+//
+// Bound by the FP64 pipe.  Per pair of a uniform-h run 3D: ~60 operations, and
+// ~35 more in the branch of approaching pairs, which holds what only the
+// viscosity needs (its two divisions among them); recomputing every division
+// per pair (six and a root) took 130 and more.
+template<int D, int K, bool VSIG>
 __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
-  PhysParams pp, Lists Ls, int kick, const DevTime * tm) {
+  PhysParams pp, Lists Ls, int kick, const DevTime * tm, const double * prho2,
+  const double * cs_old, double2 * pair) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -248,39 +291,63 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   const double * H = P.f[F_H];
   const double * M = P.f[F_M];
   const double * RHO = P.f[F_RHO];
-  const double * PR = P.f[F_P];
   const double * CS = P.f[F_CS];
   const double * VH[3] = {P.f[F_VHX], P.f[F_VHY], P.f[F_VHZ]};
-  const double h_a = H[a], rho_a = RHO[a], P_a = PR[a], c_a = CS[a];
+  const double h_a = H[a], rho_a = RHO[a], c_a = CS[a];
   double pa[3] = {X[a], Y[a], D == 3 ? Z[a] : 0.0};
   double v12a[3];
   for(int d = 0; d < D; ++d)
     v12a[d] = VH[d][a];
-  const double Prho2_a = P_a / (rho_a * rho_a);
+  const double Prho2_a = prho2[a];
   double acc[3] = {0, 0, 0};
+  double vsig = 0.0;
   const int cnt = Ls.cnt[a];
-  for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-    double xb[3] = {X[b], Y[b], D == 3 ? Z[b] : 0.0};
-    double pos_ab[3], v12_ab[3], DiWa[3];
-    bool same = true;
-    for(int d = 0; d < D; ++d) {
-      same = same && (xb[d] == pa[d]);
-      pos_ab[d] = pa[d] - xb[d];
-      v12_ab[d] = v12a[d] - VH[d][b];
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  double2 * pw = pair ? pair + pair_slot(a, 0, Ls.maxnb) : nullptr;
+  PairH<D, K> ph;
+  ph.init();
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int b = slot4(q4, u);
+      double pos_ab[3] = {0, 0, 0}, v12_ab[3] = {0, 0, 0};
+      pos_ab[0] = pa[0] - X[b];
+      pos_ab[1] = pa[1] - Y[b];
+      double dist2 = pos_ab[0] * pos_ab[0] + pos_ab[1] * pos_ab[1];
+      if(D == 3) {
+        pos_ab[2] = pa[2] - Z[b];
+        dist2 += pos_ab[2] * pos_ab[2];
+      }
+      for(int d = 0; d < D; ++d)
+        v12_ab[d] = v12a[d] - VH[d][b];
+      double dotp = v12_ab[0] * pos_ab[0] + v12_ab[1] * pos_ab[1];
+      if(D == 3)
+        dotp += v12_ab[2] * pos_ab[2];
+      ph.template set<false, true>(h_a, H[b], pp);
+      const PairR r = pair_r(dist2);
+      const double f = pair_g<D, K>(r, ph, pp);
+      // mu and Pi are zero unless the pair approaches (viscosity.h:81-93)
+      double Pi = 0.0, appr = 0.0;
+      if(dotp < 0.0) {
+        Pi = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + RHO[b]),
+          .5 * (c_a + CS[b]), ph.h, dotp, dist2);
+        if(VSIG)
+          appr = approach<D>(v12_ab, pos_ab, r);
+      }
+      if(VSIG && nonzero(dist2)) {
+        const double c_b = b >= a ? CS[b] : cs_old[b];
+        const double cand = (c_a < c_b ? c_b : c_a) - appr;
+        vsig = vsig < cand ? cand : vsig;
+      }
+      // the self pair, coincident pairs and padding slots have x_ab = 0 and
+      // f = 0: their terms vanish, as the reference's m_b = 0 makes them
+      const double s = -M[b] * (Prho2_a + prho2[b] + Pi);
+      for(int d = 0; d < D; ++d)
+        acc[d] += pos_ab[d] * f * s;
+      if(pw)
+        pw[(size_t)(j0 + u) * 32] = make_double2(f, Pi);
     }
-    const double rho_b = RHO[b];
-    const double m_b = M[b] * (!same);
-    const double h_ab = .5 * (h_a + H[b]);
-    const double mu_ab = visc_mu<D>(pp.eps, h_ab, v12_ab, pos_ab);
-    const double rho_ab = .5 * (rho_a + rho_b);
-    const double c_ab = .5 * (c_a + CS[b]);
-    const double Pi = visc_pi_pp(pp, P.f[F_ALPHA], a, b, rho_ab, c_ab, mu_ab);
-    kgrad<D, K>(pos_ab, h_ab, DiWa, pp);
-    const double Prho2_b = PR[b] / (rho_b * rho_b);
-    const double s = -m_b * (Prho2_a + Prho2_b + Pi);
-    for(int d = 0; d < D; ++d)
-      acc[d] += DiWa[d] * s;
   }
   // acc_a += external_force::acceleration(particle) (:404)
   double ext[3] = {0.0, 0.0, 0.0};
@@ -295,12 +362,37 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
       P.f[F_VX + d][a] = P.f[F_VX + d][a] + (ad + 0.0) * half_dt;
   }
   P.f[F_GPOT][a] = 0.0;
+  if(VSIG)
+    P.f[F_VSIG][a] = vsig;
 }
 
-// compute_dudt (default_physics.h:421-487)
-template<int D, int K>
+// The gradient factor and Pi of one pair: read from the acceleration pass's
+// `pair` (KEPT) or evaluated.
+template<int D, int K, bool KEPT>
+__device__ __forceinline__ double2 pair_terms(const Particles & P, const PhysParams & pp,
+  PairH<D, K> & ph, const double2 * pr, int j, int a, int b, const double * pos_ab,
+  const double * v12a, double h_a, double rho_a, double c_a) {
+  if(KEPT)
+    return pr[(size_t)j * 32];
+  double dist2 = 0.0, dotp = 0.0;
+  for(int d = 0; d < D; ++d) {
+    dist2 += pos_ab[d] * pos_ab[d];
+    dotp += (v12a[d] - P.f[F_VHX + d][b]) * pos_ab[d];
+  }
+  ph.template set<false, true>(h_a, P.f[F_H][b], pp);
+  double2 t = make_double2(pair_g<D, K>(pair_r(dist2), ph, pp), 0.0);
+  if(dotp < 0.0)
+    t.y = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + P.f[F_RHO][b]),
+      .5 * (c_a + P.f[F_CS][b]), ph.h, dotp, dist2);
+  return t;
+}
+
+// compute_dudt (default_physics.h:421-487).  KEPT: the pair terms of the
+// acceleration pass are still those of the state.
+template<int D, int K, bool KEPT>
 __global__ void __launch_bounds__(PAIR_THREADS) k_dudt(Particles P,
-  PhysParams pp, Lists Ls, const DevTime * tm) {
+  PhysParams pp, Lists Ls, const DevTime * tm, const double * prho2,
+  const double2 * pair) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -309,169 +401,154 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_dudt(Particles P,
     P.f[F_DUDT][a] = 0.0;
     return;
   }
-  const double * X = P.f[F_X];
-  const double * Y = P.f[F_Y];
-  const double * Z = P.f[F_Z];
-  const double * H = P.f[F_H];
-  const double * M = P.f[F_M];
-  const double * RHO = P.f[F_RHO];
-  const double * PR = P.f[F_P];
-  const double * CS = P.f[F_CS];
-  const double * V[3] = {P.f[F_VX], P.f[F_VY], P.f[F_VZ]};
-  const double * VH[3] = {P.f[F_VHX], P.f[F_VHY], P.f[F_VHZ]};
-  const double h_a = H[a], rho_a = RHO[a], P_a = PR[a], c_a = CS[a];
-  double pa[3] = {X[a], Y[a], D == 3 ? Z[a] : 0.0};
-  double va[3], v12a[3];
+  const double h_a = P.f[F_H][a], rho_a = P.f[F_RHO][a], c_a = P.f[F_CS][a];
+  double pa[3] = {0, 0, 0}, va[3] = {0, 0, 0}, v12a[3] = {0, 0, 0};
   for(int d = 0; d < D; ++d) {
-    va[d] = V[d][a];
-    v12a[d] = VH[d][a];
+    pa[d] = P.f[F_X + d][a];
+    va[d] = P.f[F_VX + d][a];
+    v12a[d] = P.f[F_VHX + d][a];
   }
   double dp = 0.0, dv = 0.0;
   const int cnt = Ls.cnt[a];
-  for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-    double xb[3] = {X[b], Y[b], D == 3 ? Z[b] : 0.0};
-    double pos_ab[3], v12_ab[3], vel_ab[3], DiWab[3];
-    bool same = true;
-    for(int d = 0; d < D; ++d) {
-      same = same && (xb[d] == pa[d]);
-      pos_ab[d] = pa[d] - xb[d];
-      v12_ab[d] = v12a[d] - VH[d][b];
-      vel_ab[d] = va[d] - V[d][b];
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  const double2 * pr = KEPT ? pair + pair_slot(a, 0, Ls.maxnb) : nullptr;
+  PairH<D, K> ph;
+  ph.init();
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int b = slot4(q4, u);
+      double pos_ab[3] = {0, 0, 0};
+      for(int d = 0; d < D; ++d)
+        pos_ab[d] = pa[d] - P.f[F_X + d][b];
+      const double2 t = pair_terms<D, K, KEPT>(P, pp, ph, pr, j0 + u, a, b, pos_ab, v12a,
+        h_a, rho_a, c_a);
+      double vdw = 0;
+      for(int d = 0; d < D; ++d)
+        vdw += (va[d] - P.f[F_VX + d][b]) * (pos_ab[d] * t.x);
+      const double mvdw = P.f[F_M][b] * vdw;
+      dp += mvdw;
+      dv += mvdw * t.y;
     }
-    const double m_b = M[b] * (!same);
-    const double h_ab = .5 * (h_a + H[b]);
-    const double mu_ab = visc_mu<D>(pp.eps, h_ab, v12_ab, pos_ab);
-    const double rho_ab = .5 * (rho_a + RHO[b]);
-    const double c_ab = .5 * (c_a + CS[b]);
-    const double Pi = visc_pi_pp(pp, P.f[F_ALPHA], a, b, rho_ab, c_ab, mu_ab);
-    kgrad<D, K>(pos_ab, h_ab, DiWab, pp);
-    double vdw = 0;
-    for(int d = 0; d < D; ++d)
-      vdw += vel_ab[d] * DiWab[d];
-    dp += m_b * vdw;
-    dv += m_b * vdw * Pi;
   }
-  P.f[F_DUDT][a] = P_a / (rho_a * rho_a) * dp + .5 * dv;
+  P.f[F_DUDT][a] = prho2[a] * dp + .5 * dv;
 }
 
-// compute_dedt (default_physics.h:502-566)
-template<int D, int K>
+// compute_dedt (default_physics.h:502-566).  KEPT: as in k_dudt.
+template<int D, int K, bool KEPT>
 __global__ void __launch_bounds__(PAIR_THREADS) k_dedt(Particles P,
-  PhysParams pp, Lists Ls) {
+  PhysParams pp, Lists Ls, const double * prho2, const double2 * pair) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
-  const double * X = P.f[F_X];
-  const double * Y = P.f[F_Y];
-  const double * Z = P.f[F_Z];
-  const double * H = P.f[F_H];
-  const double * M = P.f[F_M];
-  const double * RHO = P.f[F_RHO];
-  const double * PR = P.f[F_P];
-  const double * CS = P.f[F_CS];
-  const double * V[3] = {P.f[F_VX], P.f[F_VY], P.f[F_VZ]};
-  const double * VH[3] = {P.f[F_VHX], P.f[F_VHY], P.f[F_VHZ]};
-  const double h_a = H[a], rho_a = RHO[a], P_a = PR[a], c_a = CS[a];
-  double pa[3] = {X[a], Y[a], D == 3 ? Z[a] : 0.0};
-  double va[3], v12a[3];
+  const double h_a = P.f[F_H][a], rho_a = P.f[F_RHO][a], c_a = P.f[F_CS][a];
+  double pa[3] = {0, 0, 0}, va[3] = {0, 0, 0}, v12a[3] = {0, 0, 0};
   double gv = 0;
   for(int d = 0; d < D; ++d) {
-    va[d] = V[d][a];
-    v12a[d] = VH[d][a];
+    pa[d] = P.f[F_X + d][a];
+    va[d] = P.f[F_VX + d][a];
+    v12a[d] = P.f[F_VHX + d][a];
     gv += P.f[F_GAX + d][a] * va[d];
   }
-  const double Prho2_a = P_a / (rho_a * rho_a);
+  const double Prho2_a = prho2[a];
   double dedt = 0;
   const int cnt = Ls.cnt[a];
-  for(int j = 0; j < cnt; ++j) {
-    const int b = Ls.idx[list_slot(a, j, Ls.maxnb)];
-    double xb[3] = {X[b], Y[b], D == 3 ? Z[b] : 0.0};
-    double pos_ab[3], v12_ab[3], DiWab[3], vb[3];
-    bool same = true;
-    for(int d = 0; d < D; ++d) {
-      same = same && (xb[d] == pa[d]);
-      pos_ab[d] = pa[d] - xb[d];
-      v12_ab[d] = v12a[d] - VH[d][b];
-      vb[d] = V[d][b];
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  const double2 * pr = KEPT ? pair + pair_slot(a, 0, Ls.maxnb) : nullptr;
+  PairH<D, K> ph;
+  ph.init();
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+    for(int u = 0; u < 4; ++u) {
+      const int b = slot4(q4, u);
+      double pos_ab[3] = {0, 0, 0};
+      for(int d = 0; d < D; ++d)
+        pos_ab[d] = pa[d] - P.f[F_X + d][b];
+      const double2 t = pair_terms<D, K, KEPT>(P, pp, ph, pr, j0 + u, a, b, pos_ab, v12a,
+        h_a, rho_a, c_a);
+      double vad = 0, vbd = 0;
+      for(int d = 0; d < D; ++d) {
+        const double DiW = pos_ab[d] * t.x;
+        vad += va[d] * DiW;
+        vbd += P.f[F_VX + d][b] * DiW;
+      }
+      dedt -= P.f[F_M][b] * (Prho2_a * vbd + vad * prho2[b] + .5 * t.y * (vbd + vad));
     }
-    const double rho_b = RHO[b];
-    const double m_b = M[b] * (!same);
-    const double h_ab = .5 * (h_a + H[b]);
-    const double mu_ab = visc_mu<D>(pp.eps, h_ab, v12_ab, pos_ab);
-    const double rho_ab = .5 * (rho_a + rho_b);
-    const double c_ab = .5 * (c_a + CS[b]);
-    const double Pi = visc_pi_pp(pp, P.f[F_ALPHA], a, b, rho_ab, c_ab, mu_ab);
-    kgrad<D, K>(pos_ab, h_ab, DiWab, pp);
-    double vad = 0, vbd = 0;
-    for(int d = 0; d < D; ++d)
-      vad += va[d] * DiWab[d];
-    for(int d = 0; d < D; ++d)
-      vbd += vb[d] * DiWab[d];
-    const double Prho2_b = PR[b] / (rho_b * rho_b);
-    dedt -= m_b * (Prho2_a * vbd + vad * Prho2_b + .5 * Pi * (vbd + vad));
   }
   dedt += gv;
   P.f[F_DEDT][a] = dedt;
 }
 
 // ------------------------------------------------------------ dispatch --
-#define DISPATCH_DK(KERNEL_T, ...)                                             \
+#define DISPATCH_DK(KERNEL_T, TA, ...)                                             \
   do {                                                                         \
     const int nb_ = (P.n + PAIR_THREADS - 1) / PAIR_THREADS;                   \
     if(pp.dim == 3) {                                                          \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<3, FSPH_KERNEL_SINC><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SINC TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     else {                                                                     \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<2, FSPH_KERNEL_SINC><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SINC TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     *L.counter += 1;                                                           \
   } while(0)
 
+#define TARG(X) , X
+
 cudaError_t launch_density_fp64(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, double * cs_new, DevStatus * st,
-  const DevTime * t) {
-  DISPATCH_DK(k_density, P, pp, Ls, cs_new, st, t);
+  const PhysParams & pp, const Lists & Ls, double * cs_new, double * prho2,
+  DevStatus * st, const DevTime * t) {
+  if(pp.cullen)
+    DISPATCH_DK(k_density, TARG(true), P, pp, Ls, cs_new, prho2, st, t);
+  else
+    DISPATCH_DK(k_density, TARG(false), P, pp, Ls, cs_new, prho2, st, t);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prho2(const Launch & L, const Particles & P, double * prho2) {
+  k_prho2<<<(P.n + 255) / 256, 256, 0, L.stream>>>(P, prho2);
+  *L.counter += 1;
   return cudaGetLastError();
 }
 
 cudaError_t launch_alpha_cullen(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const DevTime * t) {
-  DISPATCH_DK(k_alpha_cullen, P, pp, Ls, t);
+  DISPATCH_DK(k_alpha_cullen, , P, pp, Ls, t);
   return cudaGetLastError();
 }
 
@@ -540,20 +617,32 @@ cudaError_t launch_vsig_fp64(const Launch & L, const Particles & P,
 }
 
 cudaError_t launch_accel_fp64(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, int kick, const DevTime * t) {
-  DISPATCH_DK(k_accel, P, pp, Ls, kick, t);
+  const PhysParams & pp, const Lists & Ls, int kick, const DevTime * t,
+  const double * prho2, const double * cs_old, double2 * pair) {
+  if(cs_old)
+    DISPATCH_DK(k_accel, TARG(true), P, pp, Ls, kick, t, prho2, cs_old, pair);
+  else
+    DISPATCH_DK(k_accel, TARG(false), P, pp, Ls, kick, t, prho2, cs_old, pair);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dudt_fp64(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const DevTime * t) {
-  DISPATCH_DK(k_dudt, P, pp, Ls, t);
+  const PhysParams & pp, const Lists & Ls, const DevTime * t, const double * prho2,
+  const double2 * pair) {
+  if(pair)
+    DISPATCH_DK(k_dudt, TARG(true), P, pp, Ls, t, prho2, pair);
+  else
+    DISPATCH_DK(k_dudt, TARG(false), P, pp, Ls, t, prho2, pair);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dedt_fp64(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls) {
-  DISPATCH_DK(k_dedt, P, pp, Ls);
+  const PhysParams & pp, const Lists & Ls, const double * prho2,
+  const double2 * pair) {
+  if(pair)
+    DISPATCH_DK(k_dedt, TARG(true), P, pp, Ls, prho2, pair);
+  else
+    DISPATCH_DK(k_dedt, TARG(false), P, pp, Ls, prho2, pair);
   return cudaGetLastError();
 }
 

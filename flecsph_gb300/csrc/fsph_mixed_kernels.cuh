@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "fsph_internal.cuh"
+#include "fsph_pair64.cuh"   // FP64 pair terms of the velocity divergence
 #include "fsph_sphmath.cuh"  // the FP64 EOS the density pass applies
 #include "fsph_ff.cuh"
 
@@ -265,6 +266,8 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
   float sum = 0.f, comp = 0.f;
   double gsum[3] = {0.0, 0.0, 0.0};
   double pa[3] = {0.0, 0.0, 0.0}, h_a = 0.0;
+  PairH<D, K> ph;
+  ph.init();
   if(CULL) {
     for(int d = 0; d < D; ++d)
       pa[d] = P.f[F_X + d][a];
@@ -286,13 +289,15 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
       kahan(sum, comp, j0 + u < cnt ? w : 0.f);
       if(CULL) {
         // padding slots and the self pair have x_ab = 0 and add nothing
-        double pos_ab[3] = {0.0, 0.0, 0.0}, DiW[3];
-        for(int d = 0; d < D; ++d)
+        double pos_ab[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
+        for(int d = 0; d < D; ++d) {
           pos_ab[d] = pa[d] - P.f[F_X + d][b];
-        kgrad<D, K>(pos_ab, .5 * (h_a + P.f[F_H][b]), DiW, pp);
-        const double mbd = P.f[F_M][b];
+          r2 += pos_ab[d] * pos_ab[d];
+        }
+        ph.template set<false, true>(h_a, P.f[F_H][b], pp);
+        const double mf = P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
         for(int d = 0; d < D; ++d)
-          gsum[d] += mbd * DiW[d];
+          gsum[d] += mf * pos_ab[d];
       }
     }
   }
@@ -824,15 +829,24 @@ __global__ void __launch_bounds__(MIX_THREADS, 3) k_density_ff(Particles P,
     for(int d = 0; d < D; ++d)
       pa64[d] = P.f[F_X + d][a];
     const double h_a = P.f[F_H][a];
-    for(int j = 0; j < cnt; ++j) {
-      const int b = lp[slot_off(j)];
-      double pos_ab[3] = {0.0, 0.0, 0.0}, DiW[3];
-      for(int d = 0; d < D; ++d)
-        pos_ab[d] = pa64[d] - P.f[F_X + d][b];
-      kgrad<D, K>(pos_ab, .5 * (h_a + P.f[F_H][b]), DiW, pp);
-      const double mbd = P.f[F_M][b];
-      for(int d = 0; d < D; ++d)
-        gsum[d] += mbd * DiW[d];
+    PairH<D, K> ph;
+    ph.init();
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+      for(int u = 0; u < 4; ++u) {
+        // the padding slots (a itself) add nothing: x_ab = 0
+        const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
+        double pos_ab[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
+        for(int d = 0; d < D; ++d) {
+          pos_ab[d] = pa64[d] - P.f[F_X + d][b];
+          r2 += pos_ab[d] * pos_ab[d];
+        }
+        ph.template set<false, true>(h_a, P.f[F_H][b], pp);
+        const double mf = P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
+        for(int d = 0; d < D; ++d)
+          gsum[d] += mf * pos_ab[d];
+      }
     }
   }
   const double iE = Kp.fscale[1];
