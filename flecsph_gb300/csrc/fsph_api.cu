@@ -866,7 +866,7 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
   {
     Phase ph(c, FSPH_TIMER_SORT);
     CK(radix_sort_pairs(L, c->skeys, c->svals, c->skeys_tmp, c->svals_tmp, n,
-      c->hist, 0));
+      c->hist, 63 / c->pp.dim * c->pp.dim));
     CK(launch_check_duplicates(L, c->skeys, n, c->d_status));
     if(c->io.h2d_pending) {
       // fsph_step_io: input fields copied on the copy stream land first

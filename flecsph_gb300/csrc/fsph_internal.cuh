@@ -233,9 +233,10 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long> * mask, F app
 cudaError_t launch_range_keys(const Launch & L, const Particles & P,
   const PhysParams & pp, double * d_range, unsigned long long * keys_out,
   int * idx_out);
+// `bits`: the data bits of the keys, below a constant marker bit
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
-  unsigned * hist, int nblocks_cap);
+  unsigned * hist, int bits);
 size_t radix_hist_entries(int n);
 cudaError_t launch_check_duplicates(const Launch & L,
   const unsigned long long * keys, int n, DevStatus * st);

@@ -5,6 +5,7 @@
 // neighbour predicate must round exactly like the reference's FP64 code
 // (no fused multiply-add), so keys, sort order and neighbour sets are
 // bit-identical to the CPU reference.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -13,6 +14,8 @@
 #include "fsph_internal.cuh"
 
 namespace fsph {
+
+namespace cg = cooperative_groups;
 
 #define FULL 0xffffffffu
 
@@ -371,9 +374,325 @@ __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter
   }
 }
 
+// ---- one-cluster sort --------------------------------------------------
+// Up to SC_MAX keys one launch sorts everything: a cluster of up to 16 blocks,
+// each with an equal share of the places.  A digit pass ranks a block's keys as
+// k_radix_scatter does, the blocks exchange their digit counts through
+// distributed shared memory, and the keys, put in digit order in shared memory
+// first so that they leave in runs of consecutive addresses, go to their
+// places through L2 (stores to the owner's shared memory instead moved 6 bytes
+// a clock and SM, three times slower).  Two cluster barriers a pass; no launch
+// between passes.  The multi-launch path below spends 24 launches whose tiles
+// fill a few SMs at these sizes: range, keys and sort of 2,250 / 31,000 /
+// 132,651 keys take 33 / 44 / 76 us this way, 160 / 175 / 189 that way (at
+// 139,264 keys 78 against 188; beyond it a block's registers are full).
+// Latency bounds it: a pass of 8,300 keys a block is 33,000 cycles, 8,000 of
+// them the ballots, 5,000 the scatter.
+//
+// The passes cover the top data bits of the keys only, as many as tell n
+// particles spread over the range apart (the prefix has at least 32 values per
+// particle); keys that share a prefix are adjacent then, in input order, and
+// the thread of the first sorts them by insertion.  A run longer than SC_RUN
+// (a clump in a wide range) makes the cluster go on with all eight passes.
+#define SC_THREADS 512
+#define SC_WARPS (SC_THREADS / 32)
+#define SC_ITEMS 17
+#define SC_BLOCKS 16
+#define SC_MAX (SC_BLOCKS * SC_THREADS * SC_ITEMS)
+#define SC_RUN 12
+
+// Shared memory of one block with `per` places: keys and values in digit order
+// (at the end: in place order, with the places a run may reach into), digit
+// counts per warp and per block of the cluster (16 bits: at most
+// SC_THREADS * SC_ITEMS).
+__host__ __device__ constexpr size_t sc_smem(int per) {
+  return (size_t)(per + SC_RUN + 4) * 12 + SC_WARPS * 256 * 2 + SC_BLOCKS * 256 * 2 +
+         2 * 256 * 4 + 64 * 4;
+}
+
+__global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
+  unsigned long long * keys, int * vals, unsigned long long * keys_tmp, int * vals_tmp,
+  int n, int per, int bits, int prefix_bits) {
+  extern __shared__ __align__(16) unsigned char sc_dyn[];
+  unsigned long long * okey = (unsigned long long *)sc_dyn;
+  int * oval = (int *)(okey + per + SC_RUN + 4);
+  unsigned short * wcnt = (unsigned short *)(oval + per + SC_RUN + 4);
+  unsigned short * ccnt = wcnt + SC_WARPS * 256;
+  unsigned * base = (unsigned *)(ccnt + SC_BLOCKS * 256);  // where a digit's keys go
+  unsigned * toff = base + 256;  // where they start in digit order here
+  unsigned * aux = toff + 256;   // [0..15] scans, [16] long-run flag
+  cg::cluster_group cl = cg::this_cluster();
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const unsigned me = cl.block_rank(), nc = cl.num_blocks();
+  const int g0 = (int)me * per;                       // first place
+  const int mine = max(0, min(per, n - g0));          // places of this block
+  const int rounds = (per + SC_THREADS - 1) / SC_THREADS;
+  const unsigned lt = lanemask_lt();
+  unsigned long long *kin = keys, *kout = keys_tmp;
+  int *vin = vals, *vout = vals_tmp;
+  if(t == 0)
+    aux[16] = 0;
+  int first_shift = bits - prefix_bits;
+  while(true) {
+    for(int shift = first_shift; shift < bits; shift += 8) {
+      // warp w owns the places [w * 32 * rounds, ...) of the block
+      unsigned long long kreg[SC_ITEMS];
+      int vreg[SC_ITEMS];
+      unsigned rk[SC_ITEMS];  // lanes with the same digit, then the rank among the warp's
+      unsigned short * cnt = wcnt + w * 256;
+#pragma unroll
+      for(int r = 0; r < SC_ITEMS; ++r) {
+        const int i = (w * rounds + r) * 32 + lane;
+        const bool in = r < rounds && i < mine;
+        // (the other blocks wrote these: past the L1)
+        kreg[r] = in ? __ldcg(kin + g0 + i) : 0ull;
+        vreg[r] = in ? __ldcg(vin + g0 + i) : 0;
+      }
+      for(int i = lane; i < 128; i += 32)
+        ((unsigned *)cnt)[i] = 0;
+      __syncwarp();
+      // the lanes of a round that share a digit, by one ballot per bit (a
+      // match instruction takes ~1,000 cycles on 32 different digits here):
+      // independent between rounds, so they overlap; only the counts chain
+#pragma unroll
+      for(int r = 0; r < SC_ITEMS; ++r) {
+        if(r < rounds) {
+          const bool valid = (w * rounds + r) * 32 + lane < mine;
+          const unsigned digit = (unsigned)(kreg[r] >> shift) & 255u;
+          unsigned mask = __ballot_sync(FULL, valid);
+#pragma unroll
+          for(int bit = 0; bit < 8; ++bit) {
+            const bool on = (digit >> bit) & 1u;
+            const unsigned bal = __ballot_sync(FULL, on);
+            mask &= on ? bal : ~bal;
+          }
+          rk[r] = valid ? mask : 0u;
+        }
+      }
+#pragma unroll
+      for(int r = 0; r < SC_ITEMS; ++r) {
+        if(r < rounds) {
+          const unsigned mask = rk[r];
+          const unsigned digit = (unsigned)(kreg[r] >> shift) & 255u;
+          const unsigned before = mask ? cnt[digit] : 0u;
+          __syncwarp();
+          if(mask && (__ffs(mask) - 1) == lane)
+            cnt[digit] = (unsigned short)(before + __popc(mask));
+          __syncwarp();
+          rk[r] = before + __popc(mask & lt);
+        }
+      }
+      __syncthreads();
+      // per digit: prefix over the warps (two threads a digit, half the warps
+      // each); the digit's total goes to every block of the cluster
+      {
+        const int d = t >> 1, part = t & 1;
+        unsigned c[SC_WARPS / 2], sum = 0;
+#pragma unroll
+        for(int k = 0; k < SC_WARPS / 2; ++k) {
+          c[k] = sum;
+          sum += wcnt[(part * (SC_WARPS / 2) + k) * 256 + d];
+        }
+        const unsigned other = __shfl_xor_sync(FULL, sum, 1);
+#pragma unroll
+        for(int k = 0; k < SC_WARPS / 2; ++k)
+          wcnt[(part * (SC_WARPS / 2) + k) * 256 + d] =
+            (unsigned short)((part ? other : 0u) + c[k]);
+        for(unsigned b = part; b < nc; b += 2)
+          cl.map_shared_rank(ccnt, b)[me * 256 + d] = (unsigned short)(sum + other);
+      }
+      cl.sync();
+      // first place of each digit's keys of this block, in the cluster and in
+      // the block: two scans over the digits
+      unsigned tot = 0, pre = 0, own = 0, x = 0, y = 0;
+      if(t < 256) {
+        for(unsigned b = 0; b < nc; ++b) {
+          const unsigned c = ccnt[b * 256 + t];
+          pre += b < me ? c : 0u;
+          tot += c;
+        }
+        own = ccnt[me * 256 + t];
+        x = tot;
+        y = own;
+        for(int o = 1; o < 32; o <<= 1) {
+          const unsigned xo = __shfl_up_sync(FULL, x, o), yo = __shfl_up_sync(FULL, y, o);
+          if(lane >= o) {
+            x += xo;
+            y += yo;
+          }
+        }
+        if(lane == 31) {
+          aux[w] = x;
+          aux[8 + w] = y;
+        }
+      }
+      __syncthreads();
+      if(t < 256) {
+        unsigned loc = 0;
+        for(int k = 0; k < w; ++k) {
+          pre += aux[k];
+          loc += aux[8 + k];
+        }
+        base[t] = pre + x - tot;
+        toff[t] = loc + y - own;
+      }
+      __syncthreads();
+#pragma unroll
+      for(int r = 0; r < SC_ITEMS; ++r) {
+        const int i = (w * rounds + r) * 32 + lane;
+        if(r < rounds && i < mine) {
+          const unsigned d = (unsigned)(kreg[r] >> shift) & 255u;
+          const unsigned l = toff[d] + cnt[d] + rk[r];
+          okey[l] = kreg[r];
+          oval[l] = vreg[r];
+        }
+      }
+      __syncthreads();
+#pragma unroll 4
+      for(int l = t; l < mine; l += SC_THREADS) {
+        const unsigned long long key = okey[l];
+        const unsigned d = (unsigned)(key >> shift) & 255u;
+        const unsigned pos = base[d] + ((unsigned)l - toff[d]);
+        __stcg(kout + pos, key);
+        __stcg(vout + pos, oval[l]);
+      }
+      // the keys are in place, and nobody writes where somebody still reads:
+      // a pass reads one pair of buffers and writes the other
+      cl.sync();
+      unsigned long long * tk = kin;
+      kin = kout;
+      kout = tk;
+      int * tv = vin;
+      vin = vout;
+      vout = tv;
+    }
+    if(first_shift == 0)
+      break;
+    // Runs of equal prefixes: this block's places, the ones a run may reach
+    // into and the prefix before them.
+    const int ext = max(0, min(mine + SC_RUN + 1, n - g0));
+    for(int i = t; i < ext; i += SC_THREADS) {
+      okey[i] = __ldcg(kin + g0 + i);
+      oval[i] = __ldcg(vin + g0 + i);
+    }
+    const unsigned long long kprev = g0 > 0 && mine > 0 ? __ldcg(kin + g0 - 1) : 0ull;
+    __syncthreads();
+    auto prefix = [&](int i) { return (i < 0 ? kprev : okey[i]) >> first_shift; };
+    auto in_run = [&](int i) { return g0 + i > 0 && prefix(i - 1) == prefix(i); };
+    for(int i = t; i < mine; i += SC_THREADS)
+      if(i + SC_RUN < ext && prefix(i) == prefix(i + SC_RUN)) {
+        for(unsigned b = 0; b < nc; ++b)
+          cl.map_shared_rank(aux, b)[16] = 1;
+      }
+    cl.sync();
+    if(!aux[16]) {
+      // the first of a run puts it in order, the keys that begin no run and
+      // belong to none are in place
+      for(int i = t; i < mine; i += SC_THREADS) {
+        if(in_run(i))
+          continue;
+        int len = 1;
+        while(i + len < ext && prefix(i + len) == prefix(i)) {
+          const unsigned long long kv = okey[i + len];
+          const int vv = oval[i + len];
+          int z = i + len;
+          while(z > i && okey[z - 1] > kv) {
+            okey[z] = okey[z - 1];
+            oval[z] = oval[z - 1];
+            --z;
+          }
+          okey[z] = kv;
+          oval[z] = vv;
+          ++len;
+        }
+        for(int q = 0; q < len; ++q) {
+          keys[g0 + i + q] = okey[i + q];
+          vals[g0 + i + q] = oval[i + q];
+        }
+      }
+      return;
+    }
+    // go on from here with every digit: equal keys are still in input order
+    first_shift = 0;
+    bits = 64;
+  }
+  if(kin != keys)
+    for(int i = t; i < mine; i += SC_THREADS) {
+      keys[g0 + i] = __ldcg(kin + g0 + i);
+      vals[g0 + i] = __ldcg(vin + g0 + i);
+    }
+}
+
+// Blocks of the cluster for n keys, 0 where the sort takes several launches:
+// about 1,024 keys a block (one round of ranking) until the cluster is full.
+// A cluster of 16 is beyond the portable 8: asked of the device once.
+static int sc_blocks(int n) {
+  static std::atomic<unsigned long long> ready{0}, wide{0};
+  if(n > SC_MAX)
+    return 0;
+  int dev = 0;
+  if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+    return 0;
+  const cudaError_t e = once_per_device(&ready, [&]() {
+    const size_t most = sc_smem(SC_THREADS * SC_ITEMS);
+    cudaError_t r = cudaFuncSetAttribute(k_sort_cluster,
+      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if(r == cudaSuccess)
+      r = cudaFuncSetAttribute(k_sort_cluster,
+        cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if(r != cudaSuccess)
+      return r;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {SC_BLOCKS, 1, 1};
+    cfg.gridDim = dim3(SC_BLOCKS);
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.dynamicSmemBytes = most;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if(cudaOccupancyMaxActiveClusters(&fit, k_sort_cluster, &cfg) == cudaSuccess && fit > 0)
+      wide.fetch_or(1ull << dev, std::memory_order_release);
+    else
+      cudaGetLastError();
+    return cudaSuccess;
+  });
+  if(e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const bool w16 = (wide.load(std::memory_order_acquire) >> dev) & 1ull;
+  int c = 1;
+  while(c < (w16 ? SC_BLOCKS : 8) && n > c * SC_THREADS)
+    c <<= 1;
+  return n <= c * SC_THREADS * SC_ITEMS ? c : 0;
+}
+
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
-  unsigned * hist, int) {
+  unsigned * hist, int bits) {
+  if(const int c = sc_blocks(n)) {
+    const int per = ((n + c - 1) / c + 3) & ~3;
+    // prefix bits: at least 32 prefixes per key, in whole digits
+    int lg = 0;
+    while((1 << lg) < n)
+      ++lg;
+    const int pb = (lg + 5 + 7) / 8 * 8;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)c, 1, 1};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.dynamicSmemBytes = sc_smem(per);
+    cfg.stream = L.stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    *L.counter += 1;
+    return cudaLaunchKernelEx(&cfg, k_sort_cluster, keys, vals, keys_tmp, vals_tmp, n, per,
+      bits, pb);
+  }
   static std::atomic<unsigned long long> attr_devices{0};
   cudaError_t ae = once_per_device(&attr_devices, []() {
     return cudaFuncSetAttribute(k_radix_scatter,
@@ -1745,7 +2064,7 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
        perm_out) != cudaSuccess)
     return FSPH_ERR_CUDA;
   if(radix_sort_pairs(L, (unsigned long long *)keys_out, perm_out, ktmp, vtmp,
-       (int)n, hist, 0) != cudaSuccess)
+       (int)n, hist, 63 / dimension * dimension) != cudaSuccess)
     return FSPH_ERR_CUDA;
   return FSPH_OK;
 }
