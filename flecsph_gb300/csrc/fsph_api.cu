@@ -472,8 +472,6 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   ok &= dalloc(c, &c->svals_tmp, N) == cudaSuccess;
   ok &= dalloc(c, &c->hist, radix_hist_entries((int)N)) == cudaSuccess;
   ok &= dalloc(c, &c->d_range, 8) == cudaSuccess;
-  ok &= dalloc(c, &c->T.left, N) == cudaSuccess;
-  ok &= dalloc(c, &c->T.right, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.parent, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.leaf_parent, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.first, N) == cudaSuccess;
@@ -483,11 +481,11 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   ok &= dalloc(c, &c->T.fbox2, 2 * N) == cudaSuccess;
   ok &= dalloc(c, &c->T.opar, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.gref, N) == cudaSuccess;
-  ok &= dalloc(c, &c->T.counter, N) == cudaSuccess;
+  ok &= dalloc(c, &c->T.xchg, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.edepth, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.group_first, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.group_last, N) == cudaSuccess;
-  ok &= dalloc(c, &c->T.group_start, N) == cudaSuccess;
+  ok &= dalloc(c, &c->T.group_node, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.ngroups, 1) == cudaSuccess;
   ok &= dalloc(c, &c->K.qpos, N) == cudaSuccess;
   ok &= dalloc(c, &c->K.vhm, N) == cudaSuccess;
@@ -551,7 +549,8 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
       cudaGetLastError();
     }
   }
-  if(cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess)
+  if(cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess ||
+     cudaMemsetAsync(c->T.xchg, 0xff, sizeof(*c->T.xchg) * N, c->stream) != cudaSuccess)
     return fail(FSPH_ERR_CUDA);
   // timer and mark events are made on first use: an ensemble holds hundreds
   // of contexts that never time themselves
@@ -867,7 +866,6 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
     Phase ph(c, FSPH_TIMER_SORT);
     CK(radix_sort_pairs(L, c->skeys, c->svals, c->skeys_tmp, c->svals_tmp, n,
       c->hist, 63 / c->pp.dim * c->pp.dim));
-    CK(launch_check_duplicates(L, c->skeys, n, c->d_status));
     if(c->io.h2d_pending) {
       // fsph_step_io: input fields copied on the copy stream land first
       CK(cudaStreamWaitEvent(c->stream, c->io.ev[0], 0));
@@ -884,10 +882,10 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
   }
   {
     Phase ph(c, FSPH_TIMER_TREE);
-    CK(launch_pack_positions(L, c->P, c->pp, c->d_range, c->K));
+    CK(launch_pack_positions(L, c->P, c->pp, c->d_range, c->K, c->T.ngroups));
     CK(launch_build_tree(L, c->P, c->pp, c->T,
       c->p.group_size > 0 ? c->p.group_size : GROUP_MAX, c->d_range, c->K.qpos,
-      c->K.qscale, c->mixed ? 0 : 1));
+      c->K.qscale, c->mixed ? 0 : 1, c->d_status));
   }
   {
     // FP64 mode keeps each list in the reference's order so its sums round

@@ -72,7 +72,8 @@ struct PhysParams {
 };
 
 // Binary radix tree over the sorted keys (n-1 internal nodes, node 0 is the
-// root).  Child encoding: >= 0 internal node, < 0 leaf ~index.
+// root); the children of the node split at s are s and s + 1, each a node or a
+// leaf (the flags beside the split in qbox tell).
 struct NodeBox {   // 64 bytes: two aligned double4 loads
   double lo[3];
   double hmax;
@@ -81,8 +82,6 @@ struct NodeBox {   // 64 bytes: two aligned double4 loads
 };
 
 struct Tree {
-  int * left;
-  int * right;
   int * parent;       // internal node -> parent (-1 for the root)
   int * leaf_parent;  // particle -> parent internal node
   int * first;
@@ -94,11 +93,14 @@ struct Tree {
                            // lower corner, rounded outwards (lo, hi pairs)
   int * opar;              // particle -> binary node standing for its octree parent
   int * gref;              // particle -> its reference traversal group
-  unsigned * counter;
+  unsigned long long * xchg;  // per split: what the first child left there
+                              // during a build (all ones between builds)
   unsigned char * edepth;  // reference octree depth of each particle
   int * group_first;
   int * group_last;
-  int * group_start;       // per group: the node its mixed walk starts from
+  int * group_node;        // per group: its node, -1 for a single particle;
+                           // (in large runs: the node its mixed walk starts
+                           // from, once k_walk_start ran)
   int * ngroups;           // device scalar
   double * gmom;           // with gravity only (else null): per node the raw
                            // moments of mass about the range centre,
@@ -238,22 +240,22 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
   unsigned * hist, int bits);
 size_t radix_hist_entries(int n);
-cudaError_t launch_check_duplicates(const Launch & L,
-  const unsigned long long * keys, int n, DevStatus * st);
 cudaError_t launch_permute(const Launch & L, const Particles & src,
   const Particles & dst, const int * perm, const unsigned long long * keys,
   unsigned skip, float4 * vel = nullptr, int dim = 3);
 struct Packed;
 cudaError_t launch_build_tree(const Launch & L, const Particles & P,
   const PhysParams & pp, Tree & T, int group_max,
-  const unsigned long long * rbits, const int4 * qpos, const float * qscale, int ordered);
+  const unsigned long long * rbits, const int4 * qpos, const float * qscale, int ordered,
+  DevStatus * st);
 cudaError_t launch_neighbors(const Launch & L, const Particles & P,
   const PhysParams & pp, const Tree & T, Lists & Ls, DevStatus * st, int nsm,
   const unsigned long long * rbits, const Packed & K, int ordered);
 
 // ---- fsph_mixed.cu ----
+// also empties the tree's group count for the build that follows
 cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
-  const PhysParams & pp, const unsigned long long * rbits, const Packed & K);
+  const PhysParams & pp, const unsigned long long * rbits, const Packed & K, int * ngroups);
 cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm, int vel_current);

@@ -17,7 +17,7 @@ __device__ __forceinline__ double ord_dec_m(unsigned long long u) {
 
 // ------------------------------------------------------------- packing --
 __global__ void k_pack_pos(Particles P, int dim,
-  const unsigned long long * rbits, Packed K) {
+  const unsigned long long * rbits, Packed K, int * ngroups) {
   // Every position as one 48-bit fixed-point word per axis,
   //   F = round((x - lo) / E * 2^48),  E = the largest range extent
   //   enlarged by 2^-19 (so F < 2^48 - 2^28),
@@ -39,6 +39,7 @@ __global__ void k_pack_pos(Particles P, int dim,
     s_iE = 1.0 / E;
     s_sc = s_iE * 0x1p48;
     if(blockIdx.x == 0) {
+      *ngroups = 0;
       K.fscale[0] = E;
       K.fscale[1] = s_iE;
       // h_min == h_max: the pair passes take h_ab = h_a throughout
@@ -155,9 +156,10 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
 }
 
 cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
-  const PhysParams & pp, const unsigned long long * rbits, const Packed & K) {
+  const PhysParams & pp, const unsigned long long * rbits, const Packed & K,
+  int * ngroups) {
   const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
-  k_pack_pos<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K);
+  k_pack_pos<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups);
   *L.counter += 1;
   return cudaGetLastError();
 }

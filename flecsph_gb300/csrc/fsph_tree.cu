@@ -720,24 +720,6 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   return cudaGetLastError();
 }
 
-// Two particles with one full key make the reference's build_tree loop run
-// past depth 0 (tree_topology.h:957-971); report it instead.
-__global__ void k_check_dups(const unsigned long long * keys, int n,
-  DevStatus * st) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i + 1 < n && keys[i] == keys[i + 1]) {
-    if(atomicCAS(&st->code, 0, (int)FSPH_ERR_DUPLICATE_KEY) == 0)
-      st->index = i;
-  }
-}
-
-cudaError_t launch_check_duplicates(const Launch & L,
-  const unsigned long long * keys, int n, DevStatus * st) {
-  k_check_dups<<<(n + 255) / 256, 256, 0, L.stream>>>(keys, n, st);
-  *L.counter += 1;
-  return cudaGetLastError();
-}
-
 // Fields whose bit is set in `skip` are left behind: the caller overwrites
 // them before anything reads them.  With `vel`, the mixed path's
 // {v, c_s} record of the new order is written on the way (what the density
@@ -769,449 +751,376 @@ cudaError_t launch_permute(const Launch & L, const Particles & src,
 }
 
 // ------------------------------------------------------- radix tree -----
-// Karras (2012) binary radix tree over the sorted, distinct keys.
-// Equal keys (reported as FSPH_ERR_DUPLICATE_KEY) are ordered by index so
-// the tree stays a valid binary tree and every walk over it terminates.
-__device__ __forceinline__ int kdelta(const unsigned long long * k, int n,
-  int i, int j) {
-  if(j < 0 || j >= n)
-    return -1;
-  unsigned long long x = k[i] ^ k[j];
-  return x ? __clzll(x) : 64 + __clz((unsigned)(i ^ j));
+// Binary radix tree over the sorted keys.  Equal keys (reported as
+// FSPH_ERR_DUPLICATE_KEY) are ordered by index, so the tree stays a valid
+// binary tree and every walk over it terminates.
+// One launch builds the tree bottom up: a thread per leaf climbs, and of the
+// two children of a node the thread that arrives second forms it, so topology,
+// node data and walk groups come out of one climb (a top-down construction
+// first and a second climb for the groups read the node arrays three more
+// times, one dependent load after the other on every level).
+//
+// Where a node goes follows from its two ends alone: with D(i) the number of
+// bits the keys of i and i + 1 share (kdelta), a node [l, r] is the left child
+// of the node split at r if D(r) > D(l - 1), else the right child of the node
+// split at l - 1; as a left child its index is r, as a right child l, so the
+// children of a node split at s are always s and s + 1 (leaves or nodes).
+//
+// The thread that arrives first at split s leaves the far end of its child
+// and the D beyond it, the one that arrives second takes them.  A node whose
+// keys all lie in this block's 256 leaves (told from the two keys around
+// them) meets in shared memory, child data included; above that, a 64-bit
+// device-scope exchange releases the first child's data, which the second
+// thread reads through L2, and leaves the slot empty for the next build.
+//
+// Node data: the fixed-point position box and the largest h of every node
+// (what the neighbour walk prunes with); ALL (varying h, the ordered mode, or
+// gravity) adds the reference's FP64 box of x -/+ h/2 (compute_cofm,
+// default_physics.h:79-82,90-93) with its outward FP32 copy, and with gravity
+// the raw mass moments (ten FP64 sums; left child first, so the sums do not
+// depend on who combined them).  The boxes combine on the integer pipe: FP64
+// comparisons at every node would bind the climb on this part.  The outward
+// FP32 copies combine among themselves, rounding being monotonic.
+//
+// Latency bounds it: about 150 ns a level in shared memory, 0.8 us above.
+#define TREE_THREADS 256
+#define TREE_EMPTY 0xffffffffffffffffull
+
+// smaller and larger of two finite doubles by their bits
+__device__ __forceinline__ bool less_bits(double a, double b) {
+  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  x ^= (long long)((unsigned long long)(x >> 63) >> 1);
+  y ^= (long long)((unsigned long long)(y >> 63) >> 1);
+  return x < y;
 }
 
-__global__ void k_karras(const unsigned long long * K, int n, Tree T) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n - 1)
-    return;
-  int d = (kdelta(K, n, i, i + 1) - kdelta(K, n, i, i - 1)) > 0 ? 1 : -1;
-  int dmin = kdelta(K, n, i, i - d);
-  int lmax = 2;
-  while(kdelta(K, n, i, i + lmax * d) > dmin)
-    lmax <<= 1;
-  int l = 0;
-  for(int t = lmax >> 1; t >= 1; t >>= 1)
-    if(kdelta(K, n, i, i + (l + t) * d) > dmin)
-      l += t;
-  int j = i + l * d;
-  int dnode = kdelta(K, n, i, j);
-  int s = 0, t = l;
-  while(true) {
-    t = (t + 1) >> 1;
-    if(kdelta(K, n, i, i + (s + t) * d) > dnode)
-      s += t;
-    if(t == 1)
-      break;
-  }
-  int gamma = i + s * d + (d < 0 ? -1 : 0);
-  int first = min(i, j), last = max(i, j);
-  int left = (first == gamma) ? ~gamma : gamma;
-  int right = (last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-  T.left[i] = left;
-  T.right[i] = right;
-  T.first[i] = first;
-  T.last[i] = last;
-  if(left < 0)
-    T.leaf_parent[gamma] = i;
-  else
-    T.parent[gamma] = i;
-  if(right < 0)
-    T.leaf_parent[gamma + 1] = i;
-  else
-    T.parent[gamma + 1] = i;
-  if(i == 0)
-    T.parent[0] = -1;
-}
-
-// Depth of each particle in the reference's octree: one level below its
-// deepest shared prefix with a key neighbour (tree_topology.h:957-986).
-__global__ void k_edepth(const unsigned long long * K, int n, int dim,
-  unsigned char * ed) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n)
-    return;
-  const int md = 63 / dim;
-  const int lead = 64 - md * dim;
-  int best = 0;
-  if(i > 0)
-    best = max(best, (__clzll(K[i] ^ K[i - 1]) - lead) / dim);
-  if(i + 1 < n)
-    best = max(best, (__clzll(K[i] ^ K[i + 1]) - lead) / dim);
-  ed[i] = (unsigned char)(best + 1);
-}
-
-// Bottom-up node data: the fixed-point position box and the largest h of
-// every node (what the neighbour walk prunes with); only when h varies, the
-// reference's FP64 box of x -/+ h/2 (compute_cofm, default_physics.h:
-// 79-82,90-93) used by the reference node tests; only with gravity, the
-// node's raw mass moments (ten FP64 sums: children add, so every level
-// costs ten additions whatever the order of the multipoles built from
-// them).
-// refboxes: also the reference's x +- h/2 node boxes (box2, fbox2), which
-// the walk's node tests read: with varying h, or in the ordered (FP64) mode
-// where equal-h ties take them too.
-// Shared-memory layout of one k_bounds_* block (dynamic): the node data of the
-// internal nodes whose leaf range lies inside the block's own leaves (slot =
-// node index - first leaf of the block: such a node's index is one end of
-// its range), their arrival counters, two work queues and the list of the
-// block's topmost nodes (and leaves) whose parents lie outside it.
-#define BOUNDS_THREADS 256
-__host__ __device__ constexpr size_t bounds_smem(bool gmom) {
-  return (size_t)BOUNDS_THREADS * (2 * sizeof(int4) + 6 * sizeof(double) + sizeof(unsigned) +
-                                   3 * sizeof(int) + (gmom ? 10 * sizeof(double) : 0)) +
-         4 * sizeof(int);
-}
-
-struct BoundsShared {
-  int4 * sq;        // lo, hi per slot
-  double * sb;      // box2 lo xyz, hi xyz per slot
-  unsigned * scnt;  // arrival counts per slot
-  int * queue;      // 2 x 256: nodes whose two children are done (current pass, next pass)
-  int * exits;      // nodes (~leaf for a leaf) whose parent is outside the block
-  int * counts;     // queue lengths [2], exit count
-  double * sg;      // ten moments per slot (gravity)
+template<bool ALL>
+struct TreeData {
+  int4 lo, hi;        // lo.w: float bits of h_max; hi.w: the children's code
+};
+template<>
+struct TreeData<true> {
+  int4 lo, hi;
+  double b[6];        // x - h/2 minima, x + h/2 maxima
+  float f[6];         // the same relative to the range's corner, outwards
+  double g[10];       // moments
 };
 
-// Node p's data from its two children, written to device memory and, for a
-// node inside the block (local), to its shared-memory slot.  A local node's
-// inner children are local too and are read from shared memory; the
-// children of other nodes from device memory through L2.  Children combine
-// in a fixed order (left, then right), so the sums do not depend on which
-// thread or path combined a node.
-template<int dim>
-__device__ __forceinline__ void bounds_node(const Particles & P, const Tree & T, const int4 * qpos,
-  const BoundsShared & S, int p, bool local, int b0, bool nonuni, const double * rc,
-  const double * r0) {
-  const int cg[2] = {T.left[p], T.right[p]};
-  if(T.gmom) {
-    double M[10];
-    for(int c = 0; c < 2; ++c) {
-      double C[10];
-      if(cg[c] < 0) {
-        const int j = ~cg[c];
-        const double m = P.f[F_M][j];
-        double y[3] = {0.0, 0.0, 0.0};
-        for(int d = 0; d < dim; ++d)
-          y[d] = P.f[F_X + d][j] - rc[d];
-        const double my[3] = {m * y[0], m * y[1], m * y[2]};
-        C[0] = m;
-        C[1] = my[0];
-        C[2] = my[1];
-        C[3] = my[2];
-        C[4] = my[0] * y[0];
-        C[5] = my[1] * y[1];
-        C[6] = my[2] * y[2];
-        C[7] = my[0] * y[1];
-        C[8] = my[0] * y[2];
-        C[9] = my[1] * y[2];
-      }
-      else if(local) {
-        const double * cs = S.sg + (cg[c] - b0);
-        for(int k = 0; k < 10; ++k)
-          C[k] = cs[k * BOUNDS_THREADS];
-      }
-      else {
-        const double * cs = T.gmom + 10 * (size_t)cg[c];
-        for(int k = 0; k < 10; ++k)
-          C[k] = __ldcg(cs + k);
-      }
-      for(int k = 0; k < 10; ++k)
-        M[k] = c == 0 ? C[k] : M[k] + C[k];
-    }
-    double * out = T.gmom + 10 * (size_t)p;
-    for(int k = 0; k < 10; ++k)
-      out[k] = M[k];
-    if(local)
-      for(int k = 0; k < 10; ++k)
-        S.sg[k * BOUNDS_THREADS + (p - b0)] = M[k];
+template<bool ALL>
+__host__ __device__ constexpr size_t tree_smem() {
+  return 2 * TREE_THREADS * (ALL ? 32 + 48 + 24 + 80 : 32);
+}
+
+// (1: shared-memory deposit of a child, slot q of 2 * TREE_THREADS, as
+// structure of arrays)
+template<bool ALL, bool STORE>
+__device__ __forceinline__ void tree_slot(unsigned char * sm, int q, TreeData<ALL> & d,
+  bool boxes, bool mom) {
+  constexpr int N = 2 * TREE_THREADS;
+  int4 * s4 = (int4 *)sm;
+  if(STORE) {
+    s4[q] = d.lo;
+    s4[N + q] = d.hi;
   }
-  int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
-  int hi[3] = {-1, -1, -1};
-  float hm = 0.f;
-  double blo[3] = {1e308, 1e308, 1e308}, bhi[3] = {-1e308, -1e308, -1e308};
-  for(int c = 0; c < 2; ++c) {
-    if(cg[c] < 0) {
-      const int j = ~cg[c];
-      const int4 q = qpos[j];
-      lo[0] = min(lo[0], q.x); hi[0] = max(hi[0], q.x);
-      lo[1] = min(lo[1], q.y); hi[1] = max(hi[1], q.y);
-      lo[2] = min(lo[2], q.z); hi[2] = max(hi[2], q.z);
-      hm = fmaxf(hm, __int_as_float(q.w));
-      if(nonuni) {
-        const double hj = P.f[F_H][j];
-        for(int d = 0; d < dim; ++d) {
-          double x = P.f[F_X + d][j];
-          blo[d] = fmin(blo[d], x - hj / 2.);
-          bhi[d] = fmax(bhi[d], x + hj / 2.);
-        }
-      }
-    }
-    else {
-      int4 a, b;
-      if(local) {
-        a = S.sq[2 * (cg[c] - b0)];
-        b = S.sq[2 * (cg[c] - b0) + 1];
-      }
-      else {
-        const int4 * cq = &T.qbox[2 * cg[c]];
-        a = __ldcg(cq);
-        b = __ldcg(cq + 1);
-      }
-      lo[0] = min(lo[0], a.x); lo[1] = min(lo[1], a.y); lo[2] = min(lo[2], a.z);
-      hi[0] = max(hi[0], b.x); hi[1] = max(hi[1], b.y); hi[2] = max(hi[2], b.z);
-      hm = fmaxf(hm, __int_as_float(a.w));
-      if(nonuni) {
-        if(local) {
-          const double * cb2 = S.sb + (cg[c] - b0);
-          for(int d = 0; d < dim; ++d) {
-            blo[d] = fmin(blo[d], cb2[d * BOUNDS_THREADS]);
-            bhi[d] = fmax(bhi[d], cb2[(3 + d) * BOUNDS_THREADS]);
-          }
+  else {
+    d.lo = s4[q];
+    d.hi = s4[N + q];
+  }
+  if constexpr(ALL) {
+    double * sb = (double *)(sm + (size_t)N * 32);
+    double * sg = sb + 6 * N;
+    float * sf = (float *)(sg + 10 * N);
+    if(boxes)
+      for(int k = 0; k < 6; ++k) {
+        if(STORE) {
+          sb[k * N + q] = d.b[k];
+          sf[k * N + q] = d.f[k];
         }
         else {
-          const double * cb2 = (const double *)&T.box2[cg[c]];
-          for(int d = 0; d < dim; ++d) {
-            blo[d] = fmin(blo[d], __ldcg(cb2 + d));
-            bhi[d] = fmax(bhi[d], __ldcg(cb2 + 4 + d));
-          }
+          d.b[k] = sb[k * N + q];
+          d.f[k] = sf[k * N + q];
+        }
+      }
+    if(mom)
+      for(int k = 0; k < 10; ++k) {
+        if(STORE)
+          sg[k * N + q] = d.g[k];
+        else
+          d.g[k] = sg[k * N + q];
+      }
+  }
+}
+
+template<int dim, bool ALL>
+__device__ __forceinline__ void tree_leaf(const Particles & P, const int4 * qpos, int j,
+  bool boxes, bool mom, const double * rc, const double * r0, TreeData<ALL> & d) {
+  const int4 q = qpos[j];
+  d.lo = q;
+  d.hi = make_int4(q.x, q.y, q.z, 0);
+  if constexpr(ALL) {
+    double x[3] = {0.0, 0.0, 0.0};
+    for(int k = 0; k < dim; ++k)
+      x[k] = P.f[F_X + k][j];
+    if(boxes) {
+      const double hh = P.f[F_H][j] / 2.;
+      for(int k = 0; k < 3; ++k) {
+        d.b[k] = k < dim ? x[k] - hh : 0.0;
+        d.b[3 + k] = k < dim ? x[k] + hh : 0.0;
+        d.f[k] = k < dim ? __double2float_rd(d.b[k] - r0[k]) : 0.f;
+        d.f[3 + k] = k < dim ? __double2float_ru(d.b[3 + k] - r0[k]) : 0.f;
+      }
+    }
+    if(mom) {
+      const double m = P.f[F_M][j];
+      double y[3] = {0.0, 0.0, 0.0};
+      for(int k = 0; k < dim; ++k)
+        y[k] = x[k] - rc[k];
+      const double my[3] = {m * y[0], m * y[1], m * y[2]};
+      d.g[0] = m;
+      d.g[1] = my[0];
+      d.g[2] = my[1];
+      d.g[3] = my[2];
+      d.g[4] = my[0] * y[0];
+      d.g[5] = my[1] * y[1];
+      d.g[6] = my[2] * y[2];
+      d.g[7] = my[0] * y[1];
+      d.g[8] = my[0] * y[2];
+      d.g[9] = my[1] * y[2];
+    }
+  }
+}
+
+// node p's data to (STORE) or from device memory (through L2)
+template<bool ALL, bool STORE>
+__device__ __forceinline__ void tree_node_mem(const Tree & T, int p, TreeData<ALL> & d,
+  bool boxes, bool mom) {
+  if(STORE) {
+    T.qbox[2 * p] = d.lo;
+    T.qbox[2 * p + 1] = d.hi;
+  }
+  else {
+    d.lo = __ldcg(&T.qbox[2 * p]);
+    d.hi = __ldcg(&T.qbox[2 * p + 1]);
+  }
+  if constexpr(ALL) {
+    if(boxes) {
+      // NodeBox: lo xyz, hmax (0), hi xyz, pad (0)
+      double2 * bx = (double2 *)&T.box2[p];
+      float4 * fx = T.fbox2 + 2 * (size_t)p;
+      if(STORE) {
+        bx[0] = make_double2(d.b[0], d.b[1]);
+        bx[1] = make_double2(d.b[2], 0.0);
+        bx[2] = make_double2(d.b[3], d.b[4]);
+        bx[3] = make_double2(d.b[5], 0.0);
+        fx[0] = make_float4(d.f[0], d.f[1], d.f[2], 0.f);
+        fx[1] = make_float4(d.f[3], d.f[4], d.f[5], 0.f);
+      }
+      else {
+        const double2 b0 = __ldcg(bx), b1 = __ldcg(bx + 1), b2 = __ldcg(bx + 2),
+                      b3 = __ldcg(bx + 3);
+        const float4 f0 = __ldcg(fx), f1 = __ldcg(fx + 1);
+        d.b[0] = b0.x; d.b[1] = b0.y; d.b[2] = b1.x;
+        d.b[3] = b2.x; d.b[4] = b2.y; d.b[5] = b3.x;
+        d.f[0] = f0.x; d.f[1] = f0.y; d.f[2] = f0.z;
+        d.f[3] = f1.x; d.f[4] = f1.y; d.f[5] = f1.z;
+      }
+    }
+    if(mom) {
+      double2 * gm = (double2 *)(T.gmom + 10 * (size_t)p);
+      for(int k = 0; k < 5; ++k) {
+        if(STORE)
+          gm[k] = make_double2(d.g[2 * k], d.g[2 * k + 1]);
+        else {
+          const double2 v = __ldcg(gm + k);
+          d.g[2 * k] = v.x;
+          d.g[2 * k + 1] = v.y;
         }
       }
     }
   }
-  // children of a radix-tree node are always (split, split + 1): store
-  // split and the two leaf flags with the box, so the walk needs one load
-  const int l = cg[0], r = cg[1];
-  const int split = l < 0 ? ~l : l;
-  const int code = (split << 2) | ((l < 0) << 1) | (r < 0);
-  const int4 qlo = make_int4(lo[0], lo[1], lo[2], __float_as_int(hm));
-  const int4 qhi = make_int4(hi[0], hi[1], hi[2], code);
-  T.qbox[2 * p] = qlo;
-  T.qbox[2 * p + 1] = qhi;
-  if(local) {
-    S.sq[2 * (p - b0)] = qlo;
-    S.sq[2 * (p - b0) + 1] = qhi;
-  }
-  if(nonuni) {
-    if(dim == 2)
-      blo[2] = bhi[2] = 0;
-    // NodeBox: lo xyz, hmax (0), hi xyz, pad (0)
-    double4 * bx = (double4 *)&T.box2[p];
-    bx[0] = make_double4(blo[0], blo[1], blo[2], 0.0);
-    bx[1] = make_double4(bhi[0], bhi[1], bhi[2], 0.0);
-    if(local)
-      for(int d = 0; d < 3; ++d) {
-        S.sb[d * BOUNDS_THREADS + (p - b0)] = blo[d];
-        S.sb[(3 + d) * BOUNDS_THREADS + (p - b0)] = bhi[d];
+}
+
+// d: one child on entry, the node of both on return
+template<bool ALL>
+__device__ __forceinline__ void tree_merge(TreeData<ALL> & d, const TreeData<ALL> & e,
+  bool boxes, bool mom) {
+  d.lo.x = min(d.lo.x, e.lo.x);
+  d.lo.y = min(d.lo.y, e.lo.y);
+  d.lo.z = min(d.lo.z, e.lo.z);
+  d.hi.x = max(d.hi.x, e.hi.x);
+  d.hi.y = max(d.hi.y, e.hi.y);
+  d.hi.z = max(d.hi.z, e.hi.z);
+  d.lo.w = __float_as_int(fmaxf(__int_as_float(d.lo.w), __int_as_float(e.lo.w)));
+  if constexpr(ALL) {
+    if(boxes)
+      for(int k = 0; k < 3; ++k) {
+        d.b[k] = less_bits(e.b[k], d.b[k]) ? e.b[k] : d.b[k];
+        d.b[3 + k] = less_bits(d.b[3 + k], e.b[3 + k]) ? e.b[3 + k] : d.b[3 + k];
+        d.f[k] = fminf(d.f[k], e.f[k]);
+        d.f[3 + k] = fmaxf(d.f[3 + k], e.f[3 + k]);
       }
-    float fl[3] = {0.f, 0.f, 0.f}, fh[3] = {0.f, 0.f, 0.f};
-    for(int d = 0; d < dim; ++d) {
-      fl[d] = __double2float_rd(blo[d] - r0[d]);
-      fh[d] = __double2float_ru(bhi[d] - r0[d]);
-    }
-    T.fbox2[2 * p] = make_float4(fl[0], fl[1], fl[2], 0.f);
-    T.fbox2[2 * p + 1] = make_float4(fh[0], fh[1], fh[2], 0.f);
+    if(mom)
+      for(int k = 0; k < 10; ++k)
+        d.g[k] = d.g[k] + e.g[k];
   }
 }
 
-__device__ __forceinline__ BoundsShared bounds_shared(unsigned char * bsm) {
-  BoundsShared S;
-  S.sq = (int4 *)bsm;
-  S.sb = (double *)(S.sq + 2 * BOUNDS_THREADS);
-  S.scnt = (unsigned *)(S.sb + 6 * BOUNDS_THREADS);
-  S.queue = (int *)(S.scnt + BOUNDS_THREADS);
-  S.exits = S.queue + 2 * BOUNDS_THREADS;
-  S.counts = S.exits + BOUNDS_THREADS;
-  S.sg = (double *)(S.counts + 4);
-  return S;
-}
-
-// The bottom-up pass comes in two variants; both are launched and the one
-// the run does not select returns at once.
-//
-// With gravity or varying h (FP64 moments and x +- h/2 boxes per node):
-// inside a block (its 256 leaves), rounds separated by block barriers, each
-// combining the nodes whose two children finished in earlier rounds, taken
-// from a compacted queue so that whole warps do the FP64 node arithmetic (a
-// thread per leaf climbing the tree keeps ~1/3 of its lanes busy, and the
-// FP64 pipe, not the lanes, is what the node arithmetic waits on); a
-// shared-memory count per node finds the round in which its second child
-// finishes.  Above the block -- nodes whose range straddles a block
-// boundary, a few per block -- the classic chain: the thread arriving second
-// at a node (a device-scope acquire-release count) combines it and climbs
-// on.  4M polytrope: 5.03 -> 2.84 ms per tree phase.  One block per 256
-// leaves: a smaller grid striding over the leaf blocks (so that equal-h runs
-// skip the variant in one wave) measured 4.30 ms, as each block's climb
-// above its leaves then holds back its next leaves.
-//
-// Equal h without gravity (integer boxes only): the chain from every leaf,
-// with the counts and node data of the nodes inside the block in shared
-// memory (block-scope fences order them); there the barriers of the round
-// variant cost more than the idle lanes (Sedov 128^3 tree phase 0.48 ms
-// against 0.58).
-template<int dim>
-__global__ void __launch_bounds__(BOUNDS_THREADS) k_bounds_chain(Particles P, Tree T,
-  const int4 * qpos, const unsigned long long * rbits, int refboxes) {
-  if(T.gmom || refboxes || rbits[6] != rbits[7])
-    return;  // the round variant's run
-  extern __shared__ __align__(16) unsigned char bsm[];
-  const BoundsShared S = bounds_shared(bsm);
-  const int b0 = blockIdx.x * BOUNDS_THREADS;
-  const int b1 = min(b0 + BOUNDS_THREADS, P.n) - 1;
-  S.scnt[threadIdx.x] = 0u;
-  __syncthreads();
-  const int i = b0 + threadIdx.x;
-  if(i >= P.n)
+// ALL or not: both are launched, and the one the device's range words do not
+// select returns at once.  lead: the key bits above the data.  Two particles
+// with one full key would make the reference's build_tree loop run past depth
+// 0 (tree_topology.h:957-971): reported.
+template<int dim, bool ALL>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree(const unsigned long long * K,
+  Particles P, Tree T, const int4 * qpos, const unsigned long long * rbits, int ordered,
+  int gmax, DevStatus * st) {
+  const bool boxes = ordered || rbits[6] != rbits[7], mom = T.gmom != nullptr;
+  if(ALL != (boxes || mom))
     return;
-  const double rc[3] = {0.0, 0.0, 0.0}, r0[3] = {0.0, 0.0, 0.0};
-  int p = T.leaf_parent[i];
-  while(p >= 0) {
-    const bool local = T.first[p] >= b0 && T.last[p] <= b1;
-    unsigned prior;
+  extern __shared__ __align__(16) unsigned char tsm[];
+  __shared__ unsigned long long skey[TREE_THREADS + 2];  // keys b0 - 1 .. b1 + 1
+  __shared__ unsigned sx[TREE_THREADS];  // far end - b0 | (D + 1) << 16
+  const int n = P.n, t = threadIdx.x;
+  const int b0 = blockIdx.x * TREE_THREADS;
+  const int b1 = min(b0 + TREE_THREADS, n) - 1;
+  const int i = b0 + t;
+  if(i <= b1)
+    skey[t + 1] = K[i];
+  if(t == 0)
+    skey[0] = b0 > 0 ? K[b0 - 1] : 0ull;
+  if(t == 1 || b1 == b0)
+    skey[b1 - b0 + 2] = b1 + 1 < n ? K[b1 + 1] : 0ull;
+  sx[t] = 0xffffffffu;
+  __syncthreads();
+  if(i > b1)
+    return;
+  // bits the keys of two particles share, equal keys told apart by index
+  auto shared_bits = [&](unsigned long long x, int a, unsigned long long y, int b) {
+    x ^= y;
+    return x ? __clzll(x) : 64 + __clz((unsigned)(a ^ b));
+  };
+  auto D = [&](int a) {  // of a and a + 1, both in the block or next to it
+    return a < 0 || a + 1 >= n ? -1 : shared_bits(skey[a - b0 + 1], a, skey[a - b0 + 2], a + 1);
+  };
+  double rc[3] = {0.0, 0.0, 0.0}, r0[3] = {0.0, 0.0, 0.0};
+  if(ALL)
+    for(int d = 0; d < dim; ++d) {
+      r0[d] = ord_dec(rbits[d]);
+      rc[d] = 0.5 * (r0[d] + ord_dec(rbits[3 + d]));
+    }
+  int l = i, r = i, split = -1;
+  int dl = D(i - 1), dr = D(i);
+  if(dr >= 64) {
+    if(atomicCAS(&st->code, 0, (int)FSPH_ERR_DUPLICATE_KEY) == 0)
+      st->index = i;
+  }
+  if(ordered) {
+    // depth in the reference's octree: one level below the deepest prefix
+    // shared with a key neighbour (tree_topology.h:957-986)
+    const int lead = 64 - (63 / dim) * dim;
+    int best = 0;
+    if(i > 0)
+      best = max(best, (min(dl, 64) - lead) / dim);
+    if(i + 1 < n)
+      best = max(best, (min(dr, 64) - lead) / dim);
+    T.edepth[i] = (unsigned char)(best + 1);
+  }
+  TreeData<ALL> d;
+  tree_leaf<dim, ALL>(P, qpos, i, boxes, mom, rc, r0, d);
+  while(true) {
+    const bool left = dr > dl;   // the left child of the node split at r
+    const int idx = left ? r : l;
+    if(split >= 0) {
+      d.hi.w = (split << 2) | ((l == split) << 1) | (r == split + 1);
+      T.first[idx] = l;
+      T.last[idx] = r;
+      if(l == split)
+        T.leaf_parent[split] = idx;
+      else
+        T.parent[split] = idx;
+      if(r == split + 1)
+        T.leaf_parent[split + 1] = idx;
+      else
+        T.parent[split + 1] = idx;
+      tree_node_mem<ALL, true>(T, idx, d, boxes, mom);
+      if(l == 0 && r == n - 1) {
+        T.parent[0] = -1;
+        if(n <= gmax) {
+          const int slot = atomicAdd(T.ngroups, 1);
+          T.group_first[slot] = 0;
+          T.group_last[slot] = r;
+          T.group_node[slot] = 0;
+        }
+        return;
+      }
+    }
+    const int s = left ? r : l - 1;
+    const int far = left ? l : r, outer = left ? dl : dr;
+    // the parent holds the keys that share at least D(s) bits with that of s:
+    // inside the block if neither key around the block does
+    bool local = s >= b0 && s < b1;
     if(local) {
-      // shared-memory count at block scope: the fences order this thread's
-      // node data before the count (release) and the sibling's after it
-      // (acquire)
+      const unsigned long long ks = skey[s - b0 + 1];
+      const int ds = left ? dr : dl;
+      local = (b0 == 0 || shared_bits(skey[0], b0 - 1, ks, s) < ds) &&
+              (b1 == n - 1 || shared_bits(skey[b1 - b0 + 2], b1 + 1, ks, s) < ds);
+    }
+    int sib_far, sib_outer;
+    TreeData<ALL> e;
+    if(local) {
+      const int q = s - b0;
+      tree_slot<ALL, true>(tsm, q + (left ? 0 : TREE_THREADS), d, boxes, mom);
+      // the fences order the deposit before the exchange and the sibling's
+      // deposit, read below, after it
       __threadfence_block();
-      prior = atomicAdd(&S.scnt[p - b0], 1u);
+      const unsigned prior =
+        atomicExch(&sx[q], (unsigned)(far - b0) | ((unsigned)(outer + 1) << 16));
+      if(prior == 0xffffffffu)
+        return;
       __threadfence_block();
+      sib_far = b0 + (int)(prior & 0xffffu);
+      sib_outer = (int)(prior >> 16) - 1;
+      tree_slot<ALL, false>(tsm, q + (left ? TREE_THREADS : 0), e, boxes, mom);
     }
     else {
-      // device-scope acquire-release count: publishes this thread's node
-      // data (release) to the sibling's thread, which reads it after its
-      // own arrival (acquire; the reads go through L2 with __ldcg)
-      asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], 1;"
-                   : "=r"(prior) : "l"(T.counter + p) : "memory");
+      unsigned long long prior;
+      const unsigned long long mine =
+        (unsigned long long)(unsigned)far | ((unsigned long long)(outer + 1) << 32);
+      // releases this child's data, written above, and acquires the sibling's
+      asm volatile("atom.acq_rel.gpu.exch.b64 %0, [%1], %2;"
+                   : "=l"(prior) : "l"(T.xchg + s), "l"(mine) : "memory");
+      if(prior == TREE_EMPTY)
+        return;
+      T.xchg[s] = TREE_EMPTY;  // for the next build
+      sib_far = (int)(unsigned)prior;
+      sib_outer = (int)(prior >> 32) - 1;
+      const int sib = left ? s + 1 : s;
+      if(sib_far == sib)
+        tree_leaf<dim, ALL>(P, qpos, sib, boxes, mom, rc, r0, e);
+      else
+        tree_node_mem<ALL, false>(T, sib, e, boxes, mom);
     }
-    if(prior == 0)
-      return;  // the sibling subtree is not finished yet
-    bounds_node<dim>(P, T, qpos, S, p, local, b0, false, rc, r0);
-    p = T.parent[p];
-  }
-}
-
-template<int dim>
-__global__ void __launch_bounds__(BOUNDS_THREADS) k_bounds_rounds(Particles P, Tree T,
-  const int4 * qpos, const unsigned long long * rbits, int refboxes) {
-  const bool nonuni = refboxes || rbits[6] != rbits[7];
-  if(!T.gmom && !nonuni)
-    return;  // the chain variant's run
-  extern __shared__ __align__(16) unsigned char bsm[];
-  const BoundsShared S = bounds_shared(bsm);
-  const int t = threadIdx.x;
-  const int b0 = blockIdx.x * BOUNDS_THREADS;
-  const int b1 = min(b0 + BOUNDS_THREADS, P.n) - 1;
-  S.scnt[t] = 0u;
-  if(t < 4)
-    S.counts[t] = 0;
-  double rc[3] = {0.0, 0.0, 0.0}, r0[3] = {0.0, 0.0, 0.0};
-  for(int d = 0; d < dim; ++d) {
-    r0[d] = ord_dec(rbits[d]);
-    if(T.gmom)
-      rc[d] = 0.5 * (r0[d] + ord_dec(rbits[3 + d]));
-  }
-  auto is_local = [&](int v) { return T.first[v] >= b0 && T.last[v] <= b1; };
-  // a node (or ~leaf) whose data are final: count its arrival at the parent
-  auto arrive = [&](int v, int next) {
-    const int p = v < 0 ? T.leaf_parent[~v] : T.parent[v];
-    if(p < 0)
-      return;
-    if(is_local(p)) {
-      if(atomicAdd(&S.scnt[p - b0], 1u) == 1u)
-        S.queue[next * BOUNDS_THREADS + atomicAdd(&S.counts[next], 1)] = p;
+    tree_merge<ALL>(d, e, boxes, mom);
+    if(left) {
+      r = sib_far;
+      dr = sib_outer;
     }
-    else
-      S.exits[atomicAdd(&S.counts[2], 1)] = v;
-  };
-  __syncthreads();
-  if(b0 + t <= b1)
-    arrive(~(b0 + t), 0);
-  __syncthreads();
-  for(int cur = 0;; cur ^= 1) {
-    const int len = S.counts[cur];
-    if(len == 0)
-      break;
-    __syncthreads();  // every thread has read len
-    if(t == 0)
-      S.counts[cur] = 0;  // the queue after next reuses this one
-    if(t < len) {
-      const int p = S.queue[cur * BOUNDS_THREADS + t];
-      bounds_node<dim>(P, T, qpos, S, p, true, b0, nonuni, rc, r0);
-      arrive(p, cur ^ 1);
+    else {
+      l = sib_far;
+      dl = sib_outer;
     }
-    __syncthreads();
-  }
-  const int nex = S.counts[2];
-  if(nex == 0)
-    return;
-  // the exits' data (written by any thread of the block before the last
-  // barrier) become visible device-wide before this thread's counts
-  __threadfence();
-  for(int e = t; e < nex; e += BOUNDS_THREADS) {
-    const int v = S.exits[e];
-    int p = v < 0 ? T.leaf_parent[~v] : T.parent[v];
-    while(p >= 0) {
-      unsigned prior;
-      asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], 1;"
-                   : "=r"(prior) : "l"(T.counter + p) : "memory");
-      if(prior == 0)
-        break;  // the sibling subtree is not finished yet
-      bounds_node<dim>(P, T, qpos, S, p, false, b0, nonuni, rc, r0);
-      p = T.parent[p];
-    }
-  }
-}
-
-// Groups: maximal subtrees with at most `gmax` particles.  Each group also
-// gets the node its mixed walk starts from: the lowest ancestor whose
-// fixed-point box, less one step on every side, holds the group's box grown
-// by the largest reach (max h, with the walk's 1e-5 slack and two steps for
-// the quantisation).  A radix-tree node holds every particle whose key
-// shares its prefix, so its particles' box lies in that Morton cell; a
-// particle within reach lies in the grown box, hence a step inside the
-// node's box, hence in the cell and in the subtree: the walk below that
-// node finds every candidate the walk from the root finds.
-__global__ void k_groups(int n, Tree T, int gmax, int dim, const float * qscale,
-  const unsigned long long * rbits) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n)
-    return;
-  int g = ~i;
-  int p = T.leaf_parent[i];
-  while(p >= 0 && T.last[p] - T.first[p] + 1 <= gmax) {
-    g = p;
-    p = T.parent[p];
-  }
-  int f = g < 0 ? i : T.first[g];
-  int l = g < 0 ? i : T.last[g];
-  if(f == i) {
-    int slot = atomicAdd(T.ngroups, 1);
-    T.group_first[slot] = f;
-    T.group_last[slot] = l;
-    // (a one-particle group walks from the root)
-    int v = 0;
-    int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-    if(g >= 0) {
-      const int4 glo = T.qbox[2 * g], ghi = T.qbox[2 * g + 1];
-      const int gl[3] = {glo.x, glo.y, glo.z}, gh[3] = {ghi.x, ghi.y, ghi.z};
-      const float R = (float)ord_dec(rbits[7]) * 1.00001f;
-      for(int d = 0; d < dim; ++d) {
-        const int r = (int)ceilf(R / qscale[d]) + 2;
-        lo[d] = gl[d] - r;
-        hi[d] = gh[d] + r;
+    split = s;
+    // walk groups: maximal subtrees of at most gmax particles
+    if(r - l + 1 > gmax) {
+      for(int c = 0; c < 2; ++c) {
+        const int f = c ? s + 1 : l, e_ = c ? r : s;
+        if(e_ - f + 1 <= gmax) {
+          const int slot = atomicAdd(T.ngroups, 1);
+          T.group_first[slot] = f;
+          T.group_last[slot] = e_;
+          T.group_node[slot] = f == e_ ? -1 : s + c;
+        }
       }
-      v = T.parent[g];
     }
-    while(v > 0) {
-      const int4 a = T.qbox[2 * v], b = T.qbox[2 * v + 1];
-      const int al[3] = {a.x, a.y, a.z}, bh[3] = {b.x, b.y, b.z};
-      bool in = true;
-      for(int d = 0; d < dim; ++d)
-        in = in && al[d] + 1 <= lo[d] && bh[d] - 1 >= hi[d];
-      if(in)
-        break;
-      v = T.parent[v];
-    }
-    T.group_start[slot] = v < 0 ? 0 : v;
   }
 }
 
@@ -1255,31 +1164,96 @@ __global__ void k_refgroups(const unsigned long long * K, int n, int dim,
   T.gref[i] = g;
 }
 
+// The node a group's mixed walk starts from: the lowest ancestor whose
+// fixed-point box, less one step on every side, holds the group's box grown
+// by the largest reach (max h, with the walk's 1e-5 slack and two steps for
+// the quantisation).  A radix-tree node holds every particle whose key
+// shares its prefix, so its particles' box lies in that Morton cell; a
+// particle within reach lies in the grown box, hence a step inside the
+// node's box, hence in the cell and in the subtree: the walk below that
+// node finds every candidate the walk from the root finds.  (A one-particle
+// group, node -1, walks from the root.)
+__device__ __forceinline__ int walk_start(const Tree & T, int g, const int4 & glo,
+  const int4 & ghi, float hmax, float qs0, float qs1, float qs2, int dim) {
+  if(g < 0)
+    return 0;
+  const float R = hmax * 1.00001f;
+  const int rx = (int)ceilf(R / qs0) + 2, ry = (int)ceilf(R / qs1) + 2;
+  const int rz = dim == 3 ? (int)ceilf(R / qs2) + 2 : 0;
+  int v = T.parent[g];
+  while(v > 0) {
+    const int4 a = T.qbox[2 * v], b = T.qbox[2 * v + 1];
+    bool in = a.x + 1 <= glo.x - rx && b.x - 1 >= ghi.x + rx && a.y + 1 <= glo.y - ry &&
+              b.y - 1 >= ghi.y + ry;
+    if(dim == 3)
+      in = in && a.z + 1 <= glo.z - rz && b.z - 1 >= ghi.z + rz;
+    if(in)
+      break;
+    v = T.parent[v];
+  }
+  return v < 0 ? 0 : v;
+}
+
+// walk_start of every group by a launch of its own, where there are many: in
+// the walk its chain of dependent loads (two a level) holds a whole warp, 40 us
+// of the Sedov 128^3 walk more than this launch; at 2,250 to 132,651 particles
+// the launch costs the 7 to 12 us that it does not save.
+#define WALK_START_LAUNCH (1 << 18)
+__global__ void __launch_bounds__(256) k_walk_start(Tree T, int dim, const float * qscale,
+  const unsigned long long * rbits) {
+  const int ng = *T.ngroups;
+  const float hmax = (float)ord_dec(rbits[7]);
+  const float qs0 = qscale[0], qs1 = qscale[1], qs2 = dim == 3 ? qscale[2] : 0.f;
+  for(int g = blockIdx.x * 256 + threadIdx.x; g < ng; g += gridDim.x * 256) {
+    const int v = T.group_node[g];
+    T.group_node[g] = v < 0 ? 0
+      : walk_start(T, v, T.qbox[2 * v], T.qbox[2 * v + 1], hmax, qs0, qs1, qs2, dim);
+  }
+}
+
 cudaError_t launch_build_tree(const Launch & L, const Particles & P,
   const PhysParams & pp, Tree & T, int group_max,
-  const unsigned long long * rbits, const int4 * qpos, const float * qscale,
-  int ordered) {
+  const unsigned long long * rbits, const int4 * qpos, const float * qscale, int ordered,
+  DevStatus * st) {
+  static std::atomic<unsigned long long> attr_devices{0};
+  cudaError_t ae = once_per_device(&attr_devices, []() {
+    cudaError_t e = cudaFuncSetAttribute(k_tree<3, true>,
+      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<true>());
+    if(e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_tree<2, true>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<true>());
+    return e;
+  });
+  if(ae != cudaSuccess)
+    return ae;
   const int n = P.n;
-  cudaMemsetAsync(T.counter, 0, sizeof(unsigned) * (size_t)n, L.stream);
-  cudaMemsetAsync(T.ngroups, 0, sizeof(int), L.stream);
-  k_karras<<<(n + 254) / 256, 256, 0, L.stream>>>(P.key, n, T);
-  if(ordered)  // reference octree depths order the FP64 lists
-    k_edepth<<<(n + 255) / 256, 256, 0, L.stream>>>(P.key, n, pp.dim, T.edepth);
-  const int nbb = (n + BOUNDS_THREADS - 1) / BOUNDS_THREADS;
-  const size_t bsm = bounds_smem(T.gmom != nullptr);
+  const int nb = (n + TREE_THREADS - 1) / TREE_THREADS;
+#define TREE_LAUNCH(DIM, ALL)                                                \
+  k_tree<DIM, ALL><<<nb, TREE_THREADS, tree_smem<ALL>(), L.stream>>>(P.key, P, T, qpos, \
+    rbits, ordered, group_max, st)
+  // in the ordered mode and with gravity every run is ALL; else the range
+  // words on the device tell
+  const bool full_only = ordered || T.gmom;
   if(pp.dim == 3) {
-    k_bounds_chain<3><<<nbb, BOUNDS_THREADS, bsm, L.stream>>>(P, T, qpos, rbits, ordered);
-    k_bounds_rounds<3><<<nbb, BOUNDS_THREADS, bsm, L.stream>>>(P, T, qpos, rbits, ordered);
+    if(!full_only)
+      TREE_LAUNCH(3, false);
+    TREE_LAUNCH(3, true);
   }
   else {
-    k_bounds_chain<2><<<nbb, BOUNDS_THREADS, bsm, L.stream>>>(P, T, qpos, rbits, ordered);
-    k_bounds_rounds<2><<<nbb, BOUNDS_THREADS, bsm, L.stream>>>(P, T, qpos, rbits, ordered);
+    if(!full_only)
+      TREE_LAUNCH(2, false);
+    TREE_LAUNCH(2, true);
   }
-  k_groups<<<(n + 255) / 256, 256, 0, L.stream>>>(n, T, group_max, pp.dim, qscale,
-    rbits);
+#undef TREE_LAUNCH
   k_refgroups<<<(n + 255) / 256, 256, 0, L.stream>>>(P.key, n, pp.dim, T, rbits,
     ordered);
-  *L.counter += ordered ? 6 : 5;
+  *L.counter += full_only ? 2 : 3;
+  if(!ordered && n >= WALK_START_LAUNCH) {
+    const int most = (n + 255) / 256;
+    k_walk_start<<<most < 152 * 8 ? most : 152 * 8, 256, 0, L.stream>>>(T, pp.dim, qscale,
+      rbits);
+    *L.counter += 1;
+  }
   return cudaGetLastError();
 }
 
@@ -1579,7 +1553,7 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
     float4 fglo = make_float4(0.f, 0.f, 0.f, 0.f), fghi = fglo;
     float cax = 0.f, cay = 0.f, caz = 0.f;
     // the reference's group and boxes exist with varying h, and in the
-    // ordered mode (k_bounds_rounds, k_refgroups)
+    // ordered mode (k_tree, k_refgroups)
     if(mem && (nonuni || ORDERED)) {
       gnode = T.gref[a];
       if(gnode >= 0) {
@@ -1610,8 +1584,14 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
     int ncand = 0;
     bool chunked = false;
     bool refdone = false;  // varying h: this lane's list is already filtered
+    int start = 0;
+    if(!ORDERED) {
+      start = T.group_node[g];
+      if(P.n < WALK_START_LAUNCH)
+        start = walk_start(T, start, glo, ghi, hglob, qs0, qs1, qs2, dim);
+    }
     if(lane == 0)
-      stack[0] = ORDERED ? 0 : T.qbox[2 * T.group_start[g] + 1].w;
+      stack[0] = ORDERED ? 0 : T.qbox[2 * start + 1].w;
     __syncwarp();
     while(sp > 0) {
       const int k = sp < 32 ? sp : 32;
