@@ -1405,40 +1405,40 @@ __device__ __forceinline__ int sphere_box_f(const float4 & lo,
 // separation along an axis ties with h to rounding.  Each
 // test is decided in FP32 first and in FP64 (box_box, sphere_box) only when
 // the FP32 answer is not certain, so the answers are the FP64 ones.
-__device__ bool ref_node_tests_mixed(const Tree & T, const double * X,
-  const double * Y, const double * Z, const double * H, int dim, int b, int a,
-  double xa, double ya, double za, double ha, float cax, float cay, float caz,
-  float haf, int gnode, const double * g2, const float4 & glo,
-  const float4 & ghi, const double * rlo, float tol) {
+//
+// The box-box half depends on G and b's octree parent alone: the walk asks it
+// once per candidate and traversal group, a lane per candidate.
+__device__ __forceinline__ bool ref_box_test(const Tree & T, int dim, int ob, int gnode,
+  const float4 & glo, const float4 & ghi, float tol) {
+  const int r = box_box_f(T.fbox2[2 * ob], T.fbox2[2 * ob + 1], glo, ghi, dim, tol);
+  if(r >= 0)
+    return r != 0;
+  const double * b2 = (const double *)&T.box2[ob];
+  const double * g2 = (const double *)&T.box2[gnode];
+  double bb[8], gg[8];
+  for(int k = 0; k < 8; ++k) {
+    bb[k] = b2[k];
+    gg[k] = g2[k];
+  }
+  return box_box(bb, gg, dim);
+}
+
+// The sphere-box half for the pair (a, b).  Particle a's own sphere passes
+// whenever d(a, b) <= max(h_a, h_b) and h_b <= 2 h_a: the parent's box holds
+// the cube of half-width h_b / 2 about b, hence the ball of that radius, so it
+// is no farther from a than d - h_b / 2 <= max(h_a - h_b / 2, h_b / 2).  The
+// caller skips the test for h_b <= 1.99 h_a, which leaves rounding its room.
+__device__ bool ref_sphere_test(const Tree & T, const double * X, const double * Y,
+  const double * Z, const double * H, int dim, int b, int a, int gnode, const double * rlo,
+  float tol) {
   const int ob = T.opar[b];
   const float4 blo = T.fbox2[2 * ob], bhi = T.fbox2[2 * ob + 1];
   const double * b2 = (const double *)&T.box2[ob];
-  if(gnode >= 0) {
-    const int r = box_box_f(blo, bhi, glo, ghi, dim, tol);
-    if(r == 0)
-      return false;
-    if(r < 0) {
-      double bb[8];
-      for(int k = 0; k < 8; ++k)
-        bb[k] = b2[k];
-      if(!box_box(bb, g2, dim))
-        return false;
-    }
-  }
-  const int s = sphere_box_f(blo, bhi, cax, cay, caz, haf, dim, tol);
-  if(s == 1)
-    return true;
-  if(s < 0) {
-    double bb[8];
-    for(int k = 0; k < 8; ++k)
-      bb[k] = b2[k];
-    if(sphere_box(bb, xa, ya, za, ha, dim))
-      return true;
-  }
-  if(gnode < 0)
-    return false;
-  for(int k = T.first[gnode]; k <= T.last[gnode]; ++k) {
-    if(k == a)
+  const int first = gnode < 0 ? a : T.first[gnode], last = gnode < 0 ? a : T.last[gnode];
+  // a first: the likeliest, and the only one where G is a single particle
+  for(int j = first - 1; j <= last; ++j) {
+    const int k = j < first ? a : j;
+    if(j >= first && k == a)
       continue;
     const double xk = X[k], yk = Y[k], zk = dim == 3 ? Z[k] : 0.0, hk = H[k];
     const int t = sphere_box_f(blo, bhi, (float)(xk - rlo[0]), (float)(yk - rlo[1]),
@@ -1454,6 +1454,16 @@ __device__ bool ref_node_tests_mixed(const Tree & T, const double * X,
     }
   }
   return false;
+}
+
+// both halves (equal-h ties in the ordered mode, groups of many classes)
+__device__ bool ref_node_tests(const Tree & T, const double * X, const double * Y,
+  const double * Z, const double * H, int dim, int b, int a, int gnode, const double * rlo,
+  float tol) {
+  if(gnode >= 0 && !ref_box_test(T, dim, T.opar[b], gnode, T.fbox2[2 * gnode],
+                     T.fbox2[2 * gnode + 1], tol))
+    return false;
+  return ref_sphere_test(T, X, Y, Z, H, dim, b, a, gnode, rlo, tol);
 }
 
 // Conservative pruning test in the fixed-point space: the separation of
@@ -1502,12 +1512,15 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
   float * cxs = nullptr;  // candidates as SoA: minus their position relative
   float * cys = nullptr;  // to the group box corner, h and particle index,
   float * czs = nullptr;  // so the filter reads consecutive pairs as float2
-  float * chs = nullptr;
+  float * chs = nullptr;  // (h squared)
   int * cidx = nullptr;
+  unsigned char * cflag = nullptr;  // bit k: passes class k's box-box test (varying h)
   int * stack;
   if(ORDERED) {
     ckey = (unsigned long long *)smem + (size_t)w * NB_CAND_ORDERED;
     stack = (int *)(smem + (size_t)NB_WARPS * NB_CAND_ORDERED * 8) + w * NB_STACK;
+    cflag = smem + (size_t)NB_WARPS * (NB_CAND_ORDERED * 8 + NB_STACK * 4) +
+            (size_t)w * NB_CAND_ORDERED;
   }
   else {
     constexpr int NA = UNI ? 4 : 5;  // arrays per candidate (no h with UNI)
@@ -1518,6 +1531,8 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
     chs = UNI ? nullptr : base + 3 * CAND;
     cidx = (int *)(base + (NA - 1) * CAND);
     stack = (int *)(smem + (size_t)NB_WARPS * CAND * NA * 4) + w * NB_STACK;
+    if(!UNI)
+      cflag = smem + (size_t)NB_WARPS * (CAND * NA * 4 + NB_STACK * 4) + (size_t)w * CAND;
   }
   const unsigned lt = lanemask_lt();
   const double * X = P.f[F_X];
@@ -1548,24 +1563,24 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
     if(mem)
       qa = K.qpos[a];
     const float haf = __int_as_float(qa.w);
-    int gnode = -1;
-    double g2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    float4 fglo = make_float4(0.f, 0.f, 0.f, 0.f), fghi = fglo;
-    float cax = 0.f, cay = 0.f, caz = 0.f;
-    // the reference's group and boxes exist with varying h, and in the
-    // ordered mode (k_tree, k_refgroups)
-    if(mem && (nonuni || ORDERED)) {
-      gnode = T.gref[a];
-      if(gnode >= 0) {
-        const double * gp = (const double *)&T.box2[gnode];
-        for(int k = 0; k < 8; ++k)
-          g2[k] = gp[k];
-        fglo = T.fbox2[2 * gnode];
-        fghi = T.fbox2[2 * gnode + 1];
+    // the members' traversal groups (they exist with varying h, and in the
+    // ordered mode: k_tree, k_refgroups), told apart as up to eight classes:
+    // lane k holds class k's node, every member its class
+    int gnode = -1, cls = 0, cnode = -1, ncls = 0;
+    if(!UNI && (nonuni || ORDERED)) {
+      if(mem)
+        gnode = max(T.gref[a], -1);
+      unsigned left = nonuni ? __ballot_sync(FULL, mem) : 0u;
+      while(left) {
+        const int node = __shfl_sync(FULL, gnode, __ffs(left) - 1);
+        const unsigned same = __ballot_sync(FULL, mem && gnode == node) & left;
+        if((same >> lane) & 1u)
+          cls = ncls;
+        if(lane == ncls)
+          cnode = node;
+        left &= ~same;
+        ++ncls;
       }
-      cax = (float)(X[a] - rlo[0]);
-      cay = (float)(Y[a] - rlo[1]);
-      caz = dim == 3 ? (float)(Z[a] - rlo[2]) : 0.f;
     }
     int4 glo = mem ? qa : make_int4(0x7fffffff, 0x7fffffff, 0x7fffffff, 0);
     int4 ghi = mem ? qa : make_int4(-1, -1, -1, 0);
@@ -1583,7 +1598,6 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
     int sp = 1;
     int ncand = 0;
     bool chunked = false;
-    bool refdone = false;  // varying h: this lane's list is already filtered
     int start = 0;
     if(!ORDERED) {
       start = T.group_node[g];
@@ -1656,7 +1670,7 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
             cys[pos] = -((float)(ql.y - glo.y) * qs1);
             czs[pos] = -((float)(ql.z - glo.z) * qs2);
             if(!UNI)
-              chs[pos] = __int_as_float(ql.w);
+              chs[pos] = __int_as_float(ql.w) * __int_as_float(ql.w);
             cidx[pos] = ~cc[c];
           }
         }
@@ -1707,18 +1721,48 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
           chunked = true;
         if(ORDERED)
           warp_bitonic(ckey, ncand, lane);
-        if(!ORDERED && (ncand & 1)) {
-          // pad to an even count with a candidate that can never pass
-          if(lane == 0) {
-            cxs[ncand] = 1e30f;
-            cys[ncand] = 1e30f;
-            czs[ncand] = 1e30f;
+        float rc = hg;  // varying h: the largest h among members and candidates
+        if(!ORDERED) {
+          // an even count (UNI) or whole batches of 32, with candidates that
+          // can never pass
+          const int full = UNI ? (ncand + 1) & ~1 : (ncand + 31) & ~31;
+          for(int c = ncand + lane; c < full; c += 32) {
+            cxs[c] = 1e30f;
+            cys[c] = 1e30f;
+            czs[c] = 1e30f;
             if(!UNI)
-              chs[ncand] = 0.f;
-            cidx[ncand] = -1;
+              chs[c] = 0.f;
+            cidx[c] = -1;
+          }
+        }
+        if(!UNI && nonuni) {
+          if(!ORDERED) {
+            float hc = 0.f;
+            for(int c = lane; c < ncand; c += 32)
+              hc = fmaxf(hc, chs[c]);
+            for(int o = 16; o; o >>= 1)
+              hc = fmaxf(hc, __shfl_xor_sync(FULL, hc, o));
+            rc = fmaxf(rc, sqrtf(hc) * 1.000001f);
+          }
+          // the reference's box-box test, a lane per candidate, for every class
+          // of members (the classes beyond the eighth test their own pairs)
+          for(int k = 0; k < ncls && k < 8; ++k) {
+            const int node = __shfl_sync(FULL, cnode, k);
+            float4 nlo = make_float4(0.f, 0.f, 0.f, 0.f), nhi = nlo;
+            if(node >= 0) {
+              nlo = T.fbox2[2 * node];
+              nhi = T.fbox2[2 * node + 1];
+            }
+            for(int c = lane; c < ncand; c += 32) {
+              const int bc = ORDERED ? (int)(ckey[c] & 0xffffffffu) : cidx[c];
+              const bool ok =
+                node < 0 || ref_box_test(T, dim, T.opar[bc], node, nlo, nhi, ftol);
+              cflag[c] = (unsigned char)((k ? cflag[c] : 0u) | ((unsigned)ok << k));
+            }
           }
           __syncwarp();
         }
+        __syncwarp();
         if(mem) {
           const double xa = X[a], ya = Y[a], za = dim == 3 ? Z[a] : 0.0, ha = H[a];
           int * out = Ls.idx + list_slot(a, 0, maxnb);
@@ -1749,14 +1793,17 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
             double r = ha < hbd ? hbd : ha;
             return d2 <= r * r;
           };
-          // The reference's node tests (varying h) run after the walk over
-          // each lane's whole list, where every lane of the warp has work;
-          // a list that fills up before then is filtered on the spot and
-          // the lane tests the rest as they come, so the capacity counts the
-          // same pairs as the reference's list.
-          auto refok = [&](int b) {
-            return ref_node_tests_mixed(T, X, Y, Z, H, dim, b, a, xa, ya, za, ha,
-              cax, cay, caz, haf, gnode, g2, fglo, fghi, rlo, ftol);
+          // what the reference's node tests keep of the pairs within reach
+          // (varying h): class flag, and the sphere test where h_b is far
+          // above h_a or h is so small beside the range that rounding counts
+          const bool hsmall = haf < 1e-6f * ext;
+          auto refok = [&](int c, int b, float hb) {
+            if(cls >= 8)
+              return ref_node_tests(T, X, Y, Z, H, dim, b, a, gnode, rlo, ftol);
+            if(!((cflag[c] >> cls) & 1u))
+              return false;
+            return (!hsmall && hb <= 1.99f * haf) ||
+                   ref_sphere_test(T, X, Y, Z, H, dim, b, a, gnode, rlo, ftol);
           };
           // Equal h: the node tests can only drop a pair whose separation
           // along some axis ties with h, where the rounding of x +- h/2 in
@@ -1768,20 +1815,6 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
             return fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) >= rf - kq;
           };
           auto append = [&](int b) {
-            if(nonuni && !refdone && cnt == maxnb) {
-              int kept = 0;
-              for(int j = 0; j < cnt; ++j) {
-                const int e = out[slot_off(j)];
-                if(refok(e)) {
-                  out[slot_off(kept)] = e;
-                  ++kept;
-                }
-              }
-              cnt = kept;
-              refdone = true;
-            }
-            if(nonuni && refdone && !refok(b))
-              return;
             if(cnt < maxnb)
               out[slot_off(cnt)] = b;
             ++cnt;
@@ -1797,13 +1830,21 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
               const float rf = fmaxf(haf, __int_as_float(qb.w));
               const float t = d2f - rf * rf;
               const float mg = rf * (4e-5f * rf + kq);
-              if(decide(t, mg, b) && (nonuni || !tie(fx, fy, fz, rf) || refok(b)))
+              if(decide(t, mg, b) &&
+                 (nonuni ? refok(c, b, __int_as_float(qb.w))
+                         : !tie(fx, fy, fz, rf) ||
+                             ref_node_tests(T, X, Y, Z, H, dim, b, a, gnode, rlo, ftol)))
                 append(b);
             }
           }
           else if(UNI) {
             // every h is equal: r and the margin are constants of the group
-            // and the predicate decides (ties included, see tie)
+            // and the predicate decides (ties included, see tie); two
+            // candidates per step in packed FP32x2.  Collecting the accepted
+            // ones of 32 candidates in a mask first measured the same at Sedov
+            // 128^3 (1.47 ms) and slower on small sets (52 against 34 us at
+            // 2,250 particles in 2D): a batch of neighbours in space is hit
+            // as a whole, so its append loop is as long as the batch.
             const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay);
             const float2 az2 = make_float2(az, az);
             const float r2 = haf * haf;
@@ -1826,44 +1867,73 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
                 in0 = decide(t.x, mg, id.x);
               if(fabsf(t.y) <= mg && id.y >= 0)
                 in1 = decide(t.y, mg, id.y);
-              if(in0) {
-                if(cnt < maxnb)
-                  out[slot_off(cnt)] = id.x;
-                ++cnt;
-              }
-              if(in1) {
-                if(cnt < maxnb)
-                  out[slot_off(cnt)] = id.y;
-                ++cnt;
-              }
+              if(in0)
+                append(id.x);
+              if(in1)
+                append(id.y);
             }
           }
-          else if(!UNI) {
-            // two candidates per iteration with Blackwell's packed FP32x2
-            // arithmetic
+          else {
+            // Batches of 32 candidates: the sign bits of t = d^2 -
+            // max(h_a, h_b)^2 make a mask (a funnel shift per candidate), the
+            // smallest |t| beyond its margin tells whether a pair of the batch
+            // needs the exact predicate, and the set bits are appended.  Here
+            // an accepted pair has more to do (the class flag, h_b), so taking
+            // only those through the append loop pays: 5.1 against 7.4 ms
+            // candidate by candidate on the 4M star.
             const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay);
             const float2 az2 = make_float2(az, az);
-            const float2 eps2 = make_float2(4e-5f, 4e-5f), kq2 = make_float2(kq, kq);
-            for(int c = 0; c < ncand; c += 2) {
-              const float2 nx = *(const float2 *)&cxs[c];
-              const float2 ny = *(const float2 *)&cys[c];
-              const float2 nz = *(const float2 *)&czs[c];
-              const float2 hb = *(const float2 *)&chs[c];
-              const int2 id = *(const int2 *)&cidx[c];
-              const float2 dx = __fadd2_rn(ax2, nx);
-              const float2 dy = __fadd2_rn(ay2, ny);
-              const float2 dz = __fadd2_rn(az2, nz);
-              float2 d2 = __fmul2_rn(dx, dx);
-              d2 = __ffma2_rn(dy, dy, d2);
-              d2 = __ffma2_rn(dz, dz, d2);
-              const float2 rf = make_float2(fmaxf(haf, hb.x), fmaxf(haf, hb.y));
-              const float2 nrf = make_float2(-rf.x, -rf.y);
-              const float2 t = __ffma2_rn(rf, nrf, d2);
-              const float2 mg = __fmul2_rn(rf, __ffma2_rn(rf, eps2, kq2));
-              if(id.x >= 0 && decide(t.x, mg.x, id.x))
-                append(id.x);
-              if(id.y >= 0 && decide(t.y, mg.y, id.y))
-                append(id.y);
+            const float r2 = haf * haf, mgc = kq * rc;
+            for(int c0 = 0; c0 < ncand; c0 += 32) {
+              unsigned mask = 0u;
+              float slack = 1e38f;
+#pragma unroll 2
+              for(int c = c0; c < c0 + 32; c += 4) {
+                const float4 nx = *(const float4 *)&cxs[c];
+                const float4 ny = *(const float4 *)&cys[c];
+                const float4 nz = *(const float4 *)&czs[c];
+                const float4 hb2 = *(const float4 *)&chs[c];
+                const float hh[4] = {hb2.x, hb2.y, hb2.z, hb2.w};
+                float t[4];
+                for(int q = 0; q < 2; ++q) {
+                  const float2 dx = __fadd2_rn(ax2, q ? make_float2(nx.z, nx.w)
+                                                      : make_float2(nx.x, nx.y));
+                  const float2 dy = __fadd2_rn(ay2, q ? make_float2(ny.z, ny.w)
+                                                      : make_float2(ny.x, ny.y));
+                  const float2 dz = __fadd2_rn(az2, q ? make_float2(nz.z, nz.w)
+                                                      : make_float2(nz.x, nz.y));
+                  float2 d2 = __fmul2_rn(dx, dx);
+                  d2 = __ffma2_rn(dy, dy, d2);
+                  d2 = __ffma2_rn(dz, dz, d2);
+                  t[2 * q] = d2.x;
+                  t[2 * q + 1] = d2.y;
+                }
+                for(int q = 0; q < 4; ++q) {
+                  // margin 4e-5 r^2 + kq r, r at most rc
+                  const float rr = fmaxf(r2, hh[q]);
+                  t[q] -= rr;
+                  slack = fminf(slack, __fmaf_rn(-4e-5f, rr, fabsf(t[q])));
+                  mask = __funnelshift_l(__float_as_uint(t[q]), mask, 1);
+                }
+              }
+              if(slack <= mgc) {
+                // some pair lies inside the margin: candidate by candidate
+                mask = 0u;
+                for(int c = c0; c < c0 + 32 && c < ncand; ++c) {
+                  const float dx = ax + cxs[c], dy = ay + cys[c], dz = az + czs[c];
+                  const float rf = fmaxf(haf, sqrtf(chs[c]));
+                  const float t = dx * dx + dy * dy + dz * dz - rf * rf;
+                  if(decide(t, rf * (4.1e-5f * rf + kq), cidx[c]))
+                    mask |= 0x80000000u >> (c - c0);
+                }
+              }
+              while(mask) {
+                const int k = __clz(mask);
+                mask &= ~(0x80000000u >> k);
+                const int b = cidx[c0 + k];
+                if(refok(c0 + k, b, sqrtf(chs[c0 + k])))
+                  append(b);
+              }
             }
           }
         }
@@ -1876,22 +1946,6 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
         if(atomicCAS(&st->code, 0, (int)FSPH_ERR_LIST_OVERFLOW) == 0)
           st->index = a;
         cnt = maxnb;
-      }
-      if(nonuni && !refdone) {
-        // drop the pairs the reference's node tests drop; the list keeps
-        // its order
-        const double xa = X[a], ya = Y[a], za = dim == 3 ? Z[a] : 0.0, ha = H[a];
-        int * o = Ls.idx + list_slot(a, 0, maxnb);
-        int kept = 0;
-        for(int j = 0; j < cnt; ++j) {
-          const int b = o[slot_off(j)];
-          if(ref_node_tests_mixed(T, X, Y, Z, H, dim, b, a, xa, ya, za, ha, cax,
-               cay, caz, haf, gnode, g2, fglo, fghi, rlo, ftol)) {
-            o[slot_off(kept)] = b;
-            ++kept;
-          }
-        }
-        cnt = kept;
       }
       Ls.cnt[a] = cnt;
       {
@@ -1929,9 +1983,9 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
 cudaError_t launch_neighbors(const Launch & L, const Particles & P,
   const PhysParams & pp, const Tree & T, Lists & Ls, DevStatus * st, int nsm,
   const unsigned long long * rbits, const Packed & K, int ordered) {
-  const size_t smem_o = (size_t)NB_WARPS * NB_CAND_ORDERED * 8 +
+  const size_t smem_o = (size_t)NB_WARPS * NB_CAND_ORDERED * 9 +
                         (size_t)NB_WARPS * NB_STACK * 4;
-  const size_t smem_v = (size_t)NB_WARPS * NB_CAND * 20 +
+  const size_t smem_v = (size_t)NB_WARPS * NB_CAND * 21 +
                         (size_t)NB_WARPS * NB_STACK * 4;
   const size_t smem_u = (size_t)NB_WARPS * NB_UNI_CAND * 16 +
                         (size_t)NB_WARPS * NB_STACK * 4;
