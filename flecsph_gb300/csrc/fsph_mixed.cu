@@ -158,8 +158,7 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
 cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
   const PhysParams & pp, const unsigned long long * rbits, const Packed & K,
   int * ngroups) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
-  k_pack_pos<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups);
+  k_pack_pos<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -204,14 +203,13 @@ __global__ void __launch_bounds__(MIX_THREADS) k_vsig_mixed(Particles P,
 cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm, int vel_current) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
   // velocities of this step for the signal speed (unless the permute of
   // update_iteration wrote them); masses for the FP32 density pass (the
   // float-float one reads them from the position packing)
   const int what = wendland_kernel(pp.kernel) ? (vel_current ? 0 : PACK_VEL)
                                               : PACK_VHM | PACK_VEL;
   if(what) {
-    k_pack_state<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
   if(pp.cullen)
@@ -223,10 +221,9 @@ cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
 
 cudaError_t launch_alpha_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
   // current velocities and masses; sound speeds and div v signs of the
   // neighbours
-  k_pack_state<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, K,
+  k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K,
     PACK_VHM | PACK_VEL_V | PACK_AV_IN);
   *L.counter += 1;
   run_alpha_mixed(L, P, pp, Ls, K, t);
@@ -247,7 +244,6 @@ cudaError_t launch_vsig_mixed(const Launch & L, const Particles & P,
 cudaError_t launch_accel_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,
   const DevTime * t, int fused_vsig, int fv_current) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
   // v_half of this step (set by the caller's save_velocityhalf); the thermo
   // records are refreshed unless they come straight from the density pass
   // (fused signal speed needs their previous-sound-speed slot)
@@ -255,7 +251,7 @@ cudaError_t launch_accel_mixed(const Launch & L, const Particles & P,
   const int vh = wendland_kernel(pp.kernel) ? (fv_current ? 0 : PACK_FV) : PACK_VHM;
   const int what = (fused_vsig ? vh : (vh | PACK_THERMO)) | av;
   if(what) {
-    k_pack_state<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
   if(pp.cullen)
@@ -268,11 +264,10 @@ cudaError_t launch_accel_mixed(const Launch & L, const Particles & P,
 cudaError_t launch_dudt_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t,
   int then_op, int fv_current, int fdv_current) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
   const int what = (fv_current ? 0 : PACK_FV) | (fdv_current ? 0 : PACK_FDV) |
                    (pp.cullen ? PACK_AV : 0);
   if(what) {
-    k_pack_state<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
   if(pp.cullen)
@@ -285,7 +280,6 @@ cudaError_t launch_dudt_mixed(const Launch & L, const Particles & P,
 cudaError_t launch_dedt_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,
   const DevTime * t, DevStatus * st, int use_ahyd, int fdv_current) {
-  const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
   // through a^P, v_half, rho and c_s are those the acceleration pass packed
   // (the caller's flag says so): only v - v_half is new, and not even that
   // when the acceleration pass's kick wrote it
@@ -293,7 +287,7 @@ cudaError_t launch_dedt_mixed(const Launch & L, const Particles & P,
                       ? (fdv_current ? 0 : PACK_FDV) : PACK_VHM | PACK_DEDT) |
                    (pp.cullen ? PACK_AV : 0);
   if(what) {
-    k_pack_state<<<nb, MIX_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
   if(pp.cullen)

@@ -29,7 +29,22 @@
 
 namespace fsph {
 
-#define MIX_THREADS 256
+// Threads per block of the pair passes; MIX_BLOCKS(b): how many blocks of t
+// threads hold as many as b blocks of 256 (the occupancies below are given in
+// those).  The float-float density and acceleration passes, bound by
+// arithmetic, run best in blocks of 128 (a shorter last wave: Sedov 51^3
+// density 84 -> 78 us, acceleration 149 -> 138; 128^3 0.92 -> 0.90, 1.90 ->
+// 1.89 ms); the energy passes, bound by their gathers through the L1, gain
+// from more warps of neighbouring particles on one SM (Sedov 128^3 de/dt: 64
+// threads 1.16 ms, 128 1.11, 256 1.07).
+#ifndef MIX_THREADS
+#define MIX_THREADS 128
+#endif
+#ifndef ENERGY_THREADS
+#define ENERGY_THREADS 256
+#endif
+#define MIX_BLOCKS(b, t) ((b) * 256 / (t))
+#define PACK_THREADS 256
 #define FPI 3.14159265358979323846f
 
 __device__ __forceinline__ void kahan(float & sum, float & comp, float term) {
@@ -215,6 +230,22 @@ struct PairGeom {
   float dx, dy, dz, r2;
 };
 
+// A list's chunks of four slots, read one chunk ahead: the neighbours' records
+// hang on the indices, so the index load (from L2 or HBM) would otherwise sit
+// in front of every chunk's gathers.
+struct ListChunks {
+  const int * lp;
+  int4 ahead;
+  __device__ __forceinline__ explicit ListChunks(const int * p)
+    : lp(p), ahead(*(const int4 *)p) {}
+  __device__ __forceinline__ int4 next(int j0, int cnt) {
+    const int4 q = ahead;
+    if(j0 + 4 < cnt)
+      ahead = *(const int4 *)(lp + ((j0 + 4) << 5));
+    return q;
+  }
+};
+
 // (vh_a - vh_b) . d from the high words (fv1) and low words (fv2) of
 // v_half: the high-word and low-word differences are one rounding each, so
 // the difference keeps ~2^-24 of itself
@@ -273,9 +304,10 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
       pa[d] = P.f[F_X + d][a];
     h_a = P.f[F_H][a];
   }
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
     // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -344,7 +376,7 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
 // Three blocks of 256 per SM (<= 85 registers): the pass waits on neighbour
 // gathers, and 24 warps hide more of them than 16.
 template<int D, int K, bool VSIG, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS, 3) k_accel_mixed(Particles P,
+__global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_accel_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
@@ -365,9 +397,10 @@ __global__ void __launch_bounds__(MIX_THREADS, 3) k_accel_mixed(Particles P,
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
   // The self pair and coincident pairs add exactly zero (x_ab = 0, mu = 0),
   // as the reference's m_b = 0 makes them; the loop needs no branch.
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
     // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -437,7 +470,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 3) k_accel_mixed(Particles P,
 #endif
 
 template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dudt_mixed(Particles P,
+__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dudt_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, const DevTime * tm, int then_op) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
@@ -456,9 +489,10 @@ __global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dudt_mixed(
   const int cnt = Ls.cnt[a];
   float dp = 0.f, cp = 0.f, dv = 0.f, cv = 0.f;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
     // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -501,7 +535,7 @@ __global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dudt_mixed(
 // right away: it reads only the particle's own fields, and the pass reads
 // the neighbours' P and c_s from the packed records, not the fields.
 template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS, 4) k_dedt_mixed(Particles P,
+__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(4, ENERGY_THREADS)) k_dedt_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -518,9 +552,10 @@ __global__ void __launch_bounds__(MIX_THREADS, 4) k_dedt_mixed(Particles P,
   const int cnt = Ls.cnt[a];
   float sum = 0.f, comp = 0.f;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
     // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -715,8 +750,9 @@ __device__ __forceinline__ ffloat density_ff_sum(const Packed & Kp, const int * 
   int cnt, const float4 & pa, const float4 & la, const ffloat & iha,
   const ffloat & ihDa) {
   ffloat sum = ff_make(0.f, 0.f);
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -759,8 +795,9 @@ __device__ __forceinline__ ffloat density_ff_sum2(const Packed & Kp, const int *
   const ffloat2 ih1 = ff2_bcast(iha);
   const float2 xa = f2s(pa.x), ya = f2s(pa.y), za = f2s(pa.z);
   const float2 xal = f2s(la.x), yal = f2s(la.y), zal = f2s(la.z);
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; u += 2) {
       const int b0 = u == 0 ? q4.x : q4.z, b1 = u == 0 ? q4.y : q4.w;
@@ -802,7 +839,7 @@ __device__ __forceinline__ ffloat density_ff_sum2(const Packed & Kp, const int *
 }
 
 template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS, 3) k_density_ff(Particles P,
+__global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_density_ff(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
   const DevTime * tm) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -931,8 +968,9 @@ __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
   ffloat sx = ff_make(0.f, 0.f), sy = sx, sz = sx;
   float vx = 0.f, vy = 0.f, vz = 0.f, cvx = 0.f, cvy = 0.f, cvz = 0.f;
   float vsig = 0.f;
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll(accel_ff_unroll)
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -1008,12 +1046,9 @@ __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
 #ifndef FSPH_ACCEL_FF_BLOCKS
 #define FSPH_ACCEL_FF_BLOCKS 2
 #endif
-#ifndef FSPH_ACCEL_FF_THREADS
-#define FSPH_ACCEL_FF_THREADS MIX_THREADS
-#endif
 
 template<int D, int K, bool VSIG, bool CULL>
-__global__ void __launch_bounds__(FSPH_ACCEL_FF_THREADS, FSPH_ACCEL_FF_BLOCKS) k_accel_ff(
+__global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(FSPH_ACCEL_FF_BLOCKS, MIX_THREADS)) k_accel_ff(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
@@ -1092,24 +1127,25 @@ __global__ void __launch_bounds__(FSPH_ACCEL_FF_THREADS, FSPH_ACCEL_FF_BLOCKS) k
 // positions, P/rho^2, v_half and alpha are those of the acceleration pass
 // (the caller tracks that).
 template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dedt_ahyd(Particles P,
+__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dedt_ahyd(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
-  const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
   const float alpha_a = CULL ? Kp.visc[a].x : 0.f;
   const int4 qa = Kp.qpos[a];
-  const float ha = __int_as_float(qa.w);
   const float4 h1a = Kp.fv1[a], h2a = Kp.fv2[a], dva = Kp.fdv[a];
   const float Aa = Kp.fmA[a].z;  // P_a / rho_a^2 (high word)
   const int cnt = Ls.cnt[a];
-  float sum = 0.f, comp = 0.f;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
+  const float ha = __int_as_float(qa.w);
+  float sum = 0.f, comp = 0.f;
+  ListChunks lc(lp);
   for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+    const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
@@ -1164,47 +1200,47 @@ __global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dedt_ahyd(P
 }
 
 // ------------------------------------------------------------ dispatch --
-#define MIX_DISPATCH(KERNEL_T, TA, ...)                                            \
+#define MIX_DISPATCH(THREADS, KERNEL_T, TA, ...)                                            \
   do {                                                                         \
-    const int nb_ = (P.n + MIX_THREADS - 1) / MIX_THREADS;                     \
+    const int nb_ = (P.n + THREADS - 1) / THREADS;                     \
     if(pp.dim == 3) {                                                          \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<3, FSPH_KERNEL_SINC, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SINC, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     else {                                                                     \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<2, FSPH_KERNEL_SINC, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SINC, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     *L.counter += 1;                                                           \
@@ -1215,24 +1251,24 @@ __global__ void __launch_bounds__(MIX_THREADS, FSPH_ENERGY_BLOCKS) k_dedt_ahyd(P
 // and smoothing kernel.
 // The float-float passes serve the Wendland kernels; the other kernels
 // (cubic and quintic splines, Gaussians, sinc) keep the FP32 passes.
-#define FF_DISPATCH(KERNEL_T, TA, ...)                                         \
+#define FF_DISPATCH(THREADS, KERNEL_T, TA, ...)                                         \
   do {                                                                         \
-    const int nb_ = (P.n + MIX_THREADS - 1) / MIX_THREADS;                     \
+    const int nb_ = (P.n + THREADS - 1) / THREADS;                     \
     if(pp.dim == 3) {                                                          \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
     }                                                                          \
     else {                                                                     \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, MIX_THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
     }                                                                          \
     *L.counter += 1;                                                           \
   } while(0)
@@ -1247,16 +1283,16 @@ inline void run_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm) {
   if(wendland_kernel(pp.kernel))
-    FF_DISPATCH(k_density_ff, CULL, P, pp, Ls, K, cs_new, st, tm);
+    FF_DISPATCH(MIX_THREADS, k_density_ff, CULL, P, pp, Ls, K, cs_new, st, tm);
   else
-    MIX_DISPATCH(k_density_mixed, CULL, P, pp, Ls, K, cs_new, st, tm);
+    MIX_DISPATCH(MIX_THREADS, k_density_mixed, CULL, P, pp, Ls, K, cs_new, st, tm);
 }
 
 template<bool CULL>
 inline void run_dudt_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t,
   int then_op) {
-  MIX_DISPATCH(k_dudt_mixed, CULL, P, pp, Ls, K, t, then_op);
+  MIX_DISPATCH(ENERGY_THREADS, k_dudt_mixed, CULL, P, pp, Ls, K, t, then_op);
 }
 
 template<bool CULL>
@@ -1264,16 +1300,16 @@ inline void run_dedt_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,
   const DevTime * t, DevStatus * st, int use_ahyd) {
   if(use_ahyd && wendland_kernel(pp.kernel))
-    FF_DISPATCH(k_dedt_ahyd, CULL, P, pp, Ls, K, then_op, t, st);
+    FF_DISPATCH(ENERGY_THREADS, k_dedt_ahyd, CULL, P, pp, Ls, K, then_op, t, st);
   else
-    MIX_DISPATCH(k_dedt_mixed, CULL, P, pp, Ls, K, then_op, t, st);
+    MIX_DISPATCH(ENERGY_THREADS, k_dedt_mixed, CULL, P, pp, Ls, K, then_op, t, st);
 }
 
 template<bool CULL>
 inline void run_accel_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,
   const DevTime * t, int fused_vsig) {
-  int threads = MIX_THREADS;
+  const int threads = MIX_THREADS;
   void (*fn)(Particles, PhysParams, Lists, Packed, int, const DevTime *) = nullptr;
 #define PICK(D, KK)                                                            \
   fn = fused_vsig ? k_accel_mixed<D, KK, true, CULL> : k_accel_mixed<D, KK, false, CULL>
@@ -1315,7 +1351,6 @@ inline void run_accel_mixed(const Launch & L, const Particles & P,
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4) PICK(2, FSPH_KERNEL_WENDLAND_C4);
       else PICK(2, FSPH_KERNEL_WENDLAND_C6);
     }
-    threads = FSPH_ACCEL_FF_THREADS;
   }
 #undef PICK
   fn<<<(P.n + threads - 1) / threads, threads, 0, L.stream>>>(P, pp, Ls, K, kick, t);
