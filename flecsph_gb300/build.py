@@ -19,12 +19,19 @@ LIB = os.path.join(HERE, "libfsph_gb300.so")
 DRIVER = os.path.join(HERE, "hydro_driver")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
+MIXED = ["-prec-div=false", "-prec-sqrt=false"]
+# file[:variant] -> flags
 SOURCES = {
     "fsph_tree.cu": ["-fmad=false"],
     "fsph_fp64.cu": ["-fmad=false"],
     "fsph_elementwise.cu": ["-fmad=false"],
-    "fsph_mixed.cu": ["-prec-div=false", "-prec-sqrt=false"],
-    "fsph_mixed_cullen.cu": ["-prec-div=false", "-prec-sqrt=false"],
+    "fsph_mixed.cu": MIXED,
+    "fsph_mixed_cullen.cu": MIXED,
+    # one object per viscosity and lane split (see the file)
+    "fsph_mixed_pairs.cu:00": MIXED + ["-DFSPH_PAIRS_CULLEN=0", "-DFSPH_PAIRS_SPLIT=0"],
+    "fsph_mixed_pairs.cu:01": MIXED + ["-DFSPH_PAIRS_CULLEN=0", "-DFSPH_PAIRS_SPLIT=1"],
+    "fsph_mixed_pairs.cu:10": MIXED + ["-DFSPH_PAIRS_CULLEN=1", "-DFSPH_PAIRS_SPLIT=0"],
+    "fsph_mixed_pairs.cu:11": MIXED + ["-DFSPH_PAIRS_CULLEN=1", "-DFSPH_PAIRS_SPLIT=1"],
     "fsph_gravity.cu": [],
     "fsph_periodic.cu": ["-fmad=false"],
     "fsph_peak.cu": [],
@@ -49,7 +56,8 @@ def _tuning_defines():
 
 
 def _compile(src, extra, verbose):
-    obj = os.path.join(BUILD, src.replace(".cu", ".o"))
+    src, _, variant = src.partition(":")
+    obj = os.path.join(BUILD, src.replace(".cu", variant + ".o"))
     cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
            "-Xptxas", "-v" if verbose else "-O3", *_tuning_defines(), *extra, "-c",
            os.path.join(CSRC, src), "-o", obj]
@@ -72,7 +80,7 @@ def _stale(objs):
 def build(force=False, verbose=False):
     """Compile every CUDA source and link the shared library (in-tree)."""
     os.makedirs(BUILD, exist_ok=True)
-    srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
+    srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s.partition(":")[0]))]
     if not force and not _stale(srcs):
         return LIB
     with cf.ThreadPoolExecutor(max_workers=len(srcs)) as ex:

@@ -527,6 +527,7 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   c->Ls.maxnb = (p->max_neighbors + 3) & ~3;  // whole chunks of four slots
   ok &= dalloc(c, &c->Ls.idx, Npad * (size_t)c->Ls.maxnb) == cudaSuccess;
   ok &= dalloc(c, &c->Ls.cnt, N) == cudaSuccess;
+  ok &= dalloc(c, &c->Ls.stat, 2) == cudaSuccess;
   ok &= dalloc(c, &c->d_time, 1) == cudaSuccess;
   ok &= dalloc(c, &c->d_status, 1) == cudaSuccess;
   ok &= dalloc(c, &c->d_cons, 8 * (1 + CONS_BLOCKS)) == cudaSuccess;
@@ -882,7 +883,8 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
   }
   {
     Phase ph(c, FSPH_TIMER_TREE);
-    CK(launch_pack_positions(L, c->P, c->pp, c->d_range, c->K, c->T.ngroups));
+    CK(launch_pack_positions(L, c->P, c->pp, c->d_range, c->K, c->T.ngroups,
+      c->Ls.stat));
     CK(launch_build_tree(L, c->P, c->pp, c->T,
       c->p.group_size > 0 ? c->p.group_size : GROUP_MAX, c->d_range, c->K.qpos,
       c->K.qscale, c->mixed ? 0 : 1, c->d_status));

@@ -172,6 +172,7 @@ struct GravBuffers {
   float4 * gpk;        // 2 n
 };
 
+#define LIST_STAT_MAX (1 << 18)
 // Neighbour lists, interleaved by warp in chunks of four slots:
 // [(i>>5)][slot/4][i&31][slot%4], so a lane reads four slots with one
 // 16-byte load and a warp reads 512 contiguous bytes.  maxnb is a multiple
@@ -181,6 +182,8 @@ struct GravBuffers {
 struct Lists {
   int * idx;
   int * cnt;
+  unsigned * stat;  // mixed path: longest list, all pairs (of runs whose pair
+                    // passes ask, up to LIST_STAT_MAX particles)
   int maxnb;
 };
 
@@ -253,9 +256,11 @@ cudaError_t launch_neighbors(const Launch & L, const Particles & P,
   const unsigned long long * rbits, const Packed & K, int ordered);
 
 // ---- fsph_mixed.cu ----
-// also empties the tree's group count for the build that follows
+// also empties the tree's group count and the list statistics for the build
+// that follows
 cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
-  const PhysParams & pp, const unsigned long long * rbits, const Packed & K, int * ngroups);
+  const PhysParams & pp, const unsigned long long * rbits, const Packed & K, int * ngroups,
+  unsigned * list_stat);
 cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm, int vel_current);

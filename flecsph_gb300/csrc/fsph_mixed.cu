@@ -1,13 +1,14 @@
 // fsph_mixed.cu -- the mixed-precision path: packing of the FP32 records,
 // the signal-speed pass, and the launchers of the pair kernels of
-// fsph_mixed_kernels.cuh (constant-alpha instances here, Cullen & Dehnen
-// instances in fsph_mixed_cullen.cu).
+// fsph_mixed_kernels.cuh (instances: fsph_mixed_pairs.cu).
 #include <cuda_runtime.h>
 
 #include "fsph_internal.cuh"
 #include "fsph_mixed_kernels.cuh"
 
 namespace fsph {
+
+static_assert(SPLIT_MAX <= LIST_STAT_MAX, "the walk keeps the statistics the passes read");
 
 __device__ __forceinline__ double ord_dec_m(unsigned long long u) {
   return (u & 0x8000000000000000ull)
@@ -17,7 +18,7 @@ __device__ __forceinline__ double ord_dec_m(unsigned long long u) {
 
 // ------------------------------------------------------------- packing --
 __global__ void k_pack_pos(Particles P, int dim,
-  const unsigned long long * rbits, Packed K, int * ngroups) {
+  const unsigned long long * rbits, Packed K, int * ngroups, unsigned * list_stat) {
   // Every position as one 48-bit fixed-point word per axis,
   //   F = round((x - lo) / E * 2^48),  E = the largest range extent
   //   enlarged by 2^-19 (so F < 2^48 - 2^28),
@@ -40,6 +41,7 @@ __global__ void k_pack_pos(Particles P, int dim,
     s_sc = s_iE * 0x1p48;
     if(blockIdx.x == 0) {
       *ngroups = 0;
+      list_stat[0] = list_stat[1] = 0u;
       K.fscale[0] = E;
       K.fscale[1] = s_iE;
       // h_min == h_max: the pair passes take h_ab = h_a throughout
@@ -157,8 +159,8 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
 
 cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
   const PhysParams & pp, const unsigned long long * rbits, const Packed & K,
-  int * ngroups) {
-  k_pack_pos<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups);
+  int * ngroups, unsigned * list_stat) {
+  k_pack_pos<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups, list_stat);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -167,10 +169,11 @@ cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
 // Same visiting-order rule as the FP64 pass: neighbours with a higher
 // sorted index contribute their new sound speed (thermo.z), the others the
 // previous one (thermo.w).
-template<int D>
-__global__ void __launch_bounds__(MIX_THREADS) k_vsig_mixed(Particles P,
-  Lists Ls, Packed Kp) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+template<int D, bool AUTO>
+__global__ void __launch_bounds__(MIX_THREADS) k_vsig_mixed(Particles P, Lists Ls,
+  Packed Kp) {
+  const bool split = four_lanes<AUTO>(Ls);
+  const int a = pass_particle<MIX_THREADS>(split);
   if(a >= P.n)
     return;
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
@@ -180,25 +183,49 @@ __global__ void __launch_bounds__(MIX_THREADS) k_vsig_mixed(Particles P,
   const int cnt = Ls.cnt[a];
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
   float vsig = 0.f;
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = *(const int4 *)(lp + (j0 << 5));
-#pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const PairGeom g = geom<D>(qa, Kp.qpos[b], s0, s1, s2);
-      const float4 vb = Kp.vel[b];
-      const float4 tb = Kp.thermo[b];
-      const float dotv = ((va.x - vb.x) * g.dx + (va.y - vb.y) * g.dy +
-                           (va.z - vb.z) * g.dz) * rsqrtf(g.r2);
-      const float cb = b > a ? tb.z : tb.w;
-      // the self pair and coincident pairs are NaN in the reference and drop out
-      const float cand = fmaxf(ca, cb) - fminf(dotv, 0.f);
-      vsig = fmaxf(vsig, (b != a && g.r2 > 0.f) ? cand : 0.f);
+  auto pair = [&](int b) {
+    const PairGeom g = geom<D>(qa, Kp.qpos[b], s0, s1, s2);
+    const float4 vb = Kp.vel[b];
+    const float4 tb = Kp.thermo[b];
+    const float dotv = ((va.x - vb.x) * g.dx + (va.y - vb.y) * g.dy +
+                         (va.z - vb.z) * g.dz) * rsqrtf(g.r2);
+    const float cb = b > a ? tb.z : tb.w;
+    // the self pair and coincident pairs are NaN in the reference and drop out
+    const float cand = fmaxf(ca, cb) - fminf(dotv, 0.f);
+    vsig = fmaxf(vsig, (b != a && g.r2 > 0.f) ? cand : 0.f);
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4)
+      pair(qc.next(j0, cnt));
+    vsig = fmaxf(vsig, __shfl_xor_sync(qc.mask, vsig, 1));
+    vsig = fmaxf(vsig, __shfl_xor_sync(qc.mask, vsig, 2));
+    if((threadIdx.x & 3) != 0)
+      return;
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      // four slots per 16-byte load; padding slots hold a itself
+      const int4 q4 = lc.next(j0, cnt);
+      pair(q4.x);
+      pair(q4.y);
+      pair(q4.z);
+      pair(q4.w);
     }
   }
   P.f[F_VSIG][a] = (double)vsig;
 }
+
+// a pair pass with the configured viscosity, with the choice of four lanes per
+// particle up to SPLIT_MAX particles
+#define PAIR_PASS(fn, ...)                                                     \
+  do {                                                                         \
+    if(pp.cullen)                                                              \
+      (P.n <= SPLIT_MAX ? fn##_mixed_cullen_split : fn##_mixed_cullen)(__VA_ARGS__); \
+    else                                                                       \
+      (P.n <= SPLIT_MAX ? fn##_mixed_split : fn##_mixed)(__VA_ARGS__);         \
+  } while(0)
 
 cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
@@ -212,10 +239,7 @@ cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
     k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
-  if(pp.cullen)
-    run_density_mixed_cullen(L, P, pp, Ls, K, cs_new, st, tm);
-  else
-    run_density_mixed<false>(L, P, pp, Ls, K, cs_new, st, tm);
+  PAIR_PASS(run_density, L, P, pp, Ls, K, cs_new, st, tm);
   return cudaGetLastError();
 }
 
@@ -233,10 +257,17 @@ cudaError_t launch_alpha_mixed(const Launch & L, const Particles & P,
 cudaError_t launch_vsig_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K) {
   const int nb = (P.n + MIX_THREADS - 1) / MIX_THREADS;
-  if(pp.dim == 3)
-    k_vsig_mixed<3><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+  const int ns = (P.n + MIX_THREADS / 4 - 1) / (MIX_THREADS / 4);
+  if(P.n <= SPLIT_MAX) {
+    if(pp.dim == 3)
+      k_vsig_mixed<3, true><<<ns, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+    else
+      k_vsig_mixed<2, true><<<ns, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+  }
+  else if(pp.dim == 3)
+    k_vsig_mixed<3, false><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
   else
-    k_vsig_mixed<2><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+    k_vsig_mixed<2, false><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -254,10 +285,7 @@ cudaError_t launch_accel_mixed(const Launch & L, const Particles & P,
     k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
-  if(pp.cullen)
-    run_accel_mixed_cullen(L, P, pp, Ls, K, kick, t, fused_vsig);
-  else
-    run_accel_mixed<false>(L, P, pp, Ls, K, kick, t, fused_vsig);
+  PAIR_PASS(run_accel, L, P, pp, Ls, K, kick, t, fused_vsig);
   return cudaGetLastError();
 }
 
@@ -270,10 +298,7 @@ cudaError_t launch_dudt_mixed(const Launch & L, const Particles & P,
     k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
-  if(pp.cullen)
-    run_dudt_mixed_cullen(L, P, pp, Ls, K, t, then_op);
-  else
-    run_dudt_mixed<false>(L, P, pp, Ls, K, t, then_op);
+  PAIR_PASS(run_dudt, L, P, pp, Ls, K, t, then_op);
   return cudaGetLastError();
 }
 
@@ -290,10 +315,7 @@ cudaError_t launch_dedt_mixed(const Launch & L, const Particles & P,
     k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
     *L.counter += 1;
   }
-  if(pp.cullen)
-    run_dedt_mixed_cullen(L, P, pp, Ls, K, then_op, t, st, use_ahyd);
-  else
-    run_dedt_mixed<false>(L, P, pp, Ls, K, then_op, t, st, use_ahyd);
+  PAIR_PASS(run_dedt, L, P, pp, Ls, K, then_op, t, st, use_ahyd);
   return cudaGetLastError();
 }
 

@@ -1,36 +1,12 @@
 // fsph_mixed_cullen.cu -- Cullen & Dehnen's adaptive viscosity on the
-// mixed-precision path: the pair kernels of fsph_mixed_kernels.cuh with a
-// per-particle alpha, and the alpha pass itself.
+// mixed-precision path: the alpha pass (the pair passes with a per-particle
+// alpha are instances of fsph_mixed_kernels.cuh, fsph_mixed_pairs.cu).
 #include <cuda_runtime.h>
 
 #include "fsph_internal.cuh"
 #include "fsph_mixed_kernels.cuh"
 
 namespace fsph {
-
-void run_density_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
-  DevStatus * st, const DevTime * tm) {
-  run_density_mixed<true>(L, P, pp, Ls, K, cs_new, st, tm);
-}
-
-void run_accel_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,
-  const DevTime * t, int fused_vsig) {
-  run_accel_mixed<true>(L, P, pp, Ls, K, kick, t, fused_vsig);
-}
-
-void run_dudt_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t,
-  int then_op) {
-  run_dudt_mixed<true>(L, P, pp, Ls, K, t, then_op);
-}
-
-void run_dedt_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,
-  const DevTime * t, DevStatus * st, int use_ahyd) {
-  run_dedt_mixed<true>(L, P, pp, Ls, K, then_op, t, st, use_ahyd);
-}
 
 // viscosity::compute_alpha with A_trigger and compute_xi (viscosity.h:
 // 185-363).  The neighbour sums (the signal speed over all new sound

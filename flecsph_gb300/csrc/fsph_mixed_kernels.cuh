@@ -263,6 +263,61 @@ __device__ __forceinline__ float vel_diff_dot(const float4 & h1a, const float4 &
          ((dva.x - dvb.x) * dx + (dva.y - dvb.y) * dy + (dva.z - dvb.z) * dz);
 }
 
+// ---- four lanes per particle ----------------------------------------------
+// At a few tens of thousands of particles a thread per particle leaves one or
+// two warps per scheduler, and a pass takes as long as its longest list.  Then
+// every particle gets four lanes: lane q evaluates slot q of each chunk of
+// four, and the terms are added in slot order, by the same operations as a
+// single thread would, so the sums round alike.  The per-particle work that
+// follows a list (FP64 mostly) would waste three lanes of four: a block's
+// particles are handed to its first quarter of threads for it.
+//
+// The AUTO instances (runs of up to SPLIT_MAX particles) decide on the device,
+// from the lists: four lanes while all pairs together are fewer than
+// SPLIT_PAIRS times the longest list.  On lattices, where every list is as
+// long, that is 24k particles (a pass then takes as long either way: 2D Sod
+// 16k 53 -> 49 us for the three passes, 31k 53 -> 62; Sedov 40^3 178 -> 205);
+// on the star, whose longest lists are five times the mean, 120k (20k
+// particles 323 -> 162 us, 50k 322 -> 210, 100k 380 -> 326).  Having the choice
+// costs the acceleration of one thread per particle 6 % (132k Sedov), so larger
+// runs, which would not take four lanes, do not have it.
+#ifndef SPLIT_MAX
+#define SPLIT_MAX (1 << 17)
+#endif
+#ifndef SPLIT_PAIRS
+#define SPLIT_PAIRS 24576ull
+#endif
+
+template<bool AUTO>
+__device__ __forceinline__ bool four_lanes(const Lists & Ls) {
+  return AUTO && (unsigned long long)Ls.stat[1] < SPLIT_PAIRS * Ls.stat[0];
+}
+
+// the particle of this thread, in blocks of T threads
+template<int T>
+__device__ __forceinline__ int pass_particle(bool split) {
+  return split ? blockIdx.x * (T / 4) + (int)(threadIdx.x >> 2)
+               : blockIdx.x * T + (int)threadIdx.x;
+}
+
+// The indices of one lane of four, read one chunk ahead
+struct QuadChunks {
+  const int * lp;
+  int ahead;
+  unsigned mask;  // the lanes of this particle
+  __device__ __forceinline__ explicit QuadChunks(const int * p)
+    : lp(p + (threadIdx.x & 3)), ahead(*lp), mask(0xfu << (threadIdx.x & 28)) {}
+  __device__ __forceinline__ int next(int j0, int cnt) {
+    const int b = ahead;
+    if(j0 + 4 < cnt)
+      ahead = lp[(j0 + 4) << 5];
+    return b;
+  }
+  __device__ __forceinline__ float of(float v, int s) const {
+    return __shfl_sync(mask, v, s, 4);
+  }
+};
+
 template<int D>
 __device__ __forceinline__ PairGeom geom(const int4 & qa, const int4 & qb,
   float s0, float s1, float s2) {
@@ -282,17 +337,54 @@ __device__ __forceinline__ PairGeom geom(const int4 & qa, const int4 & qb,
 // compares (2 (1 - R)^4 div v)^2 against an absolute 1e-16
 // (viscosity.h:265-266), so FP32 rounding noise in a uniform flow would
 // switch the viscosity on where the reference keeps it off.
-template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
-  PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
+// m_b and the FP64 gradient factor of one pair of the divergence sum
+template<int D, int K>
+__device__ __forceinline__ double pair_mf(const Particles & P, const PhysParams & pp,
+  PairH<D, K> & ph, int b, const double * pa, double h_a, double * pos_ab) {
+  double r2 = 0.0;
+  for(int d = 0; d < D; ++d) {
+    pos_ab[d] = pa[d] - P.f[F_X + d][b];
+    r2 += pos_ab[d] * pos_ab[d];
+  }
+  ph.template set<false, true>(h_a, P.f[F_H][b], pp);
+  return P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
+}
+
+// The same for four lanes: lane d < D adds axis d of the chunk's four pairs,
+// in slot order, into gsum[0].
+template<int D, int K>
+__device__ __forceinline__ void quad_gsum(const Particles & P, const PhysParams & pp,
+  PairH<D, K> & ph, const QuadChunks & qc, int b, const double * pa, double h_a,
+  double * gsum) {
+  double pos_ab[3] = {0.0, 0.0, 0.0};
+  const double mf = pair_mf<D, K>(P, pp, ph, b, pa, h_a, pos_ab);
+  const int axis = threadIdx.x & 3;
+  for(int q = 0; q < 4; ++q) {
+    const double m = __shfl_sync(qc.mask, mf, q, 4);
+    double x = 0.0;
+    for(int d = 0; d < D; ++d) {
+      const double xd = __shfl_sync(qc.mask, pos_ab[d], q, 4);
+      x = axis == d ? xd : x;
+    }
+    gsum[0] = fma(m, x, gsum[0]);
+  }
+}
+
+template<int D, int K, bool CULL, bool AUTO>
+__global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(
+  Particles P, PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
   const DevTime * tm) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<MIX_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
   const int4 qa = Kp.qpos[a];
   const float ha = __int_as_float(qa.w);
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
   float sum = 0.f, comp = 0.f;
   double gsum[3] = {0.0, 0.0, 0.0};
@@ -304,34 +396,63 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
       pa[d] = P.f[F_X + d][a];
     h_a = P.f[F_H][a];
   }
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = lc.next(j0, cnt);
+  auto weight = [&](int b) {
+    const int4 qb = Kp.qpos[b];
+    const float mb = Kp.mass[b];
+    const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
+    const float hab = 0.5f * (ha + __int_as_float(qb.w));
+    const float ih = __fdividef(1.f, hab);
+    const float r = sqrtf(g.r2);
+    return mb * wfun<D, K>(r, hab, ih, pp);
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      const int b = qc.next(j0, cnt);
+      const float w = j0 + (int)(threadIdx.x & 3) < cnt ? weight(b) : 0.f;
+      for(int q = 0; q < 4; ++q)
+        kahan(sum, comp, qc.of(w, q));
+      if(CULL)
+        quad_gsum<D, K>(P, pp, ph, qc, b, pa, h_a, gsum);
+    }
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      // four slots per 16-byte load; padding slots hold a itself
+      const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const int4 qb = Kp.qpos[b];
-      const float mb = Kp.mass[b];
-      const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
-      const float hab = 0.5f * (ha + __int_as_float(qb.w));
-      const float ih = __fdividef(1.f, hab);
-      const float r = sqrtf(g.r2);
-      const float w = mb * wfun<D, K>(r, hab, ih, pp);
-      kahan(sum, comp, j0 + u < cnt ? w : 0.f);
-      if(CULL) {
-        // padding slots and the self pair have x_ab = 0 and add nothing
-        double pos_ab[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
-        for(int d = 0; d < D; ++d) {
-          pos_ab[d] = pa[d] - P.f[F_X + d][b];
-          r2 += pos_ab[d] * pos_ab[d];
+      for(int u = 0; u < 4; ++u) {
+        const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
+        const float w = weight(b);
+        kahan(sum, comp, j0 + u < cnt ? w : 0.f);
+        if(CULL) {
+          // padding slots and the self pair have x_ab = 0 and add nothing
+          double pos_ab[3] = {0.0, 0.0, 0.0};
+          const double mf = pair_mf<D, K>(P, pp, ph, b, pa, h_a, pos_ab);
+          for(int d = 0; d < D; ++d)
+            gsum[d] += mf * pos_ab[d];
         }
-        ph.template set<false, true>(h_a, P.f[F_H][b], pp);
-        const double mf = P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
-        for(int d = 0; d < D; ++d)
-          gsum[d] += mf * pos_ab[d];
       }
     }
+  }
+  if(split) {
+    __shared__ float2 r_sum[(MIX_THREADS / 4)];
+    __shared__ double r_g[3][(MIX_THREADS / 4)];
+    const int k = threadIdx.x >> 2, q = threadIdx.x & 3;
+    if(q == 0)
+      r_sum[k] = make_float2(sum, comp);
+    if(CULL && q < D)
+      r_g[q][k] = gsum[0];
+    __syncthreads();
+    a = blockIdx.x * (MIX_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (MIX_THREADS / 4) || a >= P.n)
+      return;
+    sum = r_sum[threadIdx.x].x;
+    comp = r_sum[threadIdx.x].y;
+    if(CULL)
+      for(int d = 0; d < D; ++d)
+        gsum[d] = r_g[d][threadIdx.x];
   }
   const double rho = (double)sum - (double)comp;
   if(!(rho > 0)) {
@@ -375,12 +496,16 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(Particles P,
 // kick below cannot race with it.
 // Three blocks of 256 per SM (<= 85 registers): the pass waits on neighbour
 // gathers, and 24 warps hide more of them than 16.
-template<int D, int K, bool VSIG, bool CULL>
+template<int D, int K, bool VSIG, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_accel_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<MIX_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
   const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
   const float alpha_a = CULL ? Kp.visc[a].x : 0.f;
@@ -388,7 +513,7 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_acc
   const float ha = __int_as_float(qa.w);
   const float4 vha = Kp.vhm[a];
   const float4 ta = Kp.thermo[a];
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   float ax = 0.f, ay = 0.f, az = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
   float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
   if(VSIG)
@@ -397,40 +522,83 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_acc
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
   // The self pair and coincident pairs add exactly zero (x_ab = 0, mu = 0),
   // as the reference's m_b = 0 makes them; the loop needs no branch.
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = lc.next(j0, cnt);
-#pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const int4 qb = Kp.qpos[b];
-      const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
-      const float hab = 0.5f * (ha + __int_as_float(qb.w));
-      const float ih = __fdividef(1.f, hab);
-      const float r = sqrtf(g.r2);
-      const float f = gfac<D, K>(r, hab, ih, pp);
-      const float4 vhb = Kp.vhm[b];
-      const float4 tb = Kp.thermo[b];
-      const float dotp = (vha.x - vhb.x) * g.dx + (vha.y - vhb.y) * g.dy +
-                         (vha.z - vhb.z) * g.dz;
-      const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
-      const float rho_ab = 0.5f * (ta.x + tb.x);
-      const float c_ab = 0.5f * (ta.z + tb.z);
-      const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, rho_ab, c_ab, mu);
-      const float sc = -vhb.w * (ta.y + tb.y + Pi) * f;
-      if(VSIG) {
-        const float4 vb = Kp.vel[b];
-        const float dotv = ((va.x - vb.x) * g.dx + (va.y - vb.y) * g.dy +
-                             (va.z - vb.z) * g.dz) * rsqrtf(g.r2);
-        const float cb = b > a ? tb.z : tb.w;
-        const float cand = fmaxf(ta.z, cb) - fminf(dotv, 0.f);
-        vsig = fmaxf(vsig, (b != a && g.r2 > 0.f) ? cand : 0.f);
+  auto pair = [&](int b, PairGeom & g) {
+    const int4 qb = Kp.qpos[b];
+    g = geom<D>(qa, qb, s0, s1, s2);
+    const float hab = 0.5f * (ha + __int_as_float(qb.w));
+    const float ih = __fdividef(1.f, hab);
+    const float r = sqrtf(g.r2);
+    const float f = gfac<D, K>(r, hab, ih, pp);
+    const float4 vhb = Kp.vhm[b];
+    const float4 tb = Kp.thermo[b];
+    const float dotp = (vha.x - vhb.x) * g.dx + (vha.y - vhb.y) * g.dy +
+                       (vha.z - vhb.z) * g.dz;
+    const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
+    const float rho_ab = 0.5f * (ta.x + tb.x);
+    const float c_ab = 0.5f * (ta.z + tb.z);
+    const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, rho_ab, c_ab, mu);
+    const float sc = -vhb.w * (ta.y + tb.y + Pi) * f;
+    if(VSIG) {
+      const float4 vb = Kp.vel[b];
+      const float dotv = ((va.x - vb.x) * g.dx + (va.y - vb.y) * g.dy +
+                           (va.z - vb.z) * g.dz) * rsqrtf(g.r2);
+      const float cb = b > a ? tb.z : tb.w;
+      const float cand = fmaxf(ta.z, cb) - fminf(dotv, 0.f);
+      vsig = fmaxf(vsig, (b != a && g.r2 > 0.f) ? cand : 0.f);
+    }
+    return sc;
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      PairGeom g;
+      const float sc = pair(qc.next(j0, cnt), g);
+      for(int q = 0; q < 4; ++q) {
+        const float sq = qc.of(sc, q);
+        kahan(ax, cx, qc.of(g.dx, q) * sq);
+        kahan(ay, cy, qc.of(g.dy, q) * sq);
+        if(D == 3)
+          kahan(az, cz, qc.of(g.dz, q) * sq);
       }
-      kahan(ax, cx, g.dx * sc);
-      kahan(ay, cy, g.dy * sc);
-      if(D == 3)
-        kahan(az, cz, g.dz * sc);
+    }
+    if(VSIG) {
+      const unsigned qm = 0xfu << (threadIdx.x & 28);
+      vsig = fmaxf(vsig, __shfl_xor_sync(qm, vsig, 1));
+      vsig = fmaxf(vsig, __shfl_xor_sync(qm, vsig, 2));
+    }
+    __shared__ float r_acc[7][(MIX_THREADS / 4)];
+    if((threadIdx.x & 3) == 0) {
+      const float r[7] = {ax, ay, az, cx, cy, cz, vsig};
+      for(int k = 0; k < 7; ++k)
+        r_acc[k][threadIdx.x >> 2] = r[k];
+    }
+    __syncthreads();
+    a = blockIdx.x * (MIX_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (MIX_THREADS / 4) || a >= P.n)
+      return;
+    ax = r_acc[0][threadIdx.x];
+    ay = r_acc[1][threadIdx.x];
+    az = r_acc[2][threadIdx.x];
+    cx = r_acc[3][threadIdx.x];
+    cy = r_acc[4][threadIdx.x];
+    cz = r_acc[5][threadIdx.x];
+    vsig = r_acc[6][threadIdx.x];
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      // four slots per 16-byte load; padding slots hold a itself
+      const int4 q4 = lc.next(j0, cnt);
+#pragma unroll
+      for(int u = 0; u < 4; ++u) {
+        const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
+        PairGeom g;
+        const float sc = pair(b, g);
+        kahan(ax, cx, g.dx * sc);
+        kahan(ay, cy, g.dy * sc);
+        if(D == 3)
+          kahan(az, cz, g.dz * sc);
+      }
     }
   }
   double acc[3] = {(double)ax - (double)cx, (double)ay - (double)cy,
@@ -469,12 +637,16 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_acc
 #define FSPH_ENERGY_BLOCKS 3
 #endif
 
-template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dudt_mixed(Particles P,
-  PhysParams pp, Lists Ls, Packed Kp, const DevTime * tm, int then_op) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+template<int D, int K, bool CULL, bool AUTO>
+__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dudt_mixed(
+  Particles P, PhysParams pp, Lists Ls, Packed Kp, const DevTime * tm, int then_op) {
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<ENERGY_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   // no internal energy change while relaxing (default_physics.h:423-427)
   if(tm->iteration < pp.relax_steps) {
     P.f[F_DUDT][a] = 0.0;
@@ -486,29 +658,59 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
   const int4 qa = Kp.qpos[a];
   const float ha = __int_as_float(qa.w);
   const float4 h1a = Kp.fv1[a], h2a = Kp.fv2[a], dva = Kp.fdv[a];
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   float dp = 0.f, cp = 0.f, dv = 0.f, cv = 0.f;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = lc.next(j0, cnt);
+  auto pair = [&](int b, float & m, float & vdw, float & Pi) {
+    const int4 qb = Kp.qpos[b];
+    const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
+    const float hab = 0.5f * (ha + __int_as_float(qb.w));
+    const float ih = __fdividef(1.f, hab);
+    const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
+    const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b], dvb = Kp.fdv[b];
+    const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dx, g.dy, g.dz);
+    const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
+    Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (h1a.w + h1b.w),
+      0.5f * (h2a.w + h2b.w), mu);
+    vdw = f * vel_diff_dot(h1a, h2a, dva, h1b, h2b, dvb, g.dx, g.dy, g.dz);
+    m = dvb.w;
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      float m, vdw, Pi;
+      pair(qc.next(j0, cnt), m, vdw, Pi);
+      for(int q = 0; q < 4; ++q) {
+        const float mq = qc.of(m, q), vq = qc.of(vdw, q), Pq = qc.of(Pi, q);
+        kahan(dp, cp, mq * vq);
+        kahan(dv, cv, mq * vq * Pq);
+      }
+    }
+    __shared__ float4 r_sum[(ENERGY_THREADS / 4)];
+    if((threadIdx.x & 3) == 0)
+      r_sum[threadIdx.x >> 2] = make_float4(dp, cp, dv, cv);
+    __syncthreads();
+    a = blockIdx.x * (ENERGY_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (ENERGY_THREADS / 4) || a >= P.n)
+      return;
+    const float4 r = r_sum[threadIdx.x];
+    dp = r.x;
+    cp = r.y;
+    dv = r.z;
+    cv = r.w;
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      // four slots per 16-byte load; padding slots hold a itself
+      const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const int4 qb = Kp.qpos[b];
-      const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
-      const float hab = 0.5f * (ha + __int_as_float(qb.w));
-      const float ih = __fdividef(1.f, hab);
-      const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
-      const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b], dvb = Kp.fdv[b];
-      const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dx, g.dy, g.dz);
-      const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
-      const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (h1a.w + h1b.w),
-        0.5f * (h2a.w + h2b.w), mu);
-      const float vdw = f * vel_diff_dot(h1a, h2a, dva, h1b, h2b, dvb, g.dx, g.dy, g.dz);
-      kahan(dp, cp, dvb.w * vdw);
-      kahan(dv, cv, dvb.w * vdw * Pi);
+      for(int u = 0; u < 4; ++u) {
+        float m, vdw, Pi;
+        pair(u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w, m, vdw, Pi);
+        kahan(dp, cp, m * vdw);
+        kahan(dv, cv, m * vdw * Pi);
+      }
     }
   }
   const double sp = (double)dp - (double)cp, sv = (double)dv - (double)cv;
@@ -534,13 +736,17 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
 // element-wise update that follows de/dt in the driver to the particle
 // right away: it reads only the particle's own fields, and the pass reads
 // the neighbours' P and c_s from the packed records, not the fields.
-template<int D, int K, bool CULL>
+template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(4, ENERGY_THREADS)) k_dedt_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<ENERGY_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
   const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
   const float alpha_a = CULL ? Kp.visc[a].x : 0.f;
@@ -549,32 +755,57 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(4, ENERGY_THREADS))
   const float4 vha = Kp.vhm[a];
   const float4 va = Kp.velp[a];  // .w = P_a / rho_a^2
   const float2 ra = Kp.rc[a];
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   float sum = 0.f, comp = 0.f;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    // four slots per 16-byte load; padding slots hold a itself
-    const int4 q4 = lc.next(j0, cnt);
+  auto pair = [&](int b, float & m) {
+    const int4 qb = Kp.qpos[b];
+    const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
+    const float hab = 0.5f * (ha + __int_as_float(qb.w));
+    const float ih = __fdividef(1.f, hab);
+    const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
+    const float4 vhb = Kp.vhm[b];
+    const float4 vb = Kp.velp[b];
+    const float2 rb = Kp.rc[b];
+    const float dotp = (vha.x - vhb.x) * g.dx + (vha.y - vhb.y) * g.dy +
+                       (vha.z - vhb.z) * g.dz;
+    const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
+    const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (ra.x + rb.x),
+      0.5f * (ra.y + rb.y), mu);
+    const float vad = f * (va.x * g.dx + va.y * g.dy + va.z * g.dz);
+    const float vbd = f * (vb.x * g.dx + vb.y * g.dy + vb.z * g.dz);
+    m = vhb.w;
+    return va.w * vbd + vad * vb.w + 0.5f * Pi * (vbd + vad);
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      float m;
+      const float x = pair(qc.next(j0, cnt), m);
+      for(int q = 0; q < 4; ++q)
+        kahan(sum, comp, qc.of(m, q) * qc.of(x, q));
+    }
+    __shared__ float2 r_sum[(ENERGY_THREADS / 4)];
+    if((threadIdx.x & 3) == 0)
+      r_sum[threadIdx.x >> 2] = make_float2(sum, comp);
+    __syncthreads();
+    a = blockIdx.x * (ENERGY_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (ENERGY_THREADS / 4) || a >= P.n)
+      return;
+    sum = r_sum[threadIdx.x].x;
+    comp = r_sum[threadIdx.x].y;
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      // four slots per 16-byte load; padding slots hold a itself
+      const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const int4 qb = Kp.qpos[b];
-      const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
-      const float hab = 0.5f * (ha + __int_as_float(qb.w));
-      const float ih = __fdividef(1.f, hab);
-      const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
-      const float4 vhb = Kp.vhm[b];
-      const float4 vb = Kp.velp[b];
-      const float2 rb = Kp.rc[b];
-      const float dotp = (vha.x - vhb.x) * g.dx + (vha.y - vhb.y) * g.dy +
-                         (vha.z - vhb.z) * g.dz;
-      const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
-      const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (ra.x + rb.x),
-        0.5f * (ra.y + rb.y), mu);
-      const float vad = f * (va.x * g.dx + va.y * g.dy + va.z * g.dz);
-      const float vbd = f * (vb.x * g.dx + vb.y * g.dy + vb.z * g.dz);
-      kahan(sum, comp, vhb.w * (va.w * vbd + vad * vb.w + 0.5f * Pi * (vbd + vad)));
+      for(int u = 0; u < 4; ++u) {
+        float m;
+        const float x = pair(u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w, m);
+        kahan(sum, comp, m * x);
+      }
     }
   }
   double gv = 0;
@@ -744,48 +975,8 @@ __device__ __forceinline__ ffloat ff_ipow(ffloat ih) {
 
 // The density sum of one particle: sum_b m_b wpoly(t_ab) / h_ab^D, or, with
 // UNI (every h equal), sum_b m_b wpoly(t_ab), the particle's 1/h^D applied
-// once afterwards.
-template<int D, int K, bool UNI>
-__device__ __forceinline__ ffloat density_ff_sum(const Packed & Kp, const int * lp,
-  int cnt, const float4 & pa, const float4 & la, const ffloat & iha,
-  const ffloat & ihDa) {
-  ffloat sum = ff_make(0.f, 0.f);
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = lc.next(j0, cnt);
-#pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const float4 pb = Kp.fph[b], lb = Kp.fpl[b];
-      const float2 mb = ((const float2 *)Kp.fmA)[2 * b];
-      const FFGeom<D> g = ff_geom<D>(pa, la, pb, lb);
-      ffloat ih = iha, ihD = ihDa;
-      if(!UNI && (pb.w != pa.w || lb.w != la.w)) {
-        ih = ff_rcp_scaled(ff_add(ff_make(pa.w, la.w), ff_make(pb.w, lb.w)), 2.f);
-        ihD = ff_ipow<D>(ih);
-      }
-      const ffloat q = ff_mul(g.r, ih);
-      const ffloat t = ff_cadd(1.f, ff_make(-q.h, -q.l));
-      ffloat w = ff_mul(ff_wpoly<K>(t), ff_make(mb.x, mb.y));
-      if(!UNI)
-        w = ff_mul(w, ihD);
-      if(!(q.h < 1.f) || j0 + u >= cnt)
-        w = ff_make(0.f, 0.f);
-      ff_acc(sum, w);
-    }
-  }
-  if(UNI)
-    sum = ff_mul(sum, ihDa);
-  return sum;
-}
-
-// 1: the density pass takes two neighbours per step in packed FP32x2
-#ifndef FSPH_DENSITY_PAIRED
-#define FSPH_DENSITY_PAIRED 1
-#endif
-
-// density_ff_sum with two neighbours per step in packed FP32x2 (the list's
-// four-slot chunks hold two pairs of neighbours).  The two lanes keep their
+// once afterwards.  Two neighbours per step in packed FP32x2 (the list's
+// four-slot chunks hold two pairs of neighbours); the two lanes keep their
 // own running sums, added at the end.
 template<int D, int K, bool UNI>
 __device__ __forceinline__ ffloat density_ff_sum2(const Packed & Kp, const int * lp,
@@ -838,53 +1029,111 @@ __device__ __forceinline__ ffloat density_ff_sum2(const Packed & Kp, const int *
   return s1;
 }
 
-template<int D, int K, bool CULL>
+// density_ff_sum2 by four lanes.  Its two running sums (even and odd slots)
+// are kept by lanes 0 and 1; the result is lane 0's.
+template<int D, int K, bool UNI>
+__device__ __forceinline__ ffloat density_ff_quad(const Packed & Kp, const int * lp,
+  int cnt, const float4 & pa, const float4 & la, const ffloat & iha,
+  const ffloat & ihDa) {
+  QuadChunks qc(lp);
+  ffloat sum = ff_make(0.f, 0.f);
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int b = qc.next(j0, cnt);
+    const float4 pb = Kp.fph[b], lb = Kp.fpl[b];
+    const float2 mb = ((const float2 *)Kp.fmA)[2 * b];
+    const FFGeom<D> g = ff_geom<D>(pa, la, pb, lb);
+    ffloat ih = iha;
+    if(!UNI)
+      ih = ff_rcp_scaled(ff_add(ff_make(pa.w, la.w), ff_make(pb.w, lb.w)), 2.f);
+    const ffloat q = ff_mul(g.r, ih);
+    const ffloat t = ff_cadd(1.f, ff_make(-q.h, -q.l));
+    ffloat w = ff_mul(ff_wpoly<K>(t), ff_make(mb.x, mb.y));
+    if(!UNI) {
+      const ffloat i2 = ff_sqr(ih);
+      w = ff_mul(w, D == 3 ? ff_mul(i2, ih) : i2);
+    }
+    if(!(q.h < 1.f) || j0 + (int)(threadIdx.x & 3) >= cnt)
+      w = ff_make(0.f, 0.f);
+    const ffloat w2 = ff_make(__shfl_down_sync(qc.mask, w.h, 2, 4),
+      __shfl_down_sync(qc.mask, w.l, 2, 4));
+    ff_acc(sum, w);
+    ff_acc(sum, w2);
+  }
+  ffloat s1 = ff_add(sum, ff_make(__shfl_down_sync(qc.mask, sum.h, 1, 4),
+    __shfl_down_sync(qc.mask, sum.l, 1, 4)));
+  if(UNI)
+    s1 = ff_mul(s1, ihDa);
+  return s1;
+}
+
+template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_density_ff(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
   const DevTime * tm) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<MIX_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float4 pa = Kp.fph[a], la = Kp.fpl[a];
   const ffloat iha = ff_rcp_scaled(ff_make(pa.w, la.w), 1.f);
   const ffloat ihDa = ff_ipow<D>(iha);
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
-#if FSPH_DENSITY_PAIRED
-  const ffloat sum = Kp.fscale[2] != 0.0
-                       ? density_ff_sum2<D, K, true>(Kp, lp, cnt, pa, la, iha, ihDa)
-                       : density_ff_sum2<D, K, false>(Kp, lp, cnt, pa, la, iha, ihDa);
-#else
-  const ffloat sum = Kp.fscale[2] != 0.0
-                       ? density_ff_sum<D, K, true>(Kp, lp, cnt, pa, la, iha, ihDa)
-                       : density_ff_sum<D, K, false>(Kp, lp, cnt, pa, la, iha, ihDa);
-#endif
+  const bool uni = Kp.fscale[2] != 0.0;
+  ffloat sum;
+  if(split)
+    sum = uni ? density_ff_quad<D, K, true>(Kp, lp, cnt, pa, la, iha, ihDa)
+              : density_ff_quad<D, K, false>(Kp, lp, cnt, pa, la, iha, ihDa);
+  else
+    sum = uni ? density_ff_sum2<D, K, true>(Kp, lp, cnt, pa, la, iha, ihDa)
+              : density_ff_sum2<D, K, false>(Kp, lp, cnt, pa, la, iha, ihDa);
   double gsum[3] = {0.0, 0.0, 0.0};
   if(CULL) {
-    // m_b grad_a W_ab for compute_divv, in FP64 (see k_density_mixed)
+    // m_b grad_a W_ab for compute_divv, in FP64 (see k_density_mixed); the
+    // padding slots (a itself) add nothing: x_ab = 0
     double pa64[3] = {0.0, 0.0, 0.0};
     for(int d = 0; d < D; ++d)
       pa64[d] = P.f[F_X + d][a];
     const double h_a = P.f[F_H][a];
     PairH<D, K> ph;
     ph.init();
-    for(int j0 = 0; j0 < cnt; j0 += 4) {
-      const int4 q4 = *(const int4 *)(lp + (j0 << 5));
-#pragma unroll
-      for(int u = 0; u < 4; ++u) {
-        // the padding slots (a itself) add nothing: x_ab = 0
-        const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-        double pos_ab[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
-        for(int d = 0; d < D; ++d) {
-          pos_ab[d] = pa64[d] - P.f[F_X + d][b];
-          r2 += pos_ab[d] * pos_ab[d];
-        }
-        ph.template set<false, true>(h_a, P.f[F_H][b], pp);
-        const double mf = P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
-        for(int d = 0; d < D; ++d)
-          gsum[d] += mf * pos_ab[d];
-      }
+    if(split) {
+      QuadChunks qc(lp);
+      for(int j0 = 0; j0 < cnt; j0 += 4)
+        quad_gsum<D, K>(P, pp, ph, qc, qc.next(j0, cnt), pa64, h_a, gsum);
     }
+    else
+      for(int j0 = 0; j0 < cnt; j0 += 4) {
+        const int4 q4 = *(const int4 *)(lp + (j0 << 5));
+#pragma unroll
+        for(int u = 0; u < 4; ++u) {
+          const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
+          double pos_ab[3] = {0.0, 0.0, 0.0};
+          const double mf = pair_mf<D, K>(P, pp, ph, b, pa64, h_a, pos_ab);
+          for(int d = 0; d < D; ++d)
+            gsum[d] += mf * pos_ab[d];
+        }
+      }
+  }
+  if(split) {
+    __shared__ float2 r_sum[(MIX_THREADS / 4)];
+    __shared__ double r_g[3][(MIX_THREADS / 4)];
+    const int k = threadIdx.x >> 2, q = threadIdx.x & 3;
+    if(q == 0)
+      r_sum[k] = make_float2(sum.h, sum.l);
+    if(CULL && q < D)
+      r_g[q][k] = gsum[0];
+    __syncthreads();
+    a = blockIdx.x * (MIX_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (MIX_THREADS / 4) || a >= P.n)
+      return;
+    sum = ff_make(r_sum[threadIdx.x].x, r_sum[threadIdx.x].y);
+    if(CULL)
+      for(int d = 0; d < D; ++d)
+        gsum[d] = r_g[d][threadIdx.x];
   }
   const double iE = Kp.fscale[1];
   const double iED = D == 3 ? iE * iE * iE : iE * iE;
@@ -959,6 +1208,53 @@ struct AccelFFState {
   float vsig;
 };
 
+// One pair: S with S x_ab the pressure term, V with V x_ab the viscous one,
+// and the signal speed's maximum.
+template<int D, int K, bool VSIG, bool CULL, bool UNI>
+__device__ __forceinline__ void accel_ff_pair(const Packed & Kp, int b, int a,
+  const float4 & pa, const float4 & la, const ffloat & iha, const ffloat & ihPa,
+  const ffloat & Aa, const float4 & h1a, const float4 & h2a, const float4 & va, float eps,
+  float alpha, float beta, float alpha_a, FFGeom<D> & g, ffloat & S, float & V,
+  float & vsig) {
+  const float4 pb = Kp.fph[b], lb = Kp.fpl[b];
+  g = ff_geom<D>(pa, la, pb, lb);
+  ffloat ih = iha, ihP = ihPa;
+  if(!UNI && (pb.w != pa.w || lb.w != la.w)) {
+    ih = ff_rcp_scaled(ff_add(ff_make(pa.w, la.w), ff_make(pb.w, lb.w)), 2.f);
+    ihP = ff_ipow<D + 2>(ih);
+  }
+  const ffloat q = ff_mul(g.r, ih);
+  const ffloat t = ff_cadd(1.f, ff_make(-q.h, -q.l));
+  const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b];  // v_half, rho, c_s
+  const float4 mAb = Kp.fmA[b];
+  // viscosity in FP32 (the position unit cancels in mu)
+  const float hab = 0.5f * (pa.w + pb.w);
+  const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dxr[0], g.dxr[1], g.dxr[2]);
+  const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2f + eps * hab * hab) : 0.f;
+  const float rho_ab = 0.5f * (h1a.w + h1b.w);
+  const float c_ab = 0.5f * (h2a.w + h2b.w);
+  const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, rho_ab, c_ab, mu);
+  const ffloat gp = ff_gpoly<K>(t);
+  S = ff_mul(ff_mul(ff_add(Aa, ff_make(mAb.z, mAb.w)), ff_make(mAb.x, mAb.y)), gp);
+  V = mAb.x * Pi * gp.h;
+  if(!UNI) {
+    S = ff_mul(S, ihP);
+    V *= ihP.h;
+  }
+  if(!(q.h < 1.f)) {
+    S = ff_make(0.f, 0.f);
+    V = 0.f;
+  }
+  if(VSIG) {
+    const float4 vb = Kp.vel[b];  // .w: c_s before the density pass
+    const float dotv = ((va.x - vb.x) * g.dxr[0] + (va.y - vb.y) * g.dxr[1] +
+                         (va.z - vb.z) * g.dxr[2]) * rsqrtf(g.r2f);
+    const float cb = b > a ? h2b.w : vb.w;
+    const float cand = fmaxf(h2a.w, cb) - fminf(dotv, 0.f);
+    vsig = fmaxf(vsig, (b != a && g.r2f > 0.f) ? cand : 0.f);
+  }
+}
+
 template<int D, int K, bool VSIG, bool CULL, bool UNI>
 __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
   int cnt, int a, const float4 & pa, const float4 & la, const ffloat & iha,
@@ -974,44 +1270,11 @@ __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
 #pragma unroll(accel_ff_unroll)
     for(int u = 0; u < 4; ++u) {
       const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const float4 pb = Kp.fph[b], lb = Kp.fpl[b];
-      const FFGeom<D> g = ff_geom<D>(pa, la, pb, lb);
-      ffloat ih = iha, ihP = ihPa;
-      if(!UNI && (pb.w != pa.w || lb.w != la.w)) {
-        ih = ff_rcp_scaled(ff_add(ff_make(pa.w, la.w), ff_make(pb.w, lb.w)), 2.f);
-        ihP = ff_ipow<D + 2>(ih);
-      }
-      const ffloat q = ff_mul(g.r, ih);
-      const ffloat t = ff_cadd(1.f, ff_make(-q.h, -q.l));
-      const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b];  // v_half, rho, c_s
-      const float4 mAb = Kp.fmA[b];
-      // viscosity in FP32 (the position unit cancels in mu)
-      const float hab = 0.5f * (pa.w + pb.w);
-      const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dxr[0], g.dxr[1], g.dxr[2]);
-      const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2f + eps * hab * hab) : 0.f;
-      const float rho_ab = 0.5f * (h1a.w + h1b.w);
-      const float c_ab = 0.5f * (h2a.w + h2b.w);
-      const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, rho_ab, c_ab, mu);
-      const ffloat gp = ff_gpoly<K>(t);
-      ffloat S = ff_mul(ff_mul(ff_add(Aa, ff_make(mAb.z, mAb.w)), ff_make(mAb.x, mAb.y)),
-        gp);
-      float V = mAb.x * Pi * gp.h;
-      if(!UNI) {
-        S = ff_mul(S, ihP);
-        V *= ihP.h;
-      }
-      if(!(q.h < 1.f)) {
-        S = ff_make(0.f, 0.f);
-        V = 0.f;
-      }
-      if(VSIG) {
-        const float4 vb = Kp.vel[b];  // .w: c_s before the density pass
-        const float dotv = ((va.x - vb.x) * g.dxr[0] + (va.y - vb.y) * g.dxr[1] +
-                             (va.z - vb.z) * g.dxr[2]) * rsqrtf(g.r2f);
-        const float cb = b > a ? h2b.w : vb.w;
-        const float cand = fmaxf(h2a.w, cb) - fminf(dotv, 0.f);
-        vsig = fmaxf(vsig, (b != a && g.r2f > 0.f) ? cand : 0.f);
-      }
+      FFGeom<D> g;
+      ffloat S;
+      float V;
+      accel_ff_pair<D, K, VSIG, CULL, UNI>(Kp, b, a, pa, la, iha, ihPa, Aa, h1a, h2a, va,
+        eps, alpha, beta, alpha_a, g, S, V, vsig);
       // padding slots and the self pair have dx = 0 and add nothing
       ff_acc(sx, ff_mul(S, g.dx[0]));
       ff_acc(sy, ff_mul(S, g.dx[1]));
@@ -1038,6 +1301,60 @@ __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
   out.vsig = vsig;
 }
 
+// accel_ff_sum by four lanes: lane c < D adds axis c of the chunk's four pairs
+// in slot order; the pairs' terms change lanes through shared memory (`box`,
+// ACCEL_QUAD floats per particle: per axis four high words, four low words and
+// four FP32 separations, then four V).  The result for axis c, in out.sx and
+// out.vx, is lane c's, the signal speed every lane's.
+#define ACCEL_QUAD 44  // 40 used; 44 keeps the eight quads of a warp off one another's banks
+template<int D, int K, bool VSIG, bool CULL, bool UNI>
+__device__ __forceinline__ void accel_ff_quad(const Packed & Kp, const int * lp,
+  int cnt, int a, const float4 & pa, const float4 & la, const ffloat & iha,
+  const ffloat & ihPa, const ffloat & Aa, const float4 & h1a, const float4 & h2a,
+  const float4 & va, float eps, float alpha, float beta, float alpha_a, float * box,
+  AccelFFState & out) {
+  ffloat s = ff_make(0.f, 0.f);
+  float v = 0.f, cv = 0.f, vsig = 0.f;
+  QuadChunks qc(lp);
+  const int q = threadIdx.x & 3, axis = min(q, D - 1);
+  const float4 * in = (const float4 *)box;
+  for(int j0 = 0; j0 < cnt; j0 += 4) {
+    const int b = qc.next(j0, cnt);
+    FFGeom<D> g;
+    ffloat S;
+    float V;
+    accel_ff_pair<D, K, VSIG, CULL, UNI>(Kp, b, a, pa, la, iha, ihPa, Aa, h1a, h2a, va, eps,
+      alpha, beta, alpha_a, g, S, V, vsig);
+    __syncwarp(qc.mask);  // the last chunk's terms have been read
+    for(int c = 0; c < D; ++c) {
+      const ffloat t = ff_mul(S, g.dx[c]);
+      box[12 * c + q] = t.h;
+      box[12 * c + 4 + q] = t.l;
+      box[12 * c + 8 + q] = g.dxr[c];
+    }
+    box[36 + q] = V;
+    __syncwarp(qc.mask);
+    const float4 th = in[3 * axis], tl = in[3 * axis + 1], x = in[3 * axis + 2], Vs = in[9];
+    ff_acc(s, ff_make(th.x, tl.x));
+    kahan(v, cv, Vs.x * x.x);
+    ff_acc(s, ff_make(th.y, tl.y));
+    kahan(v, cv, Vs.y * x.y);
+    ff_acc(s, ff_make(th.z, tl.z));
+    kahan(v, cv, Vs.z * x.z);
+    ff_acc(s, ff_make(th.w, tl.w));
+    kahan(v, cv, Vs.w * x.w);
+  }
+  if(UNI)
+    s = ff_mul(s, ihPa);
+  out.sx = s;
+  out.vx = (v - cv) * (UNI ? ihPa.h : 1.f);
+  if(VSIG) {
+    vsig = fmaxf(vsig, __shfl_xor_sync(qc.mask, vsig, 1));
+    vsig = fmaxf(vsig, __shfl_xor_sync(qc.mask, vsig, 2));
+  }
+  out.vsig = vsig;
+}
+
 // Resident blocks of 256 per SM the acceleration pass is compiled for.  2
 // gives it up to 128 registers; 3 caps it at 80 for 24 warps to hide the
 // neighbour gathers, which measured slower on Sedov 128^3 (2.23 against
@@ -1047,12 +1364,16 @@ __device__ __forceinline__ void accel_ff_sum(const Packed & Kp, const int * lp,
 #define FSPH_ACCEL_FF_BLOCKS 2
 #endif
 
-template<int D, int K, bool VSIG, bool CULL>
+template<int D, int K, bool VSIG, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(FSPH_ACCEL_FF_BLOCKS, MIX_THREADS)) k_accel_ff(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<MIX_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
   const float alpha_a = CULL ? Kp.visc[a].x : 0.f;
   const float4 pa = Kp.fph[a], la = Kp.fpl[a];
@@ -1061,13 +1382,44 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(FSPH_ACCEL_FF_BLOCKS, 
   const ffloat iha = ff_rcp_scaled(ff_make(pa.w, la.w), 1.f);
   const ffloat ihPa = ff_ipow<D + 2>(iha);
   const float4 h1a = Kp.fv1[a], h2a = Kp.fv2[a];
-  const int cnt = Ls.cnt[a];
+  const int cnt = live ? Ls.cnt[a] : 0;
   float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
   if(VSIG)
     va = Kp.vel[a];
   const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  const bool uni = Kp.fscale[2] != 0.0;
   AccelFFState r;
-  if(Kp.fscale[2] != 0.0)
+  if(split) {
+    __shared__ __align__(16) float box[(MIX_THREADS / 4)][ACCEL_QUAD];
+    __shared__ float r_s[10][(MIX_THREADS / 4)];
+    const int k = threadIdx.x >> 2, q = threadIdx.x & 3;
+    if(uni)
+      accel_ff_quad<D, K, VSIG, CULL, true>(Kp, lp, cnt, a, pa, la, iha, ihPa, Aa, h1a,
+        h2a, va, eps, alpha, beta, alpha_a, box[k], r);
+    else
+      accel_ff_quad<D, K, VSIG, CULL, false>(Kp, lp, cnt, a, pa, la, iha, ihPa, Aa, h1a,
+        h2a, va, eps, alpha, beta, alpha_a, box[k], r);
+    if(q < D) {
+      r_s[q][k] = r.sx.h;
+      r_s[3 + q][k] = r.sx.l;
+      r_s[6 + q][k] = r.vx;
+    }
+    if(q == 0)
+      r_s[9][k] = r.vsig;
+    __syncthreads();
+    const int t = threadIdx.x;
+    a = blockIdx.x * (MIX_THREADS / 4) + t;
+    if(t >= (MIX_THREADS / 4) || a >= P.n)
+      return;
+    r.sx = ff_make(r_s[0][t], r_s[3][t]);
+    r.sy = ff_make(r_s[1][t], r_s[4][t]);
+    r.sz = D == 3 ? ff_make(r_s[2][t], r_s[5][t]) : ff_make(0.f, 0.f);
+    r.vx = r_s[6][t];
+    r.vy = r_s[7][t];
+    r.vz = D == 3 ? r_s[8][t] : 0.f;
+    r.vsig = r_s[9][t];
+  }
+  else if(uni)
     accel_ff_sum<D, K, VSIG, CULL, true>(Kp, lp, cnt, a, pa, la, iha, ihPa, Aa, h1a,
       h2a, va, eps, alpha, beta, alpha_a, r);
   else
@@ -1126,45 +1478,74 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(FSPH_ACCEL_FF_BLOCKS, 
 // over velocity differences and the viscosity, stays FP32.  Valid while
 // positions, P/rho^2, v_half and alpha are those of the acceleration pass
 // (the caller tracks that).
-template<int D, int K, bool CULL>
-__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dedt_ahyd(Particles P,
-  PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
+template<int D, int K, bool CULL, bool AUTO>
+__global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dedt_ahyd(
+  Particles P, PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if(a >= P.n)
+  const bool split = four_lanes<AUTO>(Ls);
+  int a = pass_particle<ENERGY_THREADS>(split);
+  if(!split && a >= P.n)
     return;
+  const bool live = a < P.n;
+  if(split)
+    a = min(a, P.n - 1);
   const float s0 = Kp.qscale[0], s1 = Kp.qscale[1], s2 = D == 3 ? Kp.qscale[2] : 0.f;
+  const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
   const float alpha_a = CULL ? Kp.visc[a].x : 0.f;
   const int4 qa = Kp.qpos[a];
+  const float ha = __int_as_float(qa.w);
   const float4 h1a = Kp.fv1[a], h2a = Kp.fv2[a], dva = Kp.fdv[a];
   const float Aa = Kp.fmA[a].z;  // P_a / rho_a^2 (high word)
-  const int cnt = Ls.cnt[a];
-  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
-  const float eps = (float)pp.eps, alpha = (float)pp.alpha, beta = (float)pp.beta;
-  const float ha = __int_as_float(qa.w);
+  const int cnt = live ? Ls.cnt[a] : 0;
   float sum = 0.f, comp = 0.f;
-  ListChunks lc(lp);
-  for(int j0 = 0; j0 < cnt; j0 += 4) {
-    const int4 q4 = lc.next(j0, cnt);
+  const int * lp = Ls.idx + list_slot(a, 0, Ls.maxnb);
+  auto pair = [&](int b, float & m) {
+    const int4 qb = Kp.qpos[b];
+    const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
+    const float hab = 0.5f * (ha + __int_as_float(qb.w));
+    const float ih = __fdividef(1.f, hab);
+    const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
+    const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b], dvb = Kp.fdv[b];
+    const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dx, g.dy, g.dz);
+    const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
+    const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (h1a.w + h1b.w),
+      0.5f * (h2a.w + h2b.w), mu);
+    // v_b - v_a and v_a + v_b, v = v_half + (v - v_half)
+    const float vbad = f * vel_diff_dot(h1b, h2b, dvb, h1a, h2a, dva, g.dx, g.dy, g.dz);
+    const float vsd = f * (((h1a.x + h1b.x) + (dva.x + dvb.x)) * g.dx +
+                           ((h1a.y + h1b.y) + (dva.y + dvb.y)) * g.dy +
+                           ((h1a.z + h1b.z) + (dva.z + dvb.z)) * g.dz);
+    m = dvb.w;
+    return Aa * vbad + 0.5f * Pi * vsd;
+  };
+  if(split) {
+    QuadChunks qc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      float m;
+      const float x = pair(qc.next(j0, cnt), m);
+      for(int q = 0; q < 4; ++q)
+        kahan(sum, comp, qc.of(m, q) * qc.of(x, q));
+    }
+    __shared__ float2 r_sum[(ENERGY_THREADS / 4)];
+    if((threadIdx.x & 3) == 0)
+      r_sum[threadIdx.x >> 2] = make_float2(sum, comp);
+    __syncthreads();
+    a = blockIdx.x * (ENERGY_THREADS / 4) + (int)threadIdx.x;
+    if(threadIdx.x >= (ENERGY_THREADS / 4) || a >= P.n)
+      return;
+    sum = r_sum[threadIdx.x].x;
+    comp = r_sum[threadIdx.x].y;
+  }
+  else {
+    ListChunks lc(lp);
+    for(int j0 = 0; j0 < cnt; j0 += 4) {
+      const int4 q4 = lc.next(j0, cnt);
 #pragma unroll
-    for(int u = 0; u < 4; ++u) {
-      const int b = u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w;
-      const int4 qb = Kp.qpos[b];
-      const PairGeom g = geom<D>(qa, qb, s0, s1, s2);
-      const float hab = 0.5f * (ha + __int_as_float(qb.w));
-      const float ih = __fdividef(1.f, hab);
-      const float f = gfac<D, K>(sqrtf(g.r2), hab, ih, pp);
-      const float4 h1b = Kp.fv1[b], h2b = Kp.fv2[b], dvb = Kp.fdv[b];
-      const float dotp = vdiff_dot(h1a, h2a, h1b, h2b, g.dx, g.dy, g.dz);
-      const float mu = dotp < 0.f ? __fdividef(hab * dotp, g.r2 + eps * hab * hab) : 0.f;
-      const float Pi = visc_pi_f<CULL>(alpha, beta, alpha_a, Kp, b, 0.5f * (h1a.w + h1b.w),
-        0.5f * (h2a.w + h2b.w), mu);
-      // v_b - v_a and v_a + v_b, v = v_half + (v - v_half)
-      const float vbad = f * vel_diff_dot(h1b, h2b, dvb, h1a, h2a, dva, g.dx, g.dy, g.dz);
-      const float vsd = f * (((h1a.x + h1b.x) + (dva.x + dvb.x)) * g.dx +
-                             ((h1a.y + h1b.y) + (dva.y + dvb.y)) * g.dy +
-                             ((h1a.z + h1b.z) + (dva.z + dvb.z)) * g.dz);
-      kahan(sum, comp, dvb.w * (Aa * vbad + 0.5f * Pi * vsd));
+      for(int u = 0; u < 4; ++u) {
+        float m;
+        const float x = pair(u == 0 ? q4.x : u == 1 ? q4.y : u == 2 ? q4.z : q4.w, m);
+        kahan(sum, comp, m * x);
+      }
     }
   }
   double gv = 0, vah = 0;
@@ -1202,45 +1583,46 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
 // ------------------------------------------------------------ dispatch --
 #define MIX_DISPATCH(THREADS, KERNEL_T, TA, ...)                                            \
   do {                                                                         \
-    const int nb_ = (P.n + THREADS - 1) / THREADS;                     \
+    const int nt_ = (THREADS), per_ = AUTO ? (THREADS) / 4 : (THREADS);        \
+    const int nb_ = (P.n + per_ - 1) / per_;                                   \
     if(pp.dim == 3) {                                                          \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<3, FSPH_KERNEL_SINC, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_SINC, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     else {                                                                     \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<2, FSPH_KERNEL_SINC, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_SINC, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     *L.counter += 1;                                                           \
@@ -1253,22 +1635,23 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
 // (cubic and quintic splines, Gaussians, sinc) keep the FP32 passes.
 #define FF_DISPATCH(THREADS, KERNEL_T, TA, ...)                                         \
   do {                                                                         \
-    const int nb_ = (P.n + THREADS - 1) / THREADS;                     \
+    const int nt_ = (THREADS), per_ = AUTO ? (THREADS) / 4 : (THREADS);        \
+    const int nb_ = (P.n + per_ - 1) / per_;                                   \
     if(pp.dim == 3) {                                                          \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
     }                                                                          \
     else {                                                                     \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA><<<nb_, THREADS, 0, L.stream>>>(__VA_ARGS__); \
+        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
     }                                                                          \
     *L.counter += 1;                                                           \
   } while(0)
@@ -1278,8 +1661,8 @@ inline bool wendland_kernel(int k) {
          k == FSPH_KERNEL_WENDLAND_C6;
 }
 
-template<bool CULL>
-inline void run_density_mixed(const Launch & L, const Particles & P,
+template<bool CULL, bool AUTO>
+inline void run_density_pass(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm) {
   if(wendland_kernel(pp.kernel))
@@ -1288,15 +1671,15 @@ inline void run_density_mixed(const Launch & L, const Particles & P,
     MIX_DISPATCH(MIX_THREADS, k_density_mixed, CULL, P, pp, Ls, K, cs_new, st, tm);
 }
 
-template<bool CULL>
-inline void run_dudt_mixed(const Launch & L, const Particles & P,
+template<bool CULL, bool AUTO>
+inline void run_dudt_pass(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t,
   int then_op) {
   MIX_DISPATCH(ENERGY_THREADS, k_dudt_mixed, CULL, P, pp, Ls, K, t, then_op);
 }
 
-template<bool CULL>
-inline void run_dedt_mixed(const Launch & L, const Particles & P,
+template<bool CULL, bool AUTO>
+inline void run_dedt_pass(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,
   const DevTime * t, DevStatus * st, int use_ahyd) {
   if(use_ahyd && wendland_kernel(pp.kernel))
@@ -1305,14 +1688,15 @@ inline void run_dedt_mixed(const Launch & L, const Particles & P,
     MIX_DISPATCH(ENERGY_THREADS, k_dedt_mixed, CULL, P, pp, Ls, K, then_op, t, st);
 }
 
-template<bool CULL>
-inline void run_accel_mixed(const Launch & L, const Particles & P,
+template<bool CULL, bool AUTO>
+inline void run_accel_pass(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,
   const DevTime * t, int fused_vsig) {
-  const int threads = MIX_THREADS;
+  const int threads = MIX_THREADS, per = AUTO ? MIX_THREADS / 4 : MIX_THREADS;
   void (*fn)(Particles, PhysParams, Lists, Packed, int, const DevTime *) = nullptr;
 #define PICK(D, KK)                                                            \
-  fn = fused_vsig ? k_accel_mixed<D, KK, true, CULL> : k_accel_mixed<D, KK, false, CULL>
+  fn = fused_vsig ? k_accel_mixed<D, KK, true, CULL, AUTO>                          \
+                  : k_accel_mixed<D, KK, false, CULL, AUTO>
   if(pp.dim == 3) {
     switch(pp.kernel) {
       case FSPH_KERNEL_CUBIC_SPLINE: PICK(3, FSPH_KERNEL_CUBIC_SPLINE); break;
@@ -1339,7 +1723,8 @@ inline void run_accel_mixed(const Launch & L, const Particles & P,
   }
 #undef PICK
 #define PICK(D, KK)                                                            \
-  fn = fused_vsig ? k_accel_ff<D, KK, true, CULL> : k_accel_ff<D, KK, false, CULL>
+  fn = fused_vsig ? k_accel_ff<D, KK, true, CULL, AUTO>                             \
+                  : k_accel_ff<D, KK, false, CULL, AUTO>
   if(wendland_kernel(pp.kernel)) {
     if(pp.dim == 3) {
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2) PICK(3, FSPH_KERNEL_WENDLAND_C2);
@@ -1353,23 +1738,32 @@ inline void run_accel_mixed(const Launch & L, const Particles & P,
     }
   }
 #undef PICK
-  fn<<<(P.n + threads - 1) / threads, threads, 0, L.stream>>>(P, pp, Ls, K, kick, t);
+  fn<<<(P.n + per - 1) / per, threads, 0, L.stream>>>(P, pp, Ls, K, kick, t);
   *L.counter += 1;
 }
 
-// The Cullen & Dehnen instances, compiled in fsph_mixed_cullen.cu.
-void run_density_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
-  DevStatus * st, const DevTime * tm);
-void run_accel_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,
-  const DevTime * t, int fused_vsig);
-void run_dudt_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t,
-  int then_op);
-void run_dedt_mixed_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,
-  const DevTime * t, DevStatus * st, int use_ahyd);
+// The pair passes of one viscosity (cullen), with and without the choice of
+// four lanes (split), one translation unit each so that they compile side by
+// side: fsph_mixed_pairs.cu with FSPH_PAIRS_CULLEN and FSPH_PAIRS_SPLIT of 0
+// or 1.
+#define PAIR_UNIT(NAME)                                                        \
+  void run_density_##NAME(const Launch & L, const Particles & P,               \
+    const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new, \
+    DevStatus * st, const DevTime * tm);                                       \
+  void run_accel_##NAME(const Launch & L, const Particles & P,                 \
+    const PhysParams & pp, const Lists & Ls, const Packed & K, int kick,       \
+    const DevTime * t, int fused_vsig);                                        \
+  void run_dudt_##NAME(const Launch & L, const Particles & P,                  \
+    const PhysParams & pp, const Lists & Ls, const Packed & K,                 \
+    const DevTime * t, int then_op);                                           \
+  void run_dedt_##NAME(const Launch & L, const Particles & P,                  \
+    const PhysParams & pp, const Lists & Ls, const Packed & K, int then_op,    \
+    const DevTime * t, DevStatus * st, int use_ahyd);
+PAIR_UNIT(mixed)
+PAIR_UNIT(mixed_split)
+PAIR_UNIT(mixed_cullen)
+PAIR_UNIT(mixed_cullen_split)
+#undef PAIR_UNIT
 void run_alpha_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t);
 

@@ -1941,6 +1941,15 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
         ncand = 0;
       }
     }
+    if(!ORDERED && P.n <= LIST_STAT_MAX) {
+      const unsigned kept = mem ? (unsigned)min(cnt, maxnb) : 0u;
+      const unsigned longest = __reduce_max_sync(FULL, kept);
+      const unsigned pairs = __reduce_add_sync(FULL, kept);
+      if(lane == 0) {
+        atomicMax(&Ls.stat[0], longest);
+        atomicAdd(&Ls.stat[1], pairs);
+      }
+    }
     if(mem) {
       if(cnt > maxnb) {
         if(atomicCAS(&st->code, 0, (int)FSPH_ERR_LIST_OVERFLOW) == 0)
