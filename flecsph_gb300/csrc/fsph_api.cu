@@ -165,6 +165,7 @@ void make_phys(const fsph_params * p, PhysParams * pp) {
 // analysis::set_initial_time_iteration (analysis.h:221-249)
 void init_time(const fsph_params * p, DevTime * t) {
   memset(t, 0, sizeof(*t));
+  t->dtmin_acc = TIME_DT_MAX;
   t->iteration = p->initial_iteration;
   t->totaltime = p->initial_time;
   t->dt = p->initial_dt;
@@ -467,11 +468,12 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   ok &= dalloc(c, &c->Palt.key, N) == cudaSuccess;
   ok &= dalloc(c, &c->cs_new, N) == cudaSuccess;
   ok &= dalloc(c, &c->skeys, N) == cudaSuccess;
-  ok &= dalloc(c, &c->skeys_tmp, N) == cudaSuccess;
+  // (also the range's partial words, before the keys are sorted)
+  ok &= dalloc(c, &c->skeys_tmp, N > RANGE_PART ? N : RANGE_PART) == cudaSuccess;
   ok &= dalloc(c, &c->svals, N) == cudaSuccess;
   ok &= dalloc(c, &c->svals_tmp, N) == cudaSuccess;
   ok &= dalloc(c, &c->hist, radix_hist_entries((int)N)) == cudaSuccess;
-  ok &= dalloc(c, &c->d_range, 8) == cudaSuccess;
+  ok &= dalloc(c, &c->d_range, RANGE_WORDS) == cudaSuccess;
   ok &= dalloc(c, &c->T.parent, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.leaf_parent, N) == cudaSuccess;
   ok &= dalloc(c, &c->T.first, N) == cudaSuccess;
@@ -551,6 +553,7 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
     }
   }
   if(cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess ||
+     cudaMemsetAsync(c->d_range, 0, sizeof(*c->d_range) * RANGE_WORDS, c->stream) != cudaSuccess ||
      cudaMemsetAsync(c->T.xchg, 0xff, sizeof(*c->T.xchg) * N, c->stream) != cudaSuccess)
     return fail(FSPH_ERR_CUDA);
   // timer and mark events are made on first use: an ensemble holds hundreds
@@ -829,8 +832,12 @@ fsph_status fsph_get_range(fsph_ctx * c, double * range) {
 
 // ------------------------------------------------------------ body_system
 static bool wendland(int k);
+static fsph_status update_iteration(fsph_ctx * c, bool range_known);
 
-fsph_status fsph_update_iteration(fsph_ctx * c) {
+fsph_status fsph_update_iteration(fsph_ctx * c) { return update_iteration(c, false); }
+
+// range_known: the range words already hold the range of the positions
+static fsph_status update_iteration(fsph_ctx * c, bool range_known) {
   if(!c || !c->uploaded)
     return FSPH_ERR_STATE;
   records_stale(c);
@@ -861,7 +868,9 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
   const int n = c->n;
   {
     Phase ph(c, FSPH_TIMER_RANGE_KEYS);
-    CK(launch_range_keys(L, c->P, c->pp, (double *)c->d_range, c->skeys, c->svals));
+    if(!range_known)
+      CK(launch_range(L, c->P, c->pp, c->d_range, c->skeys_tmp));
+    CK(launch_keys(L, c->P, c->pp, c->d_range, c->skeys, c->svals));
   }
   {
     Phase ph(c, FSPH_TIMER_SORT);
@@ -874,8 +883,8 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
     }
     // the mixed float-float path's {v, c_s} records come out of the permute
     float4 * vel = c->mixed && wendland(c->pp.kernel) ? c->K.vel : nullptr;
-    CK(launch_permute(L, c->P, c->Palt, c->svals, c->skeys, c->permute_skip, vel,
-      c->pp.dim));
+    CK(launch_permute(L, c->P, c->Palt, c->svals, c->skeys, c->permute_skip, c->d_range,
+      c->K, c->T.ngroups, c->Ls.stat, vel, c->pp.dim));
     c->vel_ok = vel != nullptr;
     Particles t = c->P;
     c->P = c->Palt;
@@ -883,8 +892,6 @@ fsph_status fsph_update_iteration(fsph_ctx * c) {
   }
   {
     Phase ph(c, FSPH_TIMER_TREE);
-    CK(launch_pack_positions(L, c->P, c->pp, c->d_range, c->K, c->T.ngroups,
-      c->Ls.stat));
     CK(launch_build_tree(L, c->P, c->pp, c->T,
       c->p.group_size > 0 ? c->p.group_size : GROUP_MAX, c->d_range, c->K.qpos,
       c->K.qscale, c->mixed ? 0 : 1, c->d_status));
@@ -1144,6 +1151,18 @@ static fsph_status elem(fsph_ctx * c, int op, int phase) {
   return FSPH_OK;
 }
 
+static fsph_status kick_drift(fsph_ctx * c, int op, bool with_range) {
+  records_stale(c);
+  fsph_status s = set_device(c);
+  if(s)
+    return s;
+  Launch L = c->L();
+  Phase ph(c, FSPH_TIMER_INTEGRATE);
+  CK(launch_kick_drift(L, c->P, c->pp, op, c->d_time, with_range ? c->d_range : nullptr,
+    c->skeys_tmp));
+  return FSPH_OK;
+}
+
 fsph_status fsph_eos_init(fsph_ctx * c) { return elem(c, OP_EOS_INIT, FSPH_TIMER_INTEGRATE); }
 fsph_status fsph_set_total_energy(fsph_ctx * c) {
   return elem(c, OP_SET_TOTAL_ENERGY, FSPH_TIMER_INTEGRATE);
@@ -1186,15 +1205,17 @@ fsph_status fsph_compute_dt(fsph_ctx * c) {
     return s;
   Launch L = c->L();
   Phase ph(c, FSPH_TIMER_DT);
-  CK(launch_compute_dt(L, c->P, c->pp, c->d_time, c->d_status, 0, c->mixed));
+  CK(launch_compute_dt(L, c->P, c->pp, c->d_time, c->d_status, 0, c->mixed, 0));
   return FSPH_OK;
 }
 
-// compute_dt preceded by check_nans and check_negativity in one pass
-static fsph_status checks_and_dt(fsph_ctx * c) {
+// check_nans, check_negativity, compute_dt, set_adaptive_timestep and
+// advance_time, the end of a driver iteration, in one pass
+static fsph_status checks_dt_advance(fsph_ctx * c) {
   Launch L = c->L();
   Phase ph(c, FSPH_TIMER_DT);
-  CK(launch_compute_dt(L, c->P, c->pp, c->d_time, c->d_status, 1, c->mixed));
+  CK(launch_compute_dt(L, c->P, c->pp, c->d_time, c->d_status, 1, c->mixed, 1));
+  c->iteration++;
   return FSPH_OK;
 }
 
@@ -1532,8 +1553,9 @@ fsph_status fsph_step(fsph_ctx * c) {
     }
   }
   else {
-    TRY(elem(c, !evolve ? OP_KICK_DRIFT_NONE : (thermo ? OP_KICK_DRIFT_E : OP_KICK_DRIFT_U),
-      FSPH_TIMER_INTEGRATE));
+    // (periodic copies move the range after the drift)
+    TRY(kick_drift(c, !evolve ? OP_KICK_DRIFT_NONE : (thermo ? OP_KICK_DRIFT_E : OP_KICK_DRIFT_U),
+      !c->periodic));
     // fields the rest of the iteration writes before reading stay behind
     // in the permute
     unsigned skip = (1u << F_AX) | (1u << F_AY) | (1u << F_GAX) | (1u << F_GAY) |
@@ -1549,7 +1571,7 @@ fsph_status fsph_step(fsph_ctx * c) {
     if(evolve && !thermo)
       skip |= 1u << F_DUDT;
     c->permute_skip = skip;
-    const fsph_status us = fsph_update_iteration(c);
+    const fsph_status us = update_iteration(c, !c->periodic);
     c->permute_skip = 0;
     TRY(us);
     TRY(io_stage(c, IO_UPDATE));
@@ -1605,13 +1627,11 @@ fsph_status fsph_step(fsph_ctx * c) {
   else if(p.sph_update_uniform_h)
     TRY(fsph_compute_average_smoothinglength(c));
   if(p.adaptive_timestep) {
-    TRY(checks_and_dt(c));
-    TRY(fsph_set_adaptive_timestep(c));
+    TRY(checks_dt_advance(c));
+    return FSPH_OK;
   }
-  else {
-    TRY(fsph_check_nans(c));
-    TRY(fsph_check_negativity(c));
-  }
+  TRY(fsph_check_nans(c));
+  TRY(fsph_check_negativity(c));
   return fsph_advance_time(c);
 }
 

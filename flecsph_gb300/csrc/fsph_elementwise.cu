@@ -3,22 +3,13 @@
 // compiled with -fmad=false so they round like the reference.
 #include <cuda_runtime.h>
 
+#include "fsph_range.cuh"
 #include "fsph_sphmath.cuh"
 
 namespace fsph {
 
 #define ELEM_THREADS 256
 
-__device__ __forceinline__ unsigned long long ord_enc_e(double x) {
-  long long b = __double_as_longlong(x);
-  return b < 0 ? ~(unsigned long long)b
-               : ((unsigned long long)b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double ord_dec_e(unsigned long long u) {
-  return (u & 0x8000000000000000ull)
-           ? __longlong_as_double((long long)(u & 0x7fffffffffffffffull))
-           : __longlong_as_double((long long)~u);
-}
 __device__ __forceinline__ double dmin_(double a, double b) { return b < a ? b : a; }
 
 // recover_internal_energy (default_physics.h:126-145)
@@ -89,24 +80,6 @@ __global__ void __launch_bounds__(ELEM_THREADS) k_elem(Particles P,
       for(int d = 0; d < D; ++d)
         f[F_X + d][i] = f[F_X + d][i] + f[F_VX + d][i] * dt;
       break;
-    case OP_KICK_DRIFT_E:
-    case OP_KICK_DRIFT_U:
-    case OP_KICK_DRIFT_NONE: {
-      // the start of a leapfrog step, hydro/main_driver.cc:176-188:
-      // kick e (or u), kick v, save v_half, drift
-      if(op == OP_KICK_DRIFT_E)
-        f[F_E][i] = f[F_E][i] + 0.5 * dt * f[F_DEDT][i];
-      else if(op == OP_KICK_DRIFT_U)
-        f[F_U][i] = f[F_U][i] + 0.5 * dt * f[F_DUDT][i];
-      const double s = 0.5 * dt;
-      for(int d = 0; d < D; ++d) {
-        double v = f[F_VX + d][i] + (f[F_AX + d][i] + f[F_GAX + d][i]) * s;
-        f[F_VX + d][i] = v;
-        f[F_VHX + d][i] = v;
-        f[F_X + d][i] = f[F_X + d][i] + v * dt;
-      }
-      break;
-    }
     case OP_RECOMPUTE:
     case OP_RECOMPUTE_KICK_U: {  // default_physics.h:153-161 (+ kick_u)
       double uint = f[F_U][i];
@@ -202,8 +175,86 @@ cudaError_t launch_elementwise(const Launch & L, const Particles & P,
   return cudaGetLastError();
 }
 
+// The start of a leapfrog step, hydro/main_driver.cc:176-188: kick e (or u),
+// kick v, save v_half, drift; with RANGE the range of the drifted positions is
+// gathered on the way, which a pass of its own would read them again for.
+template<int D, int OP, bool RANGE>
+__global__ void __launch_bounds__(ELEM_THREADS) k_kick_drift(Particles P,
+  const DevTime * tm, unsigned long long * range, unsigned long long * part) {
+  double ** f = P.f;
+  const double dt = tm->dt, s = 0.5 * dt;
+  RangeAcc<D> r;
+  if(RANGE)
+    r.init(f[F_H][0]);
+  auto drift = [&](int i, int d, double & v) {
+    // (a + 0 is a but for a = -0, whose sum with v is v all the same)
+    const double g = f[F_GAX + d][i];
+    double a = f[F_AX + d][i];
+    if((__double_as_longlong(g) << 1) != 0)
+      a = add_rare(a, g);
+    v = f[F_VX + d][i] + a * s;
+    return f[F_X + d][i] + v * dt;
+  };
+  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n;
+      i += gridDim.x * blockDim.x) {
+    if(OP == OP_KICK_DRIFT_E)
+      f[F_E][i] = f[F_E][i] + 0.5 * dt * f[F_DEDT][i];
+    else if(OP == OP_KICK_DRIFT_U)
+      f[F_U][i] = f[F_U][i] + 0.5 * dt * f[F_DUDT][i];
+    double x[3] = {0.0, 0.0, 0.0};
+    for(int d = 0; d < D; ++d) {
+      double v;
+      x[d] = drift(i, d, v);
+      f[F_VX + d][i] = v;
+      f[F_VHX + d][i] = v;
+      f[F_X + d][i] = x[d];
+    }
+    if(RANGE)
+      r.add(x, f[F_H][i]);
+  }
+  if(RANGE) {
+    // (the last particle lies in its own [x - h, x + h]: the reference's start
+    // from its coordinates changes nothing, and another block may hold it)
+    r.finish(range, part, nullptr);
+  }
+}
+
+cudaError_t launch_kick_drift(const Launch & L, const Particles & P, const PhysParams & pp,
+  int op, const DevTime * t, unsigned long long * range, unsigned long long * range_part) {
+  int nb = (P.n + ELEM_THREADS - 1) / ELEM_THREADS;
+  if(range && nb > RANGE_BLOCKS)
+    nb = RANGE_BLOCKS;
+#define KD_LAUNCH(D, OP)                                                       \
+  do {                                                                         \
+    if(range)                                                                  \
+      k_kick_drift<D, OP, true><<<nb, ELEM_THREADS, 0, L.stream>>>(P, t, range, range_part); \
+    else                                                                       \
+      k_kick_drift<D, OP, false><<<nb, ELEM_THREADS, 0, L.stream>>>(P, t, nullptr, nullptr); \
+  } while(0)
+#define KD_OP(D)                                                               \
+  do {                                                                         \
+    if(op == OP_KICK_DRIFT_E)                                                  \
+      KD_LAUNCH(D, OP_KICK_DRIFT_E);                                           \
+    else if(op == OP_KICK_DRIFT_U)                                             \
+      KD_LAUNCH(D, OP_KICK_DRIFT_U);                                           \
+    else                                                                       \
+      KD_LAUNCH(D, OP_KICK_DRIFT_NONE);                                        \
+  } while(0)
+  if(pp.dim == 3)
+    KD_OP(3);
+  else
+    KD_OP(2);
+#undef KD_OP
+#undef KD_LAUNCH
+  *L.counter += 1;
+  return cudaGetLastError();
+}
+
 // compute_dt (default_physics.h:602-695) per particle, then the minimum.
-__global__ void k_dt_init(DevTime * t) { t->dtmin_bits = ord_enc_e(1e24); }
+// FP32 constants of the single-precision estimate
+struct DtConst {
+  float eta_kw, cfl, sig;  // eta times the kernel width, cfl, 1 + 0.6 alpha
+};
 
 // NaN / negativity from the bit pattern: integer instructions instead of
 // FP64 compares, which run on this part's narrow FP64 pipe.
@@ -217,139 +268,14 @@ __device__ __forceinline__ bool bits_negative(double x) {  // x < 0, not -0, not
          (b & 0x7fffffffffffffffull) <= 0x7ff0000000000000ull;
 }
 
-// CHECKS folds check_nans and check_negativity (default_physics.h:918-979)
-// into the same pass, as the driver runs them back to back before dt.
-// F32 evaluates the per-particle estimate of compute_dt in single precision
-// (mixed-precision runs); the global minimum and the adaptive rule stay FP64.
-template<int D, bool CHECKS, bool F32>
-__global__ void __launch_bounds__(ELEM_THREADS) k_compute_dt(Particles P,
-  PhysParams pp, DevTime * tm, DevStatus * st) {
-  // grid-stride: one atomic per block of a grid sized to the machine
-  double dtmin = 1e24;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n;
-      i += gridDim.x * blockDim.x) {
-    double ** f = P.f;
-    double dtp = 1e24;
-    if(CHECKS) {
-      bool bad = false;
-      for(int d = 0; d < D; ++d)
-        bad |= bits_nan(f[F_X + d][i]) | bits_nan(f[F_VX + d][i]) |
-               bits_nan(f[F_VHX + d][i]) | bits_nan(f[F_AX + d][i]) |
-               bits_nan(f[F_GAX + d][i]);
-      const int sc[] = {F_M, F_GPOT, F_RHO, F_P, F_E, F_DEDT, F_DUDT, F_K, F_VSIG};
-      for(int k = 0; k < 9; ++k)
-        bad |= bits_nan(f[sc[k]][i]);
-      if(pp.evolve_u)
-        bad |= bits_nan(f[F_U][i]);
-      if(bad)
-        raise_status(st, FSPH_ERR_NAN, i);
-      if(bits_negative(f[F_RHO][i]) || bits_negative(f[F_P][i]) ||
-         (pp.evolve_u && bits_negative(f[F_U][i])))
-        raise_status(st, FSPH_ERR_NEGATIVITY, i);
-    }
-    if(F32) {
-      const float tiny = 1e-24f;
-      const float dx = (float)f[F_H][i] / (float)(pp.eta * pp.kw);
-      float vn = 0.f, acc = 0.f;
-      for(int d = 0; d < D; ++d) {
-        const float v = (float)f[F_VX + d][i];
-        const float a = (float)(f[F_AX + d][i] + f[F_GAX + d][i]);
-        vn += v * v;
-        acc += a * a;
-      }
-      const float dt_v = dx / (sqrtf(vn) + tiny);
-      const float dt_a = sqrtf(dx / (sqrtf(acc) + tiny));
-      const float dt_c = dx / (tiny + (float)f[F_VSIG][i] * (1.f + 0.6f * (float)pp.alpha));
-      dtp = (double)((float)pp.cfl * fminf(fminf(dt_v, dt_a), dt_c));
-    }
-    else {
-      const double tiny = 1e-24, mc = 0.6;
-      const double dx = f[F_H][i] / (pp.eta * pp.kw);
-      double vn = 0;
-      for(int d = 0; d < D; ++d)
-        vn += f[F_VX + d][i] * f[F_VX + d][i];
-      vn = sqrt(vn);
-      const double dt_v = dx / (vn + tiny);
-      double acc = 0;
-      for(int d = 0; d < D; ++d) {
-        double ad = f[F_AX + d][i] + f[F_GAX + d][i];
-        acc += ad * ad;
-      }
-      acc = sqrt(acc);
-      const double dt_a = sqrt(dx / (acc + tiny));
-      const double dt_c = dx / (tiny + f[F_VSIG][i] * (1 + mc * pp.alpha));
-      dtp = pp.cfl * dmin_(dmin_(dt_v, dt_a), dt_c);
-    }
-    if(pp.evolve_u && pp.thermokinetic) {
-      const double eint = f[F_U][i];
-      if(!(eint > 0))
-        raise_status(st, FSPH_ERR_NEG_ENERGY, i);
-      double gdv = 0;
-      for(int d = 0; d < D; ++d)
-        gdv += f[F_VX + d][i] * f[F_GAX + d][i];
-      // with no external potential and v . g = 0, the first test passes
-      if(gdv != 0.0 || pp.n_eforce > 0) {
-        const double pos[3] = {f[F_X][i], f[F_Y][i], D == 3 ? f[F_Z][i] : 0.0};
-        const double epot = ext_potential<D>(pp, pos);
-        int it;
-        for(it = 0; it < 20; ++it) {
-          double p1[3] = {0.0, 0.0, 0.0};
-          for(int d = 0; d < D; ++d)
-            p1[d] = pos[d] + dtp * f[F_VX + d][i];
-          double delta_epot = ext_potential<D>(pp, p1) - epot;
-          double delta_egrv = -dtp * gdv;
-          if(delta_epot + delta_egrv < eint * 0.5)
-            break;
-          dtp *= 0.25;
-        }
-        if(it >= 20)
-          raise_status(st, FSPH_ERR_DT, i);
-      }
-    }
-    f[F_DT][i] = dtp;
-    dtmin = dmin_(dtmin, dtp);
-  }
-  // block minimum first, then one atomic per block
-  __shared__ double wmin[ELEM_THREADS / 32];
-  for(int o = 16; o; o >>= 1)
-    dtmin = dmin_(dtmin, __shfl_xor_sync(0xffffffffu, dtmin, o));
-  if((threadIdx.x & 31) == 0)
-    wmin[threadIdx.x >> 5] = dtmin;
-  __syncthreads();
-  if(threadIdx.x == 0) {
-    double m = wmin[0];
-    for(int k = 1; k < ELEM_THREADS / 32; ++k)
-      m = dmin_(m, wmin[k]);
-    atomicMin(&tm->dtmin_bits, ord_enc_e(m));
-  }
+__device__ __forceinline__ bool bits_positive(double x) {  // x > 0
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7ff0000000000000ll;
 }
 
-cudaError_t launch_compute_dt(const Launch & L, const Particles & P,
-  const PhysParams & pp, DevTime * t, DevStatus * st, int with_checks,
-  int f32) {
-  k_dt_init<<<1, 1, 0, L.stream>>>(t);
-  // a few blocks per SM: the per-block minima meet in one atomic each
-  int nb = (P.n + ELEM_THREADS - 1) / ELEM_THREADS;
-  if(nb > 152 * 8)
-    nb = 152 * 8;
-#define DT_LAUNCH(D, C, F) \
-  k_compute_dt<D, C, F><<<nb, ELEM_THREADS, 0, L.stream>>>(P, pp, t, st)
-  if(pp.dim == 3) {
-    if(with_checks) { if(f32) DT_LAUNCH(3, true, true); else DT_LAUNCH(3, true, false); }
-    else { if(f32) DT_LAUNCH(3, false, true); else DT_LAUNCH(3, false, false); }
-  }
-  else {
-    if(with_checks) { if(f32) DT_LAUNCH(2, true, true); else DT_LAUNCH(2, true, false); }
-    else { if(f32) DT_LAUNCH(2, false, true); else DT_LAUNCH(2, false, false); }
-  }
-#undef DT_LAUNCH
-  *L.counter += 2;
-  return cudaGetLastError();
-}
-
-// set_adaptive_timestep (default_physics.h:761-823), one thread.
-__global__ void k_set_adaptive(PhysParams pp, DevTime * t) {
-  double dtmin = ord_dec_e(t->dtmin_bits);
+// set_adaptive_timestep (default_physics.h:761-823)
+__device__ __forceinline__ void set_adaptive(const PhysParams & pp, DevTime * t) {
+  double dtmin = ord_dec(t->dtmin_bits);
   double dt = t->dt;
   if(dtmin < dt)
     dt = dmin_(dtmin, dt / 2.0);
@@ -391,6 +317,192 @@ __global__ void k_set_adaptive(PhysParams pp, DevTime * t) {
   t->dt = next - tt;
 }
 
+// advance_time (default_physics.h:853-860)
+__device__ __forceinline__ void advance(const PhysParams & pp, DevTime * t) {
+  t->iteration++;
+  if(pp.adaptive)
+    t->totaltime = t->totaltime_next;
+  else
+    t->totaltime = t->totaltime + t->dt;
+}
+
+// compute_dt's last rule: dt shrinks until the potential energy the particle
+// can take up in it stays below half of its internal energy.
+template<int D>
+__device__ __noinline__ double limit_dt(const PhysParams & pp, double * const * f, int i,
+  double eint, double dtp, DevStatus * st) {
+  double gdv = 0;
+  for(int d = 0; d < D; ++d)
+    gdv += f[F_VX + d][i] * f[F_GAX + d][i];
+  if(!(gdv != 0.0 || pp.n_eforce > 0))
+    return dtp;
+  const double pos[3] = {f[F_X][i], f[F_Y][i], D == 3 ? f[F_Z][i] : 0.0};
+  const double epot = ext_potential<D>(pp, pos);
+  int it;
+  for(it = 0; it < 20; ++it) {
+    double p1[3] = {0.0, 0.0, 0.0};
+    for(int d = 0; d < D; ++d)
+      p1[d] = pos[d] + dtp * f[F_VX + d][i];
+    double delta_epot = ext_potential<D>(pp, p1) - epot;
+    double delta_egrv = -dtp * gdv;
+    if(delta_epot + delta_egrv < eint * 0.5)
+      break;
+    dtp *= 0.25;
+  }
+  if(it >= 20)
+    raise_status(st, FSPH_ERR_DT, i);
+  return dtp;
+}
+
+// CHECKS folds check_nans and check_negativity (default_physics.h:918-979)
+// into the same pass, as the driver runs them back to back before dt.
+// F32 evaluates the per-particle estimate of compute_dt in single precision
+// (mixed-precision runs); the global minimum and the adaptive rule stay FP64.
+// FINISH: the last block to arrive also runs set_adaptive_timestep and
+// advance_time, which follow it in the driver's iteration.
+//
+// Tests against zero run on the bit patterns, and what gravity adds is left
+// out where g is zero: the FP64 pipe, not HBM, bounded this pass (30
+// operations a particle, 163 us at 2M particles; 101 now, HBM 52).
+template<int D, bool CHECKS, bool F32, bool FINISH>
+__global__ void __launch_bounds__(ELEM_THREADS) k_compute_dt(Particles P,
+  PhysParams pp, DtConst c32, DevTime * tm, DevStatus * st) {
+  // grid-stride: one atomic per block of a grid sized to the machine
+  unsigned long long dtmin = TIME_DT_MAX;  // ordered encoding
+  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n;
+      i += gridDim.x * blockDim.x) {
+    double ** f = P.f;
+    double dtp = 1e24;
+    double v[3] = {0.0, 0.0, 0.0}, g[3] = {0.0, 0.0, 0.0}, acc3[3] = {0.0, 0.0, 0.0};
+    bool still = true;  // g = 0, v finite: v . g = 0 and a + g = a
+    for(int d = 0; d < D; ++d) {
+      v[d] = f[F_VX + d][i];
+      g[d] = f[F_GAX + d][i];
+      acc3[d] = f[F_AX + d][i];
+      still = still && (__double_as_longlong(g[d]) << 1) == 0 &&
+              ((unsigned)__double2hiint(v[d]) & 0x7ff00000u) != 0x7ff00000u;
+    }
+    if(!still)
+      for(int d = 0; d < D; ++d)
+        acc3[d] = add_rare(acc3[d], g[d]);
+    if(CHECKS) {
+      bool bad = false;
+      for(int d = 0; d < D; ++d)
+        bad |= bits_nan(f[F_X + d][i]) | bits_nan(v[d]) | bits_nan(f[F_VHX + d][i]) |
+               bits_nan(f[F_AX + d][i]) | bits_nan(g[d]);
+      const int sc[] = {F_M, F_GPOT, F_RHO, F_P, F_E, F_DEDT, F_DUDT, F_K, F_VSIG};
+      for(int k = 0; k < 9; ++k)
+        bad |= bits_nan(f[sc[k]][i]);
+      if(pp.evolve_u)
+        bad |= bits_nan(f[F_U][i]);
+      if(bad)
+        raise_status(st, FSPH_ERR_NAN, i);
+      if(bits_negative(f[F_RHO][i]) || bits_negative(f[F_P][i]) ||
+         (pp.evolve_u && bits_negative(f[F_U][i])))
+        raise_status(st, FSPH_ERR_NEGATIVITY, i);
+    }
+    if(F32) {
+      const float tiny = 1e-24f;
+      const float dx = to_f32(f[F_H][i]) / c32.eta_kw;
+      float vn = 0.f, acc = 0.f;
+      for(int d = 0; d < D; ++d) {
+        const float vf = to_f32(v[d]), af = to_f32(acc3[d]);
+        vn += vf * vf;
+        acc += af * af;
+      }
+      const float dt_v = dx / (sqrtf(vn) + tiny);
+      const float dt_a = sqrtf(dx / (sqrtf(acc) + tiny));
+      const float dt_c = dx / (tiny + to_f32(f[F_VSIG][i]) * c32.sig);
+      dtp = to_f64(c32.cfl * fminf(fminf(dt_v, dt_a), dt_c));
+    }
+    else {
+      const double tiny = 1e-24, mc = 0.6;
+      const double dx = f[F_H][i] / (pp.eta * pp.kw);
+      double vn = 0;
+      for(int d = 0; d < D; ++d)
+        vn += v[d] * v[d];
+      vn = sqrt(vn);
+      const double dt_v = dx / (vn + tiny);
+      double acc = 0;
+      for(int d = 0; d < D; ++d)
+        acc += acc3[d] * acc3[d];
+      acc = sqrt(acc);
+      const double dt_a = sqrt(dx / (acc + tiny));
+      const double dt_c = dx / (tiny + f[F_VSIG][i] * (1 + mc * pp.alpha));
+      dtp = pp.cfl * dmin_(dmin_(dt_v, dt_a), dt_c);
+    }
+    if(pp.evolve_u && pp.thermokinetic) {
+      const double eint = f[F_U][i];
+      if(!bits_positive(eint))
+        raise_status(st, FSPH_ERR_NEG_ENERGY, i);
+      // with no external potential and v . g = 0, the first test passes
+      if(!still || pp.n_eforce > 0)
+        dtp = limit_dt<D>(pp, f, i, eint, dtp, st);
+    }
+    f[F_DT][i] = dtp;
+    if(!bits_nan(dtp))  // (as dmin_ would drop it)
+      dtmin = umin64(dtmin, ord_enc(dtp));
+  }
+  // block minimum first, then one atomic per block; the last block publishes
+  __shared__ unsigned long long wmin[ELEM_THREADS / 32];
+  for(int o = 16; o; o >>= 1)
+    dtmin = umin64(dtmin, __shfl_xor_sync(0xffffffffu, dtmin, o));
+  if((threadIdx.x & 31) == 0)
+    wmin[threadIdx.x >> 5] = dtmin;
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    unsigned long long m = wmin[0];
+    for(int k = 1; k < ELEM_THREADS / 32; ++k)
+      m = umin64(m, wmin[k]);
+    atomicMin(&tm->dtmin_acc, m);
+    __threadfence();
+    if(atomicAdd(&tm->ticket, 1u) == gridDim.x - 1) {
+      __threadfence();
+      tm->dtmin_bits = atomicExch(&tm->dtmin_acc, TIME_DT_MAX);
+      tm->ticket = 0u;
+      if(FINISH) {
+        set_adaptive(pp, tm);
+        advance(pp, tm);
+      }
+    }
+  }
+}
+
+cudaError_t launch_compute_dt(const Launch & L, const Particles & P,
+  const PhysParams & pp, DevTime * t, DevStatus * st, int with_checks,
+  int f32, int finish) {
+  // a few blocks per SM: the per-block minima meet in one atomic each
+  int nb = (P.n + ELEM_THREADS - 1) / ELEM_THREADS;
+  if(nb > 152 * 8)
+    nb = 152 * 8;
+  const DtConst c32 = {(float)(pp.eta * pp.kw), (float)pp.cfl,
+    1.f + 0.6f * (float)pp.alpha};
+#define DT_LAUNCH(D, C, F, E) \
+  k_compute_dt<D, C, F, E><<<nb, ELEM_THREADS, 0, L.stream>>>(P, pp, c32, t, st)
+#define DT_PICK(D)                                                             \
+  do {                                                                         \
+    if(with_checks && finish) {                                                \
+      if(f32) DT_LAUNCH(D, true, true, true); else DT_LAUNCH(D, true, false, true); \
+    }                                                                          \
+    else if(with_checks) {                                                     \
+      if(f32) DT_LAUNCH(D, true, true, false); else DT_LAUNCH(D, true, false, false); \
+    }                                                                          \
+    else {                                                                     \
+      if(f32) DT_LAUNCH(D, false, true, false); else DT_LAUNCH(D, false, false, false); \
+    }                                                                          \
+  } while(0)
+  if(pp.dim == 3)
+    DT_PICK(3);
+  else
+    DT_PICK(2);
+#undef DT_PICK
+#undef DT_LAUNCH
+  *L.counter += 1;
+  return cudaGetLastError();
+}
+
+__global__ void k_set_adaptive(PhysParams pp, DevTime * t) { set_adaptive(pp, t); }
+
 cudaError_t launch_set_adaptive_timestep(const Launch & L,
   const PhysParams & pp, DevTime * t) {
   k_set_adaptive<<<1, 1, 0, L.stream>>>(pp, t);
@@ -398,14 +510,7 @@ cudaError_t launch_set_adaptive_timestep(const Launch & L,
   return cudaGetLastError();
 }
 
-// advance_time (default_physics.h:853-860)
-__global__ void k_advance(PhysParams pp, DevTime * t) {
-  t->iteration++;
-  if(pp.adaptive)
-    t->totaltime = t->totaltime_next;
-  else
-    t->totaltime = t->totaltime + t->dt;
-}
+__global__ void k_advance(PhysParams pp, DevTime * t) { advance(pp, t); }
 
 cudaError_t launch_advance_time(const Launch & L, const PhysParams & pp,
   DevTime * t) {

@@ -28,8 +28,13 @@ struct DevTime {
   long long iteration;
   // global reductions written by kernels
   unsigned long long dtmin_bits;  // ordered encoding of min particle dt
+  unsigned long long dtmin_acc;   // the same while a pass gathers it (else TIME_DT_MAX)
+  unsigned ticket;                // blocks done in that pass (else 0)
   double hsum;                    // sum of h (average smoothing length)
 };
+
+// ordered encoding of 1e24, the largest particle dt
+#define TIME_DT_MAX 0xc4ea784379d99db4ull
 
 // First device-side error: code (fsph_status) and the particle it concerns.
 struct DevStatus {
@@ -37,6 +42,39 @@ struct DevStatus {
   int flags;  // reserved
   long long index;
 };
+
+// FP64 work that few particles need, out of line: inline, the compiler
+// predicates it, and an instruction with every lane off still takes its turn
+// in the FP64 pipe.
+static __device__ __noinline__ double add_rare(double a, double b) { return a + b; }
+static __device__ __noinline__ double2 widen_rare(double x, double h) {
+  return make_double2(x - h, x + h);
+}
+
+// double to float (rounded to nearest even, as the conversion instruction
+// does) and float to double, on the integer pipe: a conversion from or to 64
+// bits occupies the FP64 pipe like an addition, 16 cycles of an SM per warp on
+// this part, and per-particle passes are full of them.  Denormals, infinities
+// and NaN take the instruction.
+__device__ __forceinline__ float to_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  if(e - 897u < 253u) {
+    unsigned t = __funnelshift_l(lo, hi, 3);  // low nine exponent bits, 23 mantissa bits
+    t += ((lo & 0x1fffffffu) + (t & 1u)) > 0x10000000u;
+    t -= 896u << 23;
+    return __uint_as_float((t & 0x7fffffffu) | (hi & 0x80000000u));
+  }
+  if(((hi << 1) | lo) == 0u)
+    return __uint_as_float(hi);
+  return (float)x;
+}
+__device__ __forceinline__ double to_f64(float x) {
+  const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if(m - 0x00800000u < 0x7f000000u)
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(b << 29));
+  return m == 0u ? __hiloint2double((int)b, 0) : (double)x;
+}
 
 struct Particles {
   double * f[NF];
@@ -235,18 +273,32 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long> * mask, F app
 }
 
 // ---- fsph_tree.cu ----
-cudaError_t launch_range_keys(const Launch & L, const Particles & P,
-  const PhysParams & pp, double * d_range, unsigned long long * keys_out,
-  int * idx_out);
+// Range words: [0..7] ordered encodings (x - h minima, x + h maxima, h minimum
+// and maximum), [8] blocks done (0 between passes).  range_part: RANGE_PART
+// words of scratch, free until the keys are sorted.
+#define RANGE_WORDS 9
+#define RANGE_BLOCKS (152 * 8)
+#define RANGE_PART (8 * RANGE_BLOCKS)
+cudaError_t launch_range(const Launch & L, const Particles & P, const PhysParams & pp,
+  unsigned long long * range, unsigned long long * range_part);
+cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams & pp,
+  const unsigned long long * range, unsigned long long * keys_out, int * idx_out);
 // `bits`: the data bits of the keys, below a constant marker bit
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
   unsigned * hist, int bits);
 size_t radix_hist_entries(int n);
+// the fields not in `skip`, id and key[i] in the order of perm
+cudaError_t launch_gather(const Launch & L, const Particles & src, const Particles & dst,
+  const int * perm, const unsigned long long * keys, unsigned skip);
+struct Packed;
+// Writes the position records of the new order on the way (Packed::qpos, fph,
+// fpl, fmA), with the range's scales, and empties the group and list counts
+// for the tree build and the walk.
 cudaError_t launch_permute(const Launch & L, const Particles & src,
   const Particles & dst, const int * perm, const unsigned long long * keys,
-  unsigned skip, float4 * vel = nullptr, int dim = 3);
-struct Packed;
+  unsigned skip, const unsigned long long * rbits, const Packed & K, int * ngroups,
+  unsigned * list_stat, float4 * vel, int dim);
 cudaError_t launch_build_tree(const Launch & L, const Particles & P,
   const PhysParams & pp, Tree & T, int group_max,
   const unsigned long long * rbits, const int4 * qpos, const float * qscale, int ordered,
@@ -256,11 +308,6 @@ cudaError_t launch_neighbors(const Launch & L, const Particles & P,
   const unsigned long long * rbits, const Packed & K, int ordered);
 
 // ---- fsph_mixed.cu ----
-// also empties the tree's group count and the list statistics for the build
-// that follows
-cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
-  const PhysParams & pp, const unsigned long long * rbits, const Packed & K, int * ngroups,
-  unsigned * list_stat);
 cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, double * cs_new,
   DevStatus * st, const DevTime * tm, int vel_current);
@@ -348,9 +395,15 @@ enum ElemOp {
 };
 cudaError_t launch_elementwise(const Launch & L, const Particles & P,
   const PhysParams & pp, int op, DevTime * t, DevStatus * st);
+// finish: the last block also sets the adaptive timestep and advances the time
+// (set_adaptive_timestep and advance_time of the driver's iteration)
 cudaError_t launch_compute_dt(const Launch & L, const Particles & P,
   const PhysParams & pp, DevTime * t, DevStatus * st, int with_checks,
-  int f32);
+  int f32, int finish);
+// the fused kick, save v_half and drift of a driver iteration (op one of
+// OP_KICK_DRIFT_*), with the range of the drifted positions if `range`
+cudaError_t launch_kick_drift(const Launch & L, const Particles & P, const PhysParams & pp,
+  int op, const DevTime * t, unsigned long long * range, unsigned long long * range_part);
 cudaError_t launch_set_adaptive_timestep(const Launch & L,
   const PhysParams & pp, DevTime * t);
 cudaError_t launch_advance_time(const Launch & L, const PhysParams & pp,

@@ -10,72 +10,7 @@ namespace fsph {
 
 static_assert(SPLIT_MAX <= LIST_STAT_MAX, "the walk keeps the statistics the passes read");
 
-__device__ __forceinline__ double ord_dec_m(unsigned long long u) {
-  return (u & 0x8000000000000000ull)
-           ? __longlong_as_double((long long)(u & 0x7fffffffffffffffull))
-           : __longlong_as_double((long long)~u);
-}
-
 // ------------------------------------------------------------- packing --
-__global__ void k_pack_pos(Particles P, int dim,
-  const unsigned long long * rbits, Packed K, int * ngroups, unsigned * list_stat) {
-  // Every position as one 48-bit fixed-point word per axis,
-  //   F = round((x - lo) / E * 2^48),  E = the largest range extent
-  //   enlarged by 2^-19 (so F < 2^48 - 2^28),
-  // from which both packed forms follow by integer operations:
-  //   float-float X = 1 + F / 2^48 in [1, 2): the high word takes F's top
-  //     23 bits (exactly), the low word the other 25 (rounded to 24 bits);
-  //   the walk's 31-bit fixed point q = F / 2^17 rounded to nearest, one
-  //     step = E / 2^31 on every axis.
-  // Three FP64 operations per axis (subtract, scale, convert): this kernel
-  // runs on GB300's FP64 pipe, where divisions and splits cost most.
-  __shared__ double s_lo[3], s_sc, s_iE;
-  if(threadIdx.x < dim)
-    s_lo[threadIdx.x] = ord_dec_m(rbits[threadIdx.x]);
-  if(threadIdx.x == 0) {
-    double E = 0.0;
-    for(int d = 0; d < dim; ++d)
-      E = fmax(E, ord_dec_m(rbits[3 + d]) - ord_dec_m(rbits[d]));
-    E *= 1.0 + 0x1p-19;
-    s_iE = 1.0 / E;
-    s_sc = s_iE * 0x1p48;
-    if(blockIdx.x == 0) {
-      *ngroups = 0;
-      list_stat[0] = list_stat[1] = 0u;
-      K.fscale[0] = E;
-      K.fscale[1] = s_iE;
-      // h_min == h_max: the pair passes take h_ab = h_a throughout
-      K.fscale[2] = rbits[6] == rbits[7] ? 1.0 : 0.0;
-      for(int d = 0; d < 3; ++d)
-        K.qscale[d] = d < dim ? (float)(E * 0x1p-31) : 0.f;
-    }
-  }
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= P.n)
-    return;
-  const long long fmax48 = (1LL << 48) - (1LL << 28);
-  int q[3] = {0, 0, 0};
-  float xh[4] = {1.f, 1.f, 1.f, 0.f}, xl[4] = {0.f, 0.f, 0.f, 0.f};
-  for(int d = 0; d < dim; ++d) {
-    long long F = __double2ll_rn((P.f[F_X + d][i] - s_lo[d]) * s_sc);
-    F = F < 0 ? 0 : F > fmax48 ? fmax48 : F;
-    q[d] = (int)((F + (1LL << 16)) >> 17);
-    xh[d] = __int_as_float(0x3f800000 | (int)(F >> 25));
-    xl[d] = (float)(int)(F & ((1LL << 25) - 1)) * 0x1p-48f;
-  }
-  const double h = P.f[F_H][i];
-  const double hX = h * s_iE;
-  xh[3] = (float)hX;
-  xl[3] = (float)(hX - (double)xh[3]);
-  K.qpos[i] = make_int4(q[0], q[1], q[2], __float_as_int((float)h));
-  K.fph[i] = make_float4(xh[0], xh[1], xh[2], xh[3]);
-  K.fpl[i] = make_float4(xl[0], xl[1], xl[2], xl[3]);
-  const double m = P.f[F_M][i];
-  const float mh = (float)m;
-  ((float2 *)K.fmA)[2 * i] = make_float2(mh, (float)(m - (double)mh));
-}
-
 // PACK_VHM: {v_half, m} and m alone (the FP32 passes, the alpha pass);
 // PACK_VEL: {v, c_s before the density pass} (the signal speed);
 // PACK_AV_IN: {c_s, sign(div v)} for the Cullen & Dehnen alpha pass;
@@ -100,33 +35,33 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
   // FP32 high word and low word of an FP64 velocity component
   auto hl = [&](int f, float & h, float & l) {
     const double v = P.f[f][i];
-    h = (float)v;
-    l = (float)(v - (double)h);
+    h = to_f32(v);
+    l = to_f32(v - to_f64(h));
   };
   if(what & (PACK_VHM | PACK_FV)) {
     float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
     for(int d = 0; d < dim; ++d)
       hl(F_VHX + d, h[d], l[d]);
     if(what & PACK_VHM) {
-      const float m = (float)P.f[F_M][i];
+      const float m = to_f32(P.f[F_M][i]);
       K.vhm[i] = make_float4(h[0], h[1], h[2], m);
       K.mass[i] = m;
     }
     if(what & PACK_FV) {
       // rho and c_s as the state holds them: after the density pass, the
       // new c_s
-      K.fv1[i] = make_float4(h[0], h[1], h[2], (float)P.f[F_RHO][i]);
-      K.fv2[i] = make_float4(l[0], l[1], l[2], (float)P.f[F_CS][i]);
+      K.fv1[i] = make_float4(h[0], h[1], h[2], to_f32(P.f[F_RHO][i]));
+      K.fv2[i] = make_float4(l[0], l[1], l[2], to_f32(P.f[F_CS][i]));
     }
   }
   if(what & PACK_VEL)
-    K.vel[i] = make_float4((float)P.f[F_VX][i], (float)P.f[F_VY][i],
-      dim == 3 ? (float)P.f[F_VZ][i] : 0.f, (float)P.f[F_CS][i]);
+    K.vel[i] = make_float4(to_f32(P.f[F_VX][i]), to_f32(P.f[F_VY][i]),
+      dim == 3 ? to_f32(P.f[F_VZ][i]) : 0.f, to_f32(P.f[F_CS][i]));
   if(what & PACK_VEL_V) {
     float * v = (float *)&K.vel[i];
-    v[0] = (float)P.f[F_VX][i];
-    v[1] = (float)P.f[F_VY][i];
-    v[2] = dim == 3 ? (float)P.f[F_VZ][i] : 0.f;
+    v[0] = to_f32(P.f[F_VX][i]);
+    v[1] = to_f32(P.f[F_VY][i]);
+    v[2] = dim == 3 ? to_f32(P.f[F_VZ][i]) : 0.f;
   }
   if(what & PACK_THERMO) {
     const double rho = P.f[F_RHO][i], cs = P.f[F_CS][i];
@@ -139,30 +74,22 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
     // signnum_c of the reference (viscosity.h:63-67), taken in FP64
     const double dv = P.f[F_DIVV][i];
     const float sgn = dv > 0.0 ? 1.f : (dv < 0.0 ? -1.f : (float)dv);
-    K.visc[i] = make_float2((float)P.f[F_CS][i], sgn);
+    K.visc[i] = make_float2(to_f32(P.f[F_CS][i]), sgn);
   }
   if(what & PACK_AV)
-    K.visc[i] = make_float2((float)P.f[F_ALPHA][i], 0.f);
+    K.visc[i] = make_float2(to_f32(P.f[F_ALPHA][i]), 0.f);
   if(what & PACK_DEDT) {
     const double rho = P.f[F_RHO][i];
-    K.velp[i] = make_float4((float)P.f[F_VX][i], (float)P.f[F_VY][i],
-      dim == 3 ? (float)P.f[F_VZ][i] : 0.f, (float)(P.f[F_P][i] / (rho * rho)));
-    K.rc[i] = make_float2((float)rho, (float)P.f[F_CS][i]);
+    K.velp[i] = make_float4(to_f32(P.f[F_VX][i]), to_f32(P.f[F_VY][i]),
+      dim == 3 ? to_f32(P.f[F_VZ][i]) : 0.f, (float)(P.f[F_P][i] / (rho * rho)));
+    K.rc[i] = make_float2((float)rho, to_f32(P.f[F_CS][i]));
   }
   if(what & PACK_FDV) {
     float dv[3] = {0.f, 0.f, 0.f};
     for(int d = 0; d < dim; ++d)
       dv[d] = (float)(P.f[F_VX + d][i] - P.f[F_VHX + d][i]);
-    K.fdv[i] = make_float4(dv[0], dv[1], dv[2], (float)P.f[F_M][i]);
+    K.fdv[i] = make_float4(dv[0], dv[1], dv[2], to_f32(P.f[F_M][i]));
   }
-}
-
-cudaError_t launch_pack_positions(const Launch & L, const Particles & P,
-  const PhysParams & pp, const unsigned long long * rbits, const Packed & K,
-  int * ngroups, unsigned * list_stat) {
-  k_pack_pos<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, rbits, K, ngroups, list_stat);
-  *L.counter += 1;
-  return cudaGetLastError();
 }
 
 // -------------------------------------------------------- signal speed --

@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "fsph_internal.cuh"
+#include "fsph_range.cuh"
 
 namespace fsph {
 
@@ -19,94 +20,30 @@ namespace cg = cooperative_groups;
 
 #define FULL 0xffffffffu
 
-__device__ __forceinline__ unsigned long long ord_enc(double x) {
-  long long b = __double_as_longlong(x);
-  return b < 0 ? ~(unsigned long long)b
-               : ((unsigned long long)b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double ord_dec(unsigned long long u) {
-  return (u & 0x8000000000000000ull)
-           ? __longlong_as_double((long long)(u & 0x7fffffffffffffffull))
-           : __longlong_as_double((long long)~u);
-}
-
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
 }
 
-__device__ __forceinline__ unsigned long long umin64(unsigned long long a,
-  unsigned long long b) {
-  return b < a ? b : a;
-}
-
 // ---------------------------------------------------------------- range --
-// body_system::mpi_compute_range (mpisph/bodies_system.h:231-268): the
-// bounding box of [x - h, x + h] over all particles, initialised from the
-// last particle's coordinates.  min/max are exact in any order.
-__global__ void k_range_init(Particles P, int dim, unsigned long long * bits) {
-  int d = threadIdx.x;
-  if(d < dim) {
-    double x = P.f[F_X + d][P.n - 1];
-    bits[d] = ord_enc(x);
-    bits[3 + d] = ord_enc(x);
-  }
-  if(d == 0) {
-    bits[6] = ord_enc(1e308);
-    bits[7] = ord_enc(-1e308);
-  }
-}
-
-// The comparisons run on the ordered integer encodings (the integer pipe);
-// only x + h and x - h use the FP64 pipe, which is the bound of this
-// kernel on a part with GB300's FP64 rate.
-__global__ void __launch_bounds__(256) k_range_reduce(Particles P, int dim,
-  unsigned long long * bits) {
-  // v[k]: minima of the encodings of lo[0..2], h and of the complemented
-  // encodings of hi[0..2], h (so that every slot is a minimum)
-  unsigned long long v[8];
-  for(int k = 0; k < 8; ++k)
-    v[k] = ~0ull;
+template<int dim>
+__global__ void __launch_bounds__(256) k_range(Particles P, unsigned long long * range,
+  unsigned long long * part) {
   const double * H = P.f[F_H];
+  RangeAcc<dim> r;
+  r.init(H[0]);
   for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n;
       i += gridDim.x * blockDim.x) {
-    const double h = H[i];
-    const unsigned long long eh = ord_enc(h);
-    v[6] = umin64(v[6], eh);
-    v[7] = umin64(v[7], ~eh);
-    for(int d = 0; d < dim; ++d) {
-      const double x = P.f[F_X + d][i];
-      v[d] = umin64(v[d], ord_enc(x - h));
-      v[3 + d] = umin64(v[3 + d], ~ord_enc(x + h));
-    }
+    double x[3] = {0.0, 0.0, 0.0};
+    for(int d = 0; d < dim; ++d)
+      x[d] = P.f[F_X + d][i];
+    r.add(x, H[i]);
   }
-  // warp, then block, then one atomic per block and quantity
-  __shared__ unsigned long long red[8][8];
-  for(int k = 0; k < 8; ++k)
-    for(int o = 16; o; o >>= 1)
-      v[k] = umin64(v[k], __shfl_xor_sync(FULL, v[k], o));
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if(lane == 0)
-    for(int k = 0; k < 8; ++k)
-      red[w][k] = v[k];
-  __syncthreads();
-  if(threadIdx.x < 8) {
-    const int k = threadIdx.x;
-    unsigned long long m = red[0][k];
-    for(int q = 1; q < (int)(blockDim.x >> 5); ++q)
-      m = umin64(m, red[q][k]);
-    if(k < 3) {
-      if(k < dim) atomicMin(&bits[k], m);
-    }
-    else if(k < 6) {
-      if(k - 3 < dim) atomicMax(&bits[k], ~m);
-    }
-    else if(k == 6)
-      atomicMin(&bits[6], m);
-    else
-      atomicMax(&bits[7], ~m);
-  }
+  double last[3] = {0.0, 0.0, 0.0};
+  for(int d = 0; d < dim; ++d)
+    last[d] = P.f[F_X + d][P.n - 1];
+  r.finish(range, part, last);
 }
 
 // Morton key, morton_curve_u(range, p) (filling_curve.h:503-525): bit i of
@@ -131,12 +68,19 @@ __device__ __forceinline__ unsigned long long spread2(unsigned long long x) {
   return x;
 }
 
-__global__ void k_keys(Particles P, int dim, const unsigned long long * bits,
+// The reference quantises fl(t / scale) * 2^md, t = x - min.  t times the
+// reciprocal, scaled by a further 2^20, gives that value in fixed point to a
+// few units of its 20 fraction bits; only a fraction within KEY_MARGIN of an
+// integer leaves the integer part open, and there the correctly rounded
+// division decides.  Three FP64 operations an axis (subtract, multiply,
+// convert): the FP64 pipe bounds this kernel on this part.
+#define KEY_MARGIN 16u
+template<int dim>
+__global__ void __launch_bounds__(256) k_keys(Particles P, const unsigned long long * bits,
   unsigned long long * keys, int * idx) {
-  // the range and its reciprocal scaled by 2^md, once per block (FP64
-  // division is costly at this part's FP64 rate)
+  // the range and its scaled reciprocal, once per block
   __shared__ double s_mn[3], s_scale[3], s_rs[3];
-  const int md = 63 / dim;
+  constexpr int md = 63 / dim;
   const double mult = (double)(1ull << md);
   if(threadIdx.x < dim) {
     const int d = threadIdx.x;
@@ -144,29 +88,24 @@ __global__ void k_keys(Particles P, int dim, const unsigned long long * bits,
     const double scale = ord_dec(bits[3 + d]) - mn;
     s_mn[d] = mn;
     s_scale[d] = scale;
-    s_rs[d] = (1.0 / scale) * mult;
+    s_rs[d] = (1.0 / scale) * (mult * 1048576.0);
   }
   __syncthreads();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= P.n)
     return;
-  const unsigned long long maxv = (1ull << md) - 1;
+  constexpr unsigned long long maxv = (1ull << md) - 1;
   unsigned long long c[3] = {0, 0, 0};
   for(int d = 0; d < dim; ++d) {
-    const double mn = s_mn[d];
-    const double scale = s_scale[d];
-    const double t = P.f[F_X + d][i] - mn;
-    // The reference quantises fl(t / scale) * 2^md (a power of two, exact).
-    // t * (1 / scale) can differ from fl(t / scale) by an ulp, which moves
-    // the integer part only when the scaled value lies within ~7e-7 of an
-    // integer (2D: 2^31 scale); there the correctly rounded division decides.
-    // Scaling by 2^md commutes with rounding, so t * ((1 / scale) * 2^md)
-    // equals fl(t * (1 / scale)) * 2^md.
-    double q = t * s_rs[d];
-    const double fq = floor(q);
-    if(q - fq < 1e-5 || q - fq > 1.0 - 1e-5)
-      q = t / scale * mult;
-    unsigned long long u = q > 0.0 ? __double2ull_rz(q) : 0ull;
+    const double t = P.f[F_X + d][i] - s_mn[d];
+    // saturates at 0 below and far above maxv
+    const unsigned long long F = __double2ull_rz(t * s_rs[d]);
+    unsigned long long u = F >> 20;
+    const unsigned frac = (unsigned)F & 0xfffffu;
+    if(frac - KEY_MARGIN > 0xfffffu - 2u * KEY_MARGIN) {
+      const double q = t / s_scale[d] * mult;
+      u = q > 0.0 ? __double2ull_rz(q) : 0ull;
+    }
     c[d] = u < maxv ? u : maxv;
   }
   unsigned long long k;
@@ -178,18 +117,27 @@ __global__ void k_keys(Particles P, int dim, const unsigned long long * bits,
   idx[i] = i;
 }
 
-cudaError_t launch_range_keys(const Launch & L, const Particles & P,
-  const PhysParams & pp, double * d_range, unsigned long long * keys_out,
-  int * idx_out) {
-  unsigned long long * bits = (unsigned long long *)d_range;
-  k_range_init<<<1, 32, 0, L.stream>>>(P, pp.dim, bits);
+cudaError_t launch_range(const Launch & L, const Particles & P, const PhysParams & pp,
+  unsigned long long * range, unsigned long long * range_part) {
   int nb = (P.n + 255) / 256;
-  if(nb > 152 * 8)
-    nb = 152 * 8;
-  k_range_reduce<<<nb, 256, 0, L.stream>>>(P, pp.dim, bits);
-  k_keys<<<(P.n + 255) / 256, 256, 0, L.stream>>>(P, pp.dim, bits, keys_out,
-    idx_out);
-  *L.counter += 3;
+  if(nb > RANGE_BLOCKS)
+    nb = RANGE_BLOCKS;
+  if(pp.dim == 3)
+    k_range<3><<<nb, 256, 0, L.stream>>>(P, range, range_part);
+  else
+    k_range<2><<<nb, 256, 0, L.stream>>>(P, range, range_part);
+  *L.counter += 1;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams & pp,
+  const unsigned long long * range, unsigned long long * keys_out, int * idx_out) {
+  const int nb = (P.n + 255) / 256;
+  if(pp.dim == 3)
+    k_keys<3><<<nb, 256, 0, L.stream>>>(P, range, keys_out, idx_out);
+  else
+    k_keys<2><<<nb, 256, 0, L.stream>>>(P, range, keys_out, idx_out);
+  *L.counter += 1;
   return cudaGetLastError();
 }
 
@@ -724,28 +672,101 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
 // them before anything reads them.  With `vel`, the mixed path's
 // {v, c_s} record of the new order is written on the way (what the density
 // pass would otherwise pack).
-__global__ void k_permute(Particles src, Particles dst, const int * perm,
-  const unsigned long long * keys, unsigned skip, float4 * vel, int dim) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// The gather is bound by HBM; the position records of the tree, the walk and
+// the float-float passes, whose arithmetic is FP64 and which a pass of their
+// own would read five fields for again, come out of it too.  Every position is
+// one 48-bit fixed-point word per axis,
+//   F = round((x - lo) / E * 2^48),  E = the largest range extent
+//   enlarged by 2^-19 (so F < 2^48 - 2^28),
+// from which both packed forms follow by integer operations:
+//   float-float X = 1 + F / 2^48 in [1, 2): the high word takes F's top
+//     23 bits (exactly), the low word the other 25 (rounded to 24 bits);
+//   the walk's 31-bit fixed point q = F / 2^17 rounded to nearest, one
+//     step = E / 2^31 on every axis.
+template<int dim>
+__global__ void __launch_bounds__(256) k_permute(Particles src, Particles dst,
+  const int * perm, const unsigned long long * keys, unsigned skip,
+  const unsigned long long * rbits, Packed K, int * ngroups, unsigned * list_stat,
+  float4 * vel) {
+  __shared__ double s_lo[3], s_sc, s_iE;
+  if(dim > 0 && threadIdx.x < dim)
+    s_lo[threadIdx.x] = ord_dec(rbits[threadIdx.x]);
+  if(dim > 0 && threadIdx.x == 0) {
+    double E = 0.0;
+    for(int d = 0; d < dim; ++d)
+      E = fmax(E, ord_dec(rbits[3 + d]) - ord_dec(rbits[d]));
+    E *= 1.0 + 0x1p-19;
+    s_iE = 1.0 / E;
+    s_sc = s_iE * 0x1p48;
+    if(blockIdx.x == 0) {
+      *ngroups = 0;
+      list_stat[0] = list_stat[1] = 0u;
+      K.fscale[0] = E;
+      K.fscale[1] = s_iE;
+      // h_min == h_max: the pair passes take h_ab = h_a throughout
+      K.fscale[2] = rbits[6] == rbits[7] ? 1.0 : 0.0;
+      for(int d = 0; d < 3; ++d)
+        K.qscale[d] = d < dim ? (float)(E * 0x1p-31) : 0.f;
+    }
+  }
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= src.n)
     return;
-  int p = perm[i];
+  const int p = perm[i];
 #pragma unroll
   for(int k = 0; k < NF; ++k)
     if(!((skip >> k) & 1u))
       dst.f[k][i] = src.f[k][p];
   dst.id[i] = src.id[p];
   dst.key[i] = keys[i];
+  if(dim == 0)  // a plain gather
+    return;
   if(vel)
-    vel[i] = make_float4((float)src.f[F_VX][p], (float)src.f[F_VY][p],
-      dim == 3 ? (float)src.f[F_VZ][p] : 0.f, (float)src.f[F_CS][p]);
+    vel[i] = make_float4(to_f32(src.f[F_VX][p]), to_f32(src.f[F_VY][p]),
+      dim == 3 ? to_f32(src.f[F_VZ][p]) : 0.f, to_f32(src.f[F_CS][p]));
+  const long long fmax48 = (1LL << 48) - (1LL << 28);
+  int q[3] = {0, 0, 0};
+  float xh[4] = {1.f, 1.f, 1.f, 0.f}, xl[4] = {0.f, 0.f, 0.f, 0.f};
+  for(int d = 0; d < dim; ++d) {
+    long long F = __double2ll_rn((src.f[F_X + d][p] - s_lo[d]) * s_sc);
+    F = F < 0 ? 0 : F > fmax48 ? fmax48 : F;
+    q[d] = (int)((F + (1LL << 16)) >> 17);
+    xh[d] = __int_as_float(0x3f800000 | (int)(F >> 25));
+    xl[d] = (float)(int)(F & ((1LL << 25) - 1)) * 0x1p-48f;
+  }
+  const double h = src.f[F_H][p];
+  const double hX = h * s_iE;
+  xh[3] = to_f32(hX);
+  xl[3] = to_f32(hX - to_f64(xh[3]));
+  K.qpos[i] = make_int4(q[0], q[1], q[2], __float_as_int(to_f32(h)));
+  K.fph[i] = make_float4(xh[0], xh[1], xh[2], xh[3]);
+  K.fpl[i] = make_float4(xl[0], xl[1], xl[2], xl[3]);
+  const double m = src.f[F_M][p];
+  const float mh = to_f32(m);
+  ((float2 *)K.fmA)[2 * i] = make_float2(mh, to_f32(m - to_f64(mh)));
+}
+
+cudaError_t launch_gather(const Launch & L, const Particles & src, const Particles & dst,
+  const int * perm, const unsigned long long * keys, unsigned skip) {
+  k_permute<0><<<(src.n + 255) / 256, 256, 0, L.stream>>>(src, dst, perm, keys, skip,
+    nullptr, Packed{}, nullptr, nullptr, nullptr);
+  *L.counter += 1;
+  return cudaGetLastError();
 }
 
 cudaError_t launch_permute(const Launch & L, const Particles & src,
   const Particles & dst, const int * perm, const unsigned long long * keys,
-  unsigned skip, float4 * vel, int dim) {
-  k_permute<<<(src.n + 255) / 256, 256, 0, L.stream>>>(src, dst, perm, keys, skip, vel,
-    dim);
+  unsigned skip, const unsigned long long * rbits, const Packed & K, int * ngroups,
+  unsigned * list_stat, float4 * vel, int dim) {
+  const int nb = (src.n + 255) / 256;
+  if(dim == 3)
+    k_permute<3><<<nb, 256, 0, L.stream>>>(src, dst, perm, keys, skip, rbits, K, ngroups,
+      list_stat, vel);
+  else
+    k_permute<2><<<nb, 256, 0, L.stream>>>(src, dst, perm, keys, skip, rbits, K, ngroups,
+      list_stat, vel);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -2044,6 +2065,8 @@ cudaError_t launch_neighbors(const Launch & L, const Particles & P,
 // GPU loading the library holds until the process exits.
 #define FSPH_NOALLOC_SORT_MAX (1 << 20)
 #define NOALLOC_RANGE_BYTES 256
+static_assert(RANGE_WORDS * 8 <= NOALLOC_RANGE_BYTES &&
+                RANGE_PART <= FSPH_NOALLOC_SORT_MAX, "range scratch");
 #define NOALLOC_KEYS_BYTES ((size_t)FSPH_NOALLOC_SORT_MAX * 8)
 #define NOALLOC_VALS_BYTES ((size_t)FSPH_NOALLOC_SORT_MAX * 4)
 #define NOALLOC_HIST_BYTES \
@@ -2086,7 +2109,7 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
     base = g_noalloc_addr[dev];
   }
   unsigned char * b = (unsigned char *)base;
-  double * range = (double *)b;
+  unsigned long long * range = (unsigned long long *)b;
   unsigned long long * ktmp = (unsigned long long *)(b + NOALLOC_RANGE_BYTES);
   int * vtmp = (int *)(b + NOALLOC_RANGE_BYTES + NOALLOC_KEYS_BYTES);
   unsigned * hist =
@@ -2101,10 +2124,11 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
   pp.dim = dimension;
   long long launches = 0;
   Launch L{(cudaStream_t)stream, &launches};
-  // every scratch word that is read is first written by these launches: the
-  // range words by k_range_init, the histogram by k_radix_hist per pass
-  if(launch_range_keys(L, P, pp, range, (unsigned long long *)keys_out,
-       perm_out) != cudaSuccess)
+  // every scratch word that is read is first written by these launches (the
+  // range's partial words share the keys' scratch), but the range's block
+  // counter: zero at load, and left zero by every call
+  if(launch_range(L, P, pp, range, ktmp) != cudaSuccess ||
+     launch_keys(L, P, pp, range, (unsigned long long *)keys_out, perm_out) != cudaSuccess)
     return FSPH_ERR_CUDA;
   if(radix_sort_pairs(L, (unsigned long long *)keys_out, perm_out, ktmp, vtmp,
        (int)n, hist, 63 / dimension * dimension) != cudaSuccess)
