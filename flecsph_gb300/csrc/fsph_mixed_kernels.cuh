@@ -347,7 +347,7 @@ __device__ __forceinline__ double pair_mf(const Particles & P, const PhysParams 
     r2 += pos_ab[d] * pos_ab[d];
   }
   ph.template set<false, true>(h_a, P.f[F_H][b], pp);
-  return P.f[F_M][b] * pair_g<D, K>(pair_r(r2), ph, pp);
+  return P.f[F_M][b] * pair_g_free<D, K>(r2, ph, pp);
 }
 
 // The same for four lanes: lane d < D adds axis d of the chunk's four pairs,
