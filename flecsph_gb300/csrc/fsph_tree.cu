@@ -789,8 +789,8 @@ cudaError_t launch_permute(const Launch & L, const Particles & src,
 //
 // The thread that arrives first at split s leaves the far end of its child
 // and the D beyond it, the one that arrives second takes them.  A node whose
-// keys all lie in this block's 256 leaves (told from the two keys around
-// them) meets in shared memory, child data included; above that, a 64-bit
+// keys all lie in this block's leaves (told from the two keys around them)
+// meets in shared memory, child data included; above that, a 64-bit
 // device-scope exchange releases the first child's data, which the second
 // thread reads through L2, and leaves the slot empty for the next build.
 //
@@ -804,7 +804,17 @@ cudaError_t launch_permute(const Launch & L, const Particles & src,
 // FP32 copies combine among themselves, rounding being monotonic.
 //
 // Latency bounds it: about 150 ns a level in shared memory, 0.8 us above.
-#define TREE_THREADS 256
+// Leaves per block, measured (the tree phase, ms; 2k 2D and 2M 3D with one h,
+// 50k and 4M star with gravity):
+//   one h    256: 0.029, 0.196   512: 0.032, 0.202   1024: 0.034, 0.210
+//   ALL      128: 0.069, 1.73    256: 0.071, 1.88     512: 0.071, 2.16
+// A block waits for its longest climb; with the 368 bytes that a leaf's two
+// slots take in ALL, 128 leaves let four blocks share an SM instead of two.
+constexpr int TREE_UNI_THREADS = 256, TREE_ALL_THREADS = 128;
+template<bool ALL>
+__host__ __device__ constexpr int tree_threads() {
+  return ALL ? TREE_ALL_THREADS : TREE_UNI_THREADS;
+}
 #define TREE_EMPTY 0xffffffffffffffffull
 
 // smaller and larger of two finite doubles by their bits
@@ -829,15 +839,15 @@ struct TreeData<true> {
 
 template<bool ALL>
 __host__ __device__ constexpr size_t tree_smem() {
-  return 2 * TREE_THREADS * (ALL ? 32 + 48 + 24 + 80 : 32);
+  return 2 * tree_threads<ALL>() * (ALL ? 32 + 48 + 24 + 80 : 32);
 }
 
-// (1: shared-memory deposit of a child, slot q of 2 * TREE_THREADS, as
+// (1: shared-memory deposit of a child, slot q of two per thread, as
 // structure of arrays)
 template<bool ALL, bool STORE>
 __device__ __forceinline__ void tree_slot(unsigned char * sm, int q, TreeData<ALL> & d,
   bool boxes, bool mom) {
-  constexpr int N = 2 * TREE_THREADS;
+  constexpr int N = 2 * tree_threads<ALL>();
   int4 * s4 = (int4 *)sm;
   if(STORE) {
     s4[q] = d.lo;
@@ -991,12 +1001,13 @@ __device__ __forceinline__ void tree_merge(TreeData<ALL> & d, const TreeData<ALL
 // with one full key would make the reference's build_tree loop run past depth
 // 0 (tree_topology.h:957-971): reported.
 template<int dim, bool ALL>
-__global__ void __launch_bounds__(TREE_THREADS) k_tree(const unsigned long long * K,
+__global__ void __launch_bounds__(tree_threads<ALL>()) k_tree(const unsigned long long * K,
   Particles P, Tree T, const int4 * qpos, const unsigned long long * rbits, int ordered,
   int gmax, DevStatus * st) {
   const bool boxes = ordered || rbits[6] != rbits[7], mom = T.gmom != nullptr;
   if(ALL != (boxes || mom))
     return;
+  constexpr int TREE_THREADS = tree_threads<ALL>();
   extern __shared__ __align__(16) unsigned char tsm[];
   __shared__ unsigned long long skey[TREE_THREADS + 2];  // keys b0 - 1 .. b1 + 1
   __shared__ unsigned sx[TREE_THREADS];  // far end - b0 | (D + 1) << 16
@@ -1248,9 +1259,9 @@ cudaError_t launch_build_tree(const Launch & L, const Particles & P,
   if(ae != cudaSuccess)
     return ae;
   const int n = P.n;
-  const int nb = (n + TREE_THREADS - 1) / TREE_THREADS;
 #define TREE_LAUNCH(DIM, ALL)                                                \
-  k_tree<DIM, ALL><<<nb, TREE_THREADS, tree_smem<ALL>(), L.stream>>>(P.key, P, T, qpos, \
+  k_tree<DIM, ALL><<<(n + tree_threads<ALL>() - 1) / tree_threads<ALL>(),      \
+    tree_threads<ALL>(), tree_smem<ALL>(), L.stream>>>(P.key, P, T, qpos, \
     rbits, ordered, group_max, st)
   // in the ordered mode and with gravity every run is ALL; else the range
   // words on the device tell
