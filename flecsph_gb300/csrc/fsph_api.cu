@@ -880,12 +880,14 @@ static fsph_status update_iteration(fsph_ctx * c, bool range_known) {
       // fsph_step_io: input fields copied on the copy stream land first
       CK(cudaStreamWaitEvent(c->stream, c->io.ev[0], 0));
       c->io.h2d_pending = false;
+      L.chained = false;
     }
     // the mixed float-float path's {v, c_s} records come out of the permute
     float4 * vel = c->mixed && wendland(c->pp.kernel) ? c->K.vel : nullptr;
     CK(launch_permute(L, c->P, c->Palt, c->svals, c->skeys, c->permute_skip, c->d_range,
       c->K, c->T.ngroups, c->Ls.stat, vel, c->pp.dim));
     c->vel_ok = vel != nullptr;
+    L = c->L();
     Particles t = c->P;
     c->P = c->Palt;
     c->Palt = t;

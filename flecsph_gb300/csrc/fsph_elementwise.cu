@@ -29,6 +29,7 @@ __device__ __forceinline__ double recover_u(const Particles & P,
 template<int D>
 __global__ void __launch_bounds__(ELEM_THREADS) k_elem(Particles P,
   PhysParams pp, int op, const DevTime * tm, DevStatus * st) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= P.n)
     return;
@@ -168,9 +169,9 @@ cudaError_t launch_elementwise(const Launch & L, const Particles & P,
   const PhysParams & pp, int op, DevTime * t, DevStatus * st) {
   const int nb = (P.n + ELEM_THREADS - 1) / ELEM_THREADS;
   if(pp.dim == 3)
-    k_elem<3><<<nb, ELEM_THREADS, 0, L.stream>>>(P, pp, op, t, st);
+    chain(L, k_elem<3>, nb, ELEM_THREADS, 0, P, pp, op, t, st);
   else
-    k_elem<2><<<nb, ELEM_THREADS, 0, L.stream>>>(P, pp, op, t, st);
+    chain(L, k_elem<2>, nb, ELEM_THREADS, 0, P, pp, op, t, st);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -181,6 +182,7 @@ cudaError_t launch_elementwise(const Launch & L, const Particles & P,
 template<int D, int OP, bool RANGE>
 __global__ void __launch_bounds__(ELEM_THREADS) k_kick_drift(Particles P,
   const DevTime * tm, unsigned long long * range, unsigned long long * part) {
+  chain_begin();
   double ** f = P.f;
   const double dt = tm->dt, s = 0.5 * dt;
   RangeAcc<D> r;
@@ -227,9 +229,9 @@ cudaError_t launch_kick_drift(const Launch & L, const Particles & P, const PhysP
 #define KD_LAUNCH(D, OP)                                                       \
   do {                                                                         \
     if(range)                                                                  \
-      k_kick_drift<D, OP, true><<<nb, ELEM_THREADS, 0, L.stream>>>(P, t, range, range_part); \
+      chain(L, k_kick_drift<D, OP, true>, nb, ELEM_THREADS, 0, P, t, range, range_part); \
     else                                                                       \
-      k_kick_drift<D, OP, false><<<nb, ELEM_THREADS, 0, L.stream>>>(P, t, nullptr, nullptr); \
+      chain(L, k_kick_drift<D, OP, false>, nb, ELEM_THREADS, 0, P, t, nullptr, nullptr); \
   } while(0)
 #define KD_OP(D)                                                               \
   do {                                                                         \
@@ -367,6 +369,7 @@ __device__ __noinline__ double limit_dt(const PhysParams & pp, double * const * 
 template<int D, bool CHECKS, bool F32, bool FINISH>
 __global__ void __launch_bounds__(ELEM_THREADS) k_compute_dt(Particles P,
   PhysParams pp, DtConst c32, DevTime * tm, DevStatus * st) {
+  chain_begin();
   // grid-stride: one atomic per block of a grid sized to the machine
   unsigned long long dtmin = TIME_DT_MAX;  // ordered encoding
   for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n;
@@ -478,7 +481,7 @@ cudaError_t launch_compute_dt(const Launch & L, const Particles & P,
   const DtConst c32 = {(float)(pp.eta * pp.kw), (float)pp.cfl,
     1.f + 0.6f * (float)pp.alpha};
 #define DT_LAUNCH(D, C, F, E) \
-  k_compute_dt<D, C, F, E><<<nb, ELEM_THREADS, 0, L.stream>>>(P, pp, c32, t, st)
+  chain(L, k_compute_dt<D, C, F, E>, nb, ELEM_THREADS, 0, P, pp, c32, t, st)
 #define DT_PICK(D)                                                             \
   do {                                                                         \
     if(with_checks && finish) {                                                \
@@ -501,20 +504,26 @@ cudaError_t launch_compute_dt(const Launch & L, const Particles & P,
   return cudaGetLastError();
 }
 
-__global__ void k_set_adaptive(PhysParams pp, DevTime * t) { set_adaptive(pp, t); }
+__global__ void k_set_adaptive(PhysParams pp, DevTime * t) {
+  chain_begin();
+  set_adaptive(pp, t);
+}
 
 cudaError_t launch_set_adaptive_timestep(const Launch & L,
   const PhysParams & pp, DevTime * t) {
-  k_set_adaptive<<<1, 1, 0, L.stream>>>(pp, t);
+  chain(L, k_set_adaptive, 1, 1, 0, pp, t);
   *L.counter += 1;
   return cudaGetLastError();
 }
 
-__global__ void k_advance(PhysParams pp, DevTime * t) { advance(pp, t); }
+__global__ void k_advance(PhysParams pp, DevTime * t) {
+  chain_begin();
+  advance(pp, t);
+}
 
 cudaError_t launch_advance_time(const Launch & L, const PhysParams & pp,
   DevTime * t) {
-  k_advance<<<1, 1, 0, L.stream>>>(pp, t);
+  chain(L, k_advance, 1, 1, 0, pp, t);
   *L.counter += 1;
   return cudaGetLastError();
 }

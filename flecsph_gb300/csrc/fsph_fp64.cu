@@ -35,6 +35,7 @@ template<int D, int K, bool CULL>
 __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
   PhysParams pp, Lists Ls, double * cs_new, double * prho2, DevStatus * st,
   const DevTime * tm) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
 // P / rho^2 of every particle where the density pass's is out of date (a
 // caller changed P or rho in between).
 __global__ void __launch_bounds__(256) k_prho2(Particles P, double * prho2) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i < P.n) {
     const double rho = P.f[F_RHO][i];
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(256) k_prho2(Particles P, double * prho2) {
 template<int D, int K>
 __global__ void __launch_bounds__(PAIR_THREADS) k_alpha_cullen(Particles P,
   PhysParams pp, Lists Ls, const DevTime * tm) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -226,6 +229,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_alpha_cullen(Particles P,
 template<int D>
 __global__ void __launch_bounds__(PAIR_THREADS) k_vsig(Particles P, Lists Ls,
   const double * cs_new) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -282,6 +286,7 @@ template<int D, int K, bool VSIG>
 __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   PhysParams pp, Lists Ls, int kick, const DevTime * tm, const double * prho2,
   const double * cs_old, double2 * pair) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -393,6 +398,7 @@ template<int D, int K, bool KEPT>
 __global__ void __launch_bounds__(PAIR_THREADS) k_dudt(Particles P,
   PhysParams pp, Lists Ls, const DevTime * tm, const double * prho2,
   const double2 * pair) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_dudt(Particles P,
 template<int D, int K, bool KEPT>
 __global__ void __launch_bounds__(PAIR_THREADS) k_dedt(Particles P,
   PhysParams pp, Lists Ls, const double * prho2, const double2 * pair) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -488,41 +495,41 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_dedt(Particles P,
     if(pp.dim == 3) {                                                          \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_GAUSSIAN TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<3, FSPH_KERNEL_SINC TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_SINC TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     else {                                                                     \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_GAUSSIAN TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<2, FSPH_KERNEL_SINC TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_SINC TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6 TA><<<nb_, PAIR_THREADS, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6 TA>, nb_, PAIR_THREADS, 0, __VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     *L.counter += 1;                                                           \
@@ -541,7 +548,7 @@ cudaError_t launch_density_fp64(const Launch & L, const Particles & P,
 }
 
 cudaError_t launch_prho2(const Launch & L, const Particles & P, double * prho2) {
-  k_prho2<<<(P.n + 255) / 256, 256, 0, L.stream>>>(P, prho2);
+  chain(L, k_prho2, (P.n + 255) / 256, 256, 0, P, prho2);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -609,9 +616,9 @@ cudaError_t launch_vsig_fp64(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const double * cs_new) {
   const int nb = (P.n + PAIR_THREADS - 1) / PAIR_THREADS;
   if(pp.dim == 3)
-    k_vsig<3><<<nb, PAIR_THREADS, 0, L.stream>>>(P, Ls, cs_new);
+    chain(L, k_vsig<3>, nb, PAIR_THREADS, 0, P, Ls, cs_new);
   else
-    k_vsig<2><<<nb, PAIR_THREADS, 0, L.stream>>>(P, Ls, cs_new);
+    chain(L, k_vsig<2>, nb, PAIR_THREADS, 0, P, Ls, cs_new);
   *L.counter += 1;
   return cudaGetLastError();
 }

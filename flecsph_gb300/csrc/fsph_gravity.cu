@@ -75,6 +75,7 @@ __device__ __forceinline__ void split_hi_lo(double v, float & hi, float & lo) {
 // Every particle also gets its FP32 walk record here.
 __global__ void k_grav_nodes(Particles P, int dim, Tree T, GravBuffers G,
   const unsigned long long * rbits, int order) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = P.n;
   if(i >= n)
@@ -190,6 +191,7 @@ template<bool MIXED>
 __global__ void __launch_bounds__(GW_WARPS * 32) k_gravity_walk(Particles P,
   Tree T, GravBuffers G, float theta, double Gc, int order, int dim,
   DevStatus * st) {
+  chain_begin();
   typedef typename std::conditional<MIXED, float, double>::type R;
   extern __shared__ __align__(16) unsigned char gsm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -668,7 +670,7 @@ cudaError_t launch_gravity(const Launch & L, const Particles & P,
   const int n = P.n;
   if(n < 2)  // a lone particle feels no force
     return cudaSuccess;
-  k_grav_nodes<<<(n + 255) / 256, 256, 0, L.stream>>>(P, pp.dim, T, G, rbits, order);
+  chain(L, k_grav_nodes, (n + 255) / 256, 256, 0, P, pp.dim, T, G, rbits, order);
   const size_t smem = (mixed ? gw_warp_bytes<true>() : gw_warp_bytes<false>()) * GW_WARPS;
   static std::atomic<unsigned long long> attr_devices{0};
   cudaError_t ae = once_per_device(&attr_devices, [&]() {
@@ -687,10 +689,10 @@ cudaError_t launch_gravity(const Launch & L, const Particles & P,
   if(blocks > maxb)
     blocks = maxb > 0 ? maxb : 1;
   if(mixed)
-    k_gravity_walk<true><<<blocks, GW_WARPS * 32, smem, L.stream>>>(P, T, G,
+    chain(L, k_gravity_walk<true>, blocks, GW_WARPS * 32, smem, P, T, G,
       (float)theta, pp.G, order, pp.dim, st);
   else
-    k_gravity_walk<false><<<blocks, GW_WARPS * 32, smem, L.stream>>>(P, T, G,
+    chain(L, k_gravity_walk<false>, blocks, GW_WARPS * 32, smem, P, T, G,
       (float)theta, pp.G, order, pp.dim, st);
   *L.counter += 2;
   return cudaGetLastError();

@@ -238,7 +238,42 @@ __host__ __device__ inline int slot_off(int j) { return ((j & ~3) << 5) | (j & 3
 struct Launch {
   cudaStream_t stream;
   long long * counter;  // launches issued
+  bool chained = false; // may chain() overlap this launch with the one before
 };
+
+// The kernels of one iteration follow each other on one stream.  With chain()
+// a kernel's launch and the set-up of its blocks overlap the end of the kernel
+// before, whose blocks leave the SMs one by one; the new blocks wait in
+// chain_begin() until all of that kernel has finished and its writes can be
+// seen.  chain_begin() is the first statement of every kernel launched so,
+// ahead of any access to memory and of any return: a kernel that ended before
+// its predecessor would let its successor start too early.  Work that is not a
+// chained kernel (copies, events, the other kernels) is ordered as ever.
+// Ten iterations, plain launches -> chained: 2k particles in 2D 2.83 -> 2.26 ms,
+// 32k in 3D by single calls 2.33 -> 2.04, 50k star 2.75 -> 2.67, 133k 3.66 -> 3.52,
+// 8k in FP64 2.38 -> 2.26, 2M 26.6 -> 26.2.  No block calls
+// griddepcontrol.launch_dependents: the successor's blocks would be dealt out
+// while the predecessor's still hold SMs, unevenly (91k in FP64: 15.4 ms
+// against 13.4; 50k star 2.79 against 2.67).
+template<class... P, class... A>
+inline cudaError_t chain(const Launch & L, void (*kernel)(P...), unsigned grid,
+  unsigned block, size_t smem, A &&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = L.stream;
+  cfg.attrs = at;
+  cfg.numAttrs = L.chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Kernel attributes (cudaFuncSetAttribute) belong to a device.  Runs
 // `apply` (returning a cudaError_t) once for the current device, bit d of

@@ -29,6 +29,7 @@ enum { PACK_VHM = 1, PACK_VEL = 2, PACK_THERMO = 4, PACK_AV_IN = 8, PACK_AV = 16
 // pass sees the current v_half, v, rho, P and c_s whatever the caller did
 // in between (separate kicks, repeated pressure updates).
 __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= P.n)
     return;
@@ -99,6 +100,7 @@ __global__ void k_pack_state(Particles P, int dim, Packed K, int what) {
 template<int D, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS) k_vsig_mixed(Particles P, Lists Ls,
   Packed Kp) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   const int a = pass_particle<MIX_THREADS>(split);
   if(a >= P.n)
@@ -163,7 +165,7 @@ cudaError_t launch_density_mixed(const Launch & L, const Particles & P,
   const int what = wendland_kernel(pp.kernel) ? (vel_current ? 0 : PACK_VEL)
                                               : PACK_VHM | PACK_VEL;
   if(what) {
-    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    chain(L, k_pack_state, (P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, P, pp.dim, K, what);
     *L.counter += 1;
   }
   PAIR_PASS(run_density, L, P, pp, Ls, K, cs_new, st, tm);
@@ -174,7 +176,7 @@ cudaError_t launch_alpha_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t) {
   // current velocities and masses; sound speeds and div v signs of the
   // neighbours
-  k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K,
+  chain(L, k_pack_state, (P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, P, pp.dim, K,
     PACK_VHM | PACK_VEL_V | PACK_AV_IN);
   *L.counter += 1;
   run_alpha_mixed(L, P, pp, Ls, K, t);
@@ -187,14 +189,14 @@ cudaError_t launch_vsig_mixed(const Launch & L, const Particles & P,
   const int ns = (P.n + MIX_THREADS / 4 - 1) / (MIX_THREADS / 4);
   if(P.n <= SPLIT_MAX) {
     if(pp.dim == 3)
-      k_vsig_mixed<3, true><<<ns, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+      chain(L, k_vsig_mixed<3, true>, ns, MIX_THREADS, 0, P, Ls, K);
     else
-      k_vsig_mixed<2, true><<<ns, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+      chain(L, k_vsig_mixed<2, true>, ns, MIX_THREADS, 0, P, Ls, K);
   }
   else if(pp.dim == 3)
-    k_vsig_mixed<3, false><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+    chain(L, k_vsig_mixed<3, false>, nb, MIX_THREADS, 0, P, Ls, K);
   else
-    k_vsig_mixed<2, false><<<nb, MIX_THREADS, 0, L.stream>>>(P, Ls, K);
+    chain(L, k_vsig_mixed<2, false>, nb, MIX_THREADS, 0, P, Ls, K);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -209,7 +211,7 @@ cudaError_t launch_accel_mixed(const Launch & L, const Particles & P,
   const int vh = wendland_kernel(pp.kernel) ? (fv_current ? 0 : PACK_FV) : PACK_VHM;
   const int what = (fused_vsig ? vh : (vh | PACK_THERMO)) | av;
   if(what) {
-    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    chain(L, k_pack_state, (P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, P, pp.dim, K, what);
     *L.counter += 1;
   }
   PAIR_PASS(run_accel, L, P, pp, Ls, K, kick, t, fused_vsig);
@@ -222,7 +224,7 @@ cudaError_t launch_dudt_mixed(const Launch & L, const Particles & P,
   const int what = (fv_current ? 0 : PACK_FV) | (fdv_current ? 0 : PACK_FDV) |
                    (pp.cullen ? PACK_AV : 0);
   if(what) {
-    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    chain(L, k_pack_state, (P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, P, pp.dim, K, what);
     *L.counter += 1;
   }
   PAIR_PASS(run_dudt, L, P, pp, Ls, K, t, then_op);
@@ -239,7 +241,7 @@ cudaError_t launch_dedt_mixed(const Launch & L, const Particles & P,
                       ? (fdv_current ? 0 : PACK_FDV) : PACK_VHM | PACK_DEDT) |
                    (pp.cullen ? PACK_AV : 0);
   if(what) {
-    k_pack_state<<<(P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, L.stream>>>(P, pp.dim, K, what);
+    chain(L, k_pack_state, (P.n + PACK_THREADS - 1) / PACK_THREADS, PACK_THREADS, 0, P, pp.dim, K, what);
     *L.counter += 1;
   }
   PAIR_PASS(run_dedt, L, P, pp, Ls, K, then_op, t, st, use_ahyd);

@@ -19,6 +19,7 @@ namespace fsph {
 template<int D, int K>
 __global__ void __launch_bounds__(MIX_THREADS) k_alpha_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, const DevTime * tm) {
+  chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
     return;
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(MIX_THREADS) k_alpha_mixed(Particles P,
 }
 
 #define ALPHA_LAUNCH(DD, KK) \
-  k_alpha_mixed<DD, KK><<<nb, MIX_THREADS, 0, L.stream>>>(P, pp, Ls, K, t)
+  chain(L, k_alpha_mixed<DD, KK>, nb, MIX_THREADS, 0, P, pp, Ls, K, t)
 
 void run_alpha_mixed(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const Packed & K, const DevTime * t) {

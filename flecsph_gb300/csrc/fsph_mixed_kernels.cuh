@@ -374,6 +374,7 @@ template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
   const DevTime * tm) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<MIX_THREADS>(split);
   if(!split && a >= P.n)
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(MIX_THREADS) k_density_mixed(
 template<int D, int K, bool VSIG, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_accel_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<MIX_THREADS>(split);
   if(!split && a >= P.n)
@@ -640,6 +642,7 @@ __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_acc
 template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dudt_mixed(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, const DevTime * tm, int then_op) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<ENERGY_THREADS>(split);
   if(!split && a >= P.n)
@@ -740,6 +743,7 @@ template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(4, ENERGY_THREADS)) k_dedt_mixed(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<ENERGY_THREADS>(split);
   if(!split && a >= P.n)
@@ -1070,6 +1074,7 @@ template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(3, MIX_THREADS)) k_density_ff(Particles P,
   PhysParams pp, Lists Ls, Packed Kp, double * cs_new, DevStatus * st,
   const DevTime * tm) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<MIX_THREADS>(split);
   if(!split && a >= P.n)
@@ -1401,6 +1406,7 @@ __device__ __forceinline__ void accel_ff_quad(const Packed & Kp, const int * lp,
 template<int D, int K, bool VSIG, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(MIX_THREADS, MIX_BLOCKS(FSPH_ACCEL_FF_BLOCKS, MIX_THREADS)) k_accel_ff(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, int kick, const DevTime * tm) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<MIX_THREADS>(split);
   if(!split && a >= P.n)
@@ -1516,6 +1522,7 @@ template<int D, int K, bool CULL, bool AUTO>
 __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS, ENERGY_THREADS)) k_dedt_ahyd(
   Particles P, PhysParams pp, Lists Ls, Packed Kp, int then_op, const DevTime * tm,
   DevStatus * st) {
+  chain_begin();
   const bool split = four_lanes<AUTO>(Ls);
   int a = pass_particle<ENERGY_THREADS>(split);
   if(!split && a >= P.n)
@@ -1622,41 +1629,41 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
     if(pp.dim == 3) {                                                          \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_GAUSSIAN, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<3, FSPH_KERNEL_SINC, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_SINC, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     else {                                                                     \
       switch(pp.kernel) {                                                      \
         case FSPH_KERNEL_CUBIC_SPLINE:                                         \
-          KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_CUBIC_SPLINE, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_QUINTIC_SPLINE:                                       \
-          KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_QUINTIC_SPLINE, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_GAUSSIAN:                                             \
-          KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_GAUSSIAN, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SUPER_GAUSSIAN:                                       \
-          KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_SUPER_GAUSSIAN, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_SINC:                                                 \
-          KERNEL_T<2, FSPH_KERNEL_SINC, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_SINC, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C2:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         case FSPH_KERNEL_WENDLAND_C4:                                          \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
         default:                                                               \
-          KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); break; \
+          chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); break; \
       }                                                                        \
     }                                                                          \
     *L.counter += 1;                                                           \
@@ -1673,19 +1680,19 @@ __global__ void __launch_bounds__(ENERGY_THREADS, MIX_BLOCKS(FSPH_ENERGY_BLOCKS,
     const int nb_ = (P.n + per_ - 1) / per_;                                   \
     if(pp.dim == 3) {                                                          \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C2, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C4, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<3, FSPH_KERNEL_WENDLAND_C6, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
     }                                                                          \
     else {                                                                     \
       if(pp.kernel == FSPH_KERNEL_WENDLAND_C2)                                 \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C2, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
       else if(pp.kernel == FSPH_KERNEL_WENDLAND_C4)                            \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C4, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
       else                                                                     \
-        KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO><<<nb_, nt_, 0, L.stream>>>(__VA_ARGS__); \
+        chain(L, KERNEL_T<2, FSPH_KERNEL_WENDLAND_C6, TA, AUTO>, nb_, nt_, 0, __VA_ARGS__); \
     }                                                                          \
     *L.counter += 1;                                                           \
   } while(0)
@@ -1772,7 +1779,7 @@ inline void run_accel_pass(const Launch & L, const Particles & P,
     }
   }
 #undef PICK
-  fn<<<(P.n + per - 1) / per, threads, 0, L.stream>>>(P, pp, Ls, K, kick, t);
+  chain(L, fn, (P.n + per - 1) / per, threads, 0, P, pp, Ls, K, kick, t);
   *L.counter += 1;
 }
 

@@ -30,6 +30,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 template<int dim>
 __global__ void __launch_bounds__(256) k_range(Particles P, unsigned long long * range,
   unsigned long long * part) {
+  chain_begin();
   const double * H = P.f[F_H];
   RangeAcc<dim> r;
   r.init(H[0]);
@@ -78,6 +79,7 @@ __device__ __forceinline__ unsigned long long spread2(unsigned long long x) {
 template<int dim>
 __global__ void __launch_bounds__(256) k_keys(Particles P, const unsigned long long * bits,
   unsigned long long * keys, int * idx) {
+  chain_begin();
   // the range and its scaled reciprocal, once per block
   __shared__ double s_mn[3], s_scale[3], s_rs[3];
   constexpr int md = 63 / dim;
@@ -123,9 +125,9 @@ cudaError_t launch_range(const Launch & L, const Particles & P, const PhysParams
   if(nb > RANGE_BLOCKS)
     nb = RANGE_BLOCKS;
   if(pp.dim == 3)
-    k_range<3><<<nb, 256, 0, L.stream>>>(P, range, range_part);
+    chain(L, k_range<3>, nb, 256, 0, P, range, range_part);
   else
-    k_range<2><<<nb, 256, 0, L.stream>>>(P, range, range_part);
+    chain(L, k_range<2>, nb, 256, 0, P, range, range_part);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -134,9 +136,9 @@ cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams 
   const unsigned long long * range, unsigned long long * keys_out, int * idx_out) {
   const int nb = (P.n + 255) / 256;
   if(pp.dim == 3)
-    k_keys<3><<<nb, 256, 0, L.stream>>>(P, range, keys_out, idx_out);
+    chain(L, k_keys<3>, nb, 256, 0, P, range, keys_out, idx_out);
   else
-    k_keys<2><<<nb, 256, 0, L.stream>>>(P, range, keys_out, idx_out);
+    chain(L, k_keys<2>, nb, 256, 0, P, range, keys_out, idx_out);
   *L.counter += 1;
   return cudaGetLastError();
 }
@@ -163,6 +165,7 @@ size_t radix_hist_entries(int n) {
 
 __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
   const unsigned long long * keys, int n, int shift, unsigned * hist) {
+  chain_begin();
   __shared__ unsigned sh[256];
   sh[threadIdx.x] = 0;
   __syncthreads();
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
 // block per digit) and the row total in tot[digit].
 __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
   unsigned * tot) {
+  chain_begin();
   __shared__ unsigned wsum[32];
   const int d = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
   unsigned * row = hist + (size_t)d * nb;
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
 __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter(
   const unsigned long long * kin, const int * vin, unsigned long long * kout,
   int * vout, int n, int shift, const unsigned * offs) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char rs_dyn[];
   unsigned long long * skey = (unsigned long long *)rs_dyn;
   int * sval = (int *)(rs_dyn + (size_t)RS_TILE * 8);
@@ -361,6 +366,7 @@ __host__ __device__ constexpr size_t sc_smem(int per) {
 __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
   unsigned long long * keys, int * vals, unsigned long long * keys_tmp, int * vals_tmp,
   int n, int per, int bits, int prefix_bits) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char sc_dyn[];
   unsigned long long * okey = (unsigned long long *)sc_dyn;
   int * oval = (int *)(okey + per + SC_RUN + 4);
@@ -628,15 +634,17 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
       ++lg;
     const int pb = (lg + 5 + 7) / 8 * 8;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim = {(unsigned)c, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(c);
     cfg.blockDim = dim3(SC_THREADS);
     cfg.dynamicSmemBytes = sc_smem(per);
     cfg.stream = L.stream;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = L.chained ? 2 : 1;
     *L.counter += 1;
     return cudaLaunchKernelEx(&cfg, k_sort_cluster, keys, vals, keys_tmp, vals_tmp, n, per,
       bits, pb);
@@ -652,9 +660,9 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   unsigned long long *ka = keys, *kb = keys_tmp;
   int *va = vals, *vb = vals_tmp;
   for(int shift = 0; shift < 64; shift += 8) {
-    k_radix_hist<<<nb, RS_THREADS, 0, L.stream>>>(ka, n, shift, hist);
-    k_scan_rows<<<256, 1024, 0, L.stream>>>(hist, nb, hist + (size_t)256 * nb);
-    k_radix_scatter<<<nb, RS_THREADS, RS_DYN_SMEM, L.stream>>>(ka, va, kb, vb, n,
+    chain(L, k_radix_hist, nb, RS_THREADS, 0, ka, n, shift, hist);
+    chain(L, k_scan_rows, 256, 1024, 0, hist, nb, hist + (size_t)256 * nb);
+    chain(L, k_radix_scatter, nb, RS_THREADS, RS_DYN_SMEM, ka, va, kb, vb, n,
       shift, hist);
     *L.counter += 3;
     unsigned long long * tk = ka;
@@ -689,6 +697,7 @@ __global__ void __launch_bounds__(256) k_permute(Particles src, Particles dst,
   const int * perm, const unsigned long long * keys, unsigned skip,
   const unsigned long long * rbits, Packed K, int * ngroups, unsigned * list_stat,
   float4 * vel) {
+  chain_begin();
   __shared__ double s_lo[3], s_sc, s_iE;
   if(dim > 0 && threadIdx.x < dim)
     s_lo[threadIdx.x] = ord_dec(rbits[threadIdx.x]);
@@ -750,7 +759,7 @@ __global__ void __launch_bounds__(256) k_permute(Particles src, Particles dst,
 
 cudaError_t launch_gather(const Launch & L, const Particles & src, const Particles & dst,
   const int * perm, const unsigned long long * keys, unsigned skip) {
-  k_permute<0><<<(src.n + 255) / 256, 256, 0, L.stream>>>(src, dst, perm, keys, skip,
+  chain(L, k_permute<0>, (src.n + 255) / 256, 256, 0, src, dst, perm, keys, skip,
     nullptr, Packed{}, nullptr, nullptr, nullptr);
   *L.counter += 1;
   return cudaGetLastError();
@@ -762,10 +771,10 @@ cudaError_t launch_permute(const Launch & L, const Particles & src,
   unsigned * list_stat, float4 * vel, int dim) {
   const int nb = (src.n + 255) / 256;
   if(dim == 3)
-    k_permute<3><<<nb, 256, 0, L.stream>>>(src, dst, perm, keys, skip, rbits, K, ngroups,
+    chain(L, k_permute<3>, nb, 256, 0, src, dst, perm, keys, skip, rbits, K, ngroups,
       list_stat, vel);
   else
-    k_permute<2><<<nb, 256, 0, L.stream>>>(src, dst, perm, keys, skip, rbits, K, ngroups,
+    chain(L, k_permute<2>, nb, 256, 0, src, dst, perm, keys, skip, rbits, K, ngroups,
       list_stat, vel);
   *L.counter += 1;
   return cudaGetLastError();
@@ -1004,6 +1013,7 @@ template<int dim, bool ALL>
 __global__ void __launch_bounds__(tree_threads<ALL>()) k_tree(const unsigned long long * K,
   Particles P, Tree T, const int4 * qpos, const unsigned long long * rbits, int ordered,
   int gmax, DevStatus * st) {
+  chain_begin();
   const bool boxes = ordered || rbits[6] != rbits[7], mom = T.gmom != nullptr;
   if(ALL != (boxes || mom))
     return;
@@ -1170,6 +1180,7 @@ __device__ __forceinline__ int node_level(const unsigned long long * K,
 // (tree_topology.h:220-235, sub_entities_ = 128 at :2121).
 __global__ void k_refgroups(const unsigned long long * K, int n, int dim,
   Tree T, const unsigned long long * rbits, int refboxes) {
+  chain_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   // read only when h varies, or for ties in the ordered mode
   if(i >= n || (!refboxes && rbits[6] == rbits[7]))
@@ -1233,6 +1244,7 @@ __device__ __forceinline__ int walk_start(const Tree & T, int g, const int4 & gl
 #define WALK_START_LAUNCH (1 << 18)
 __global__ void __launch_bounds__(256) k_walk_start(Tree T, int dim, const float * qscale,
   const unsigned long long * rbits) {
+  chain_begin();
   const int ng = *T.ngroups;
   const float hmax = (float)ord_dec(rbits[7]);
   const float qs0 = qscale[0], qs1 = qscale[1], qs2 = dim == 3 ? qscale[2] : 0.f;
@@ -1260,8 +1272,8 @@ cudaError_t launch_build_tree(const Launch & L, const Particles & P,
     return ae;
   const int n = P.n;
 #define TREE_LAUNCH(DIM, ALL)                                                \
-  k_tree<DIM, ALL><<<(n + tree_threads<ALL>() - 1) / tree_threads<ALL>(),      \
-    tree_threads<ALL>(), tree_smem<ALL>(), L.stream>>>(P.key, P, T, qpos, \
+  chain(L, k_tree<DIM, ALL>, (n + tree_threads<ALL>() - 1) / tree_threads<ALL>(),      \
+    tree_threads<ALL>(), tree_smem<ALL>(), P.key, P, T, qpos, \
     rbits, ordered, group_max, st)
   // in the ordered mode and with gravity every run is ALL; else the range
   // words on the device tell
@@ -1277,12 +1289,12 @@ cudaError_t launch_build_tree(const Launch & L, const Particles & P,
     TREE_LAUNCH(2, true);
   }
 #undef TREE_LAUNCH
-  k_refgroups<<<(n + 255) / 256, 256, 0, L.stream>>>(P.key, n, pp.dim, T, rbits,
+  chain(L, k_refgroups, (n + 255) / 256, 256, 0, P.key, n, pp.dim, T, rbits,
     ordered);
   *L.counter += full_only ? 2 : 3;
   if(!ordered && n >= WALK_START_LAUNCH) {
     const int most = (n + 255) / 256;
-    k_walk_start<<<most < 152 * 8 ? most : 152 * 8, 256, 0, L.stream>>>(T, pp.dim, qscale,
+    chain(L, k_walk_start, most < 152 * 8 ? most : 152 * 8, 256, 0, T, pp.dim, qscale,
       rbits);
     *L.counter += 1;
   }
@@ -1532,6 +1544,7 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
   : MODE == NB_MODE_UNI ? NB_UNI_BLOCKS_PER_SM : NB_BLOCKS_PER_SM) k_neighbors(
   Particles P, Tree T, Lists Ls, DevStatus * st, int dim,
   const unsigned long long * rbits, Packed K) {
+  chain_begin();
   constexpr bool ORDERED = MODE == NB_MODE_ORDERED;
   constexpr bool UNI = MODE == NB_MODE_UNI;
   if(!ORDERED && UNI != (rbits[6] == rbits[7]))
@@ -2048,16 +2061,16 @@ cudaError_t launch_neighbors(const Launch & L, const Particles & P,
   const int maxb = maxb0 > 0 ? maxb0 : 1;
   auto grid = [&](int per_sm) { return nsm * per_sm < maxb ? nsm * per_sm : maxb; };
   if(ordered) {
-    k_neighbors<NB_MODE_ORDERED><<<grid(NB_ORDERED_BLOCKS_PER_SM), NB_WARPS * 32,
-      smem_o, L.stream>>>(P, T, Ls, st, pp.dim, rbits, K);
+    chain(L, k_neighbors<NB_MODE_ORDERED>, grid(NB_ORDERED_BLOCKS_PER_SM), NB_WARPS * 32,
+      smem_o, P, T, Ls, st, pp.dim, rbits, K);
     *L.counter += 1;
   }
   else {
     // both variants; the one the range words do not select returns at once
-    k_neighbors<NB_MODE_UNI><<<grid(NB_UNI_BLOCKS_PER_SM), NB_WARPS * 32, smem_u,
-      L.stream>>>(P, T, Ls, st, pp.dim, rbits, K);
-    k_neighbors<NB_MODE_VAR><<<grid(NB_BLOCKS_PER_SM), NB_WARPS * 32, smem_v,
-      L.stream>>>(P, T, Ls, st, pp.dim, rbits, K);
+    chain(L, k_neighbors<NB_MODE_UNI>, grid(NB_UNI_BLOCKS_PER_SM), NB_WARPS * 32, smem_u,
+      P, T, Ls, st, pp.dim, rbits, K);
+    chain(L, k_neighbors<NB_MODE_VAR>, grid(NB_BLOCKS_PER_SM), NB_WARPS * 32, smem_v,
+      P, T, Ls, st, pp.dim, rbits, K);
     *L.counter += 2;
   }
   return cudaGetLastError();
