@@ -1,5 +1,6 @@
 // fsph_api.cu -- the C ABI (include/fsph.h): context, data movement and the
 // body_system / physics call surface, sequenced on one CUDA stream.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cctype>
@@ -592,6 +593,36 @@ void fsph_destroy(fsph_ctx * c) {
   delete c;
 }
 
+// Whether a kernel on this device may touch [p, p + bytes): 8-byte aligned and
+// within one allocation of the device.  What is not (host memory, a peer's, a
+// range past its allocation) goes to the runtime's copies, which take it or
+// refuse it.
+static bool kernel_reaches(int device, const void * p, size_t bytes) {
+  typedef CUresult (*Get)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+  static const Get get = []() {
+    void * f = nullptr;
+    if(cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000,
+         cudaEnableDefault) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (Get)f;
+  }();
+  if(!get || ((size_t)p & 7))
+    return false;
+  unsigned type = 0;
+  int dev = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute at[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,
+    CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+    CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void * data[4] = {&type, &dev, &start, &size};
+  return get(4, at, data, (CUdeviceptr)p) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE &&
+         dev == device && (CUdeviceptr)p >= start && bytes <= size &&
+         (CUdeviceptr)p - start <= size - bytes;
+}
+
 // The view's arrays are host memory (kind cudaMemcpyHostToDevice) or device
 // memory of the context's device (cudaMemcpyDeviceToDevice).
 static fsph_status upload_impl(fsph_ctx * c, const fsph_soa_view * v,
@@ -628,18 +659,32 @@ static fsph_status upload_impl(fsph_ctx * c, const fsph_soa_view * v,
     v->vhy, v->vhz, v->ax, v->ay, v->az, v->gax, v->gay, v->gaz, v->gpot, v->m,
     v->h, v->rho, v->P, v->cs, v->u, v->e, v->dudt, v->dedt, v->K, v->alpha,
     v->vsig, v->dt, v->divv, v->ddivvdt, v->Ye};
-  for(int k = 0; k < NF; ++k) {
-    if(src[k])
-      CK(cudaMemcpyAsync(c->P.f[k], src[k], sizeof(double) * n, kind, c->stream));
-    else
-      CK(cudaMemsetAsync(c->P.f[k], 0, sizeof(double) * n, c->stream));
-  }
-  CK(cudaMemcpyAsync(c->P.id, v->id, sizeof(long long) * n, kind, c->stream));
-  CK(cudaMemsetAsync(c->P.key, 0, sizeof(unsigned long long) * n, c->stream));
+  const size_t bytes = sizeof(double) * (size_t)n;
   DevTime t;
   init_time(&c->p, &t);
-  CK(cudaMemcpyAsync(c->d_time, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemsetAsync(c->d_status, 0, sizeof(DevStatus), c->stream));
+  Moves m;
+  bool one = kind == cudaMemcpyDeviceToDevice && kernel_reaches(c->device, v->id, bytes);
+  for(int k = 0; k < NF && one; ++k) {
+    one = !src[k] || kernel_reaches(c->device, src[k], bytes);
+    m.add(c->P.f[k], src[k]);
+  }
+  if(one) {
+    m.add(c->P.id, v->id);
+    m.add(c->P.key, nullptr);
+    CK(launch_move(c->L(), m, n, nullptr, c->d_time, t, c->d_status));
+  }
+  else {
+    for(int k = 0; k < NF; ++k) {
+      if(src[k])
+        CK(cudaMemcpyAsync(c->P.f[k], src[k], bytes, kind, c->stream));
+      else
+        CK(cudaMemsetAsync(c->P.f[k], 0, bytes, c->stream));
+    }
+    CK(cudaMemcpyAsync(c->P.id, v->id, bytes, kind, c->stream));
+    CK(cudaMemsetAsync(c->P.key, 0, bytes, c->stream));
+    CK(cudaMemcpyAsync(c->d_time, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(c->d_status, 0, sizeof(DevStatus), c->stream));
+  }
   CK(cudaStreamSynchronize(c->stream));
   c->iteration = c->p.initial_iteration;
   c->tree_ok = false;
@@ -749,26 +794,40 @@ static fsph_status download_impl(fsph_ctx * c, fsph_soa_view * v,
   cudaMemcpyKind kind) {
   if(!c || !v || v->n != c->n || !c->uploaded)
     return FSPH_ERR_ARG;
-  fsph_status s = fsph_sync(c);
-  if(s)
-    return s;
   const int n = c->n;
   double * dst[NF] = {v->x, v->y, v->z, v->vx, v->vy, v->vz, v->vhx, v->vhy,
     v->vhz, v->ax, v->ay, v->az, v->gax, v->gay, v->gaz, v->gpot, v->m, v->h,
     v->rho, v->P, v->cs, v->u, v->e, v->dudt, v->dedt, v->K, v->alpha, v->vsig,
     v->dt, v->divv, v->ddivvdt, v->Ye};
+  const size_t bytes = sizeof(double) * (size_t)n;
+  Moves m;
   for(int k = 0; k < NF; ++k) {
     if(k == F_Z || k == F_VZ || k == F_VHZ || k == F_AZ || k == F_GAZ)
       if(c->p.dimension == 2)
         continue;
     if(dst[k])
-      CK(cudaMemcpyAsync(dst[k], c->P.f[k], sizeof(double) * n, kind, c->stream));
+      m.add(dst[k], c->P.f[k]);
   }
   if(v->id)
-    CK(cudaMemcpyAsync(v->id, c->P.id, sizeof(long long) * n, kind, c->stream));
+    m.add(v->id, c->P.id);
   if(v->key)
-    CK(cudaMemcpyAsync(v->key, c->P.key, sizeof(unsigned long long) * n, kind,
-      c->stream));
+    m.add(v->key, c->P.key);
+  bool one = kind == cudaMemcpyDeviceToDevice;
+  for(int k = 0; k < m.count && one; ++k)
+    one = kernel_reaches(c->device, m.dst[k], bytes);
+  if(one) {
+    // behind the work in flight, and without effect if that raised an error
+    fsph_status s = set_device(c);
+    if(s)
+      return s;
+    CK(launch_move(c->L(), m, n, c->d_status, nullptr, DevTime{}, nullptr));
+    return fsph_sync(c);
+  }
+  fsph_status s = fsph_sync(c);
+  if(s)
+    return s;
+  for(int k = 0; k < m.count; ++k)
+    CK(cudaMemcpyAsync(m.dst[k], m.src[k], bytes, kind, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return FSPH_OK;
 }

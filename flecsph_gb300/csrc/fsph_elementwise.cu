@@ -528,6 +528,74 @@ cudaError_t launch_advance_time(const Launch & L, const PhysParams & pp,
   return cudaGetLastError();
 }
 
+// The device-side upload and download: the arrays along y, 2048 words of one
+// per block.  Memory-bound for large n; for small n it stands in for a copy or
+// a clear per array (34 for an upload), each a command of 2 to 5 us.  Upload,
+// ten iterations and download, copies per array -> this: 2k particles 2.29 ->
+// 2.10 ms, 32k 2.04 -> 1.78, 50k 2.65 -> 2.40, 2M 26.20 -> 25.85, 17M with two
+// iterations 137.1 -> 136.3; 32 members' downloads and eight steps 15.5 -> 11.9.
+#define MOVE_THREADS 256
+#define MOVE_WORDS (MOVE_THREADS * 8)
+__global__ void __launch_bounds__(MOVE_THREADS) k_move(Moves m, int n,
+  const DevStatus * status, DevTime * time, DevTime t0, DevStatus * clear) {
+  chain_begin();
+  if(status && status->code)
+    return;
+  const int t = threadIdx.x;
+  if(time && blockIdx.x == 0 && blockIdx.y == 0 && t == 0) {
+    *time = t0;
+    *clear = DevStatus{};
+  }
+  typedef unsigned long long word;
+  const word * src = (const word *)m.src[blockIdx.y];
+  word * dst = (word *)m.dst[blockIdx.y];
+  const int i0 = blockIdx.x * MOVE_WORDS;
+  if((((size_t)src | (size_t)dst) & 15) == 0) {
+    ulonglong2 v[4];
+#pragma unroll
+    for(int k = 0; k < 4; ++k) {
+      const int i = i0 + 2 * (k * MOVE_THREADS + t);
+      v[k] = make_ulonglong2(0, 0);
+      if(src && i + 1 < n)
+        v[k] = *(const ulonglong2 *)(src + i);
+      else if(src && i < n)
+        v[k].x = src[i];
+    }
+#pragma unroll
+    for(int k = 0; k < 4; ++k) {
+      const int i = i0 + 2 * (k * MOVE_THREADS + t);
+      if(i + 1 < n)
+        *(ulonglong2 *)(dst + i) = v[k];
+      else if(i < n)
+        dst[i] = v[k].x;
+    }
+  }
+  else {
+    word v[8];
+#pragma unroll
+    for(int k = 0; k < 8; ++k) {
+      const int i = i0 + k * MOVE_THREADS + t;
+      v[k] = src && i < n ? src[i] : 0;
+    }
+#pragma unroll
+    for(int k = 0; k < 8; ++k) {
+      const int i = i0 + k * MOVE_THREADS + t;
+      if(i < n)
+        dst[i] = v[k];
+    }
+  }
+}
+
+cudaError_t launch_move(const Launch & L, const Moves & m, int n, const DevStatus * status,
+  DevTime * time, const DevTime & t0, DevStatus * clear) {
+  if(m.count == 0 || n <= 0)
+    return cudaSuccess;
+  chain(L, k_move, dim3((n - 1) / MOVE_WORDS + 1, m.count), MOVE_THREADS, 0, m, n, status,
+    time, t0, clear);
+  *L.counter += 1;
+  return cudaGetLastError();
+}
+
 // Deterministic sum of h (fixed two-level order) for the averaged h.
 __global__ void __launch_bounds__(1024) k_hsum(Particles P, DevTime * t) {
   __shared__ double part[1024];

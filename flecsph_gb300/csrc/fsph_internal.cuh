@@ -256,13 +256,13 @@ struct Launch {
 // while the predecessor's still hold SMs, unevenly (91k in FP64: 15.4 ms
 // against 13.4; 50k star 2.79 against 2.67).
 template<class... P, class... A>
-inline cudaError_t chain(const Launch & L, void (*kernel)(P...), unsigned grid,
+inline cudaError_t chain(const Launch & L, void (*kernel)(P...), dim3 grid,
   unsigned block, size_t smem, A &&... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = L.stream;
@@ -443,6 +443,21 @@ cudaError_t launch_set_adaptive_timestep(const Launch & L,
   const PhysParams & pp, DevTime * t);
 cudaError_t launch_advance_time(const Launch & L, const PhysParams & pp,
   DevTime * t);
+// Arrays of n 8-byte words to copy within the device (a null src: to clear).
+struct Moves {
+  const void * src[NF + 2];
+  void * dst[NF + 2];
+  int count = 0;
+  void add(void * d, const void * s) {
+    dst[count] = d;
+    src[count++] = s;
+  }
+};
+// All of them in one launch.  status: nothing is written if it holds an error
+// (null: not looked at).  time: set to t0, and clear emptied, on the way (null:
+// not).
+cudaError_t launch_move(const Launch & L, const Moves & m, int n, const DevStatus * status,
+  DevTime * time, const DevTime & t0, DevStatus * clear);
 cudaError_t launch_hsum(const Launch & L, const Particles & P, DevTime * t);
 #define CONS_BLOCKS 1024
 // out8: 8 * (1 + CONS_BLOCKS) doubles; the totals land in the first 8
