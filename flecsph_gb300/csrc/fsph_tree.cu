@@ -144,9 +144,19 @@ cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams 
 }
 
 // ---------------------------------------------------------- radix sort --
-// LSD radix sort of (key, value) pairs, 8-bit digits.  Tiles of 4096 keys:
+// LSD radix sort of (key, value) pairs, 8-bit digits.  Tiles of 4608 keys:
 // histogram per tile, one exclusive scan over [digit][tile], then a stable
 // scatter in which each tile ranks its keys with warp match/ballot.
+//
+// A pass reads and writes every pair through HBM, so the passes cover the top
+// data bits only: at least 32 prefixes per key, in whole pairs of digits (32
+// bits up to 2^27 keys: four passes for eight).  k_prefix_runs then puts the few
+// keys that share a prefix in order; a run of more than RS_RUN_MAX of them
+// (particles crowded into a small part of the range) marks the sort, and the
+// eight passes over all bits follow, which return at once without the mark.
+// Sort with the permute, all bits -> prefix (ms): 216k 0.140 -> 0.103, 552k 0.178
+// -> 0.150, 1M 0.278 -> 0.228, 2M 0.480 -> 0.327, 4M star 0.884 -> 0.664, 19.7M
+// 3.59 -> 2.67.
 #define RS_THREADS 256
 #ifndef RS_ITEMS
 #define RS_ITEMS 18
@@ -158,14 +168,21 @@ cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams 
 #define RS_SCATTER_BLOCKS 3
 #endif
 
+#define RS_RUN_MAX 24
+
 size_t radix_hist_entries(int n) {
   size_t nb = ((size_t)n + RS_TILE - 1) / RS_TILE;
   return 256 * nb + 256;  // [digit][tile] counts, then the 256 digit totals
 }
 
 __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
-  const unsigned long long * keys, int n, int shift, unsigned * hist) {
+  const unsigned long long * keys, int n, int shift, unsigned * hist,
+  const unsigned * gate, unsigned * clear) {
   chain_begin();
+  if(gate && *gate == 0u)
+    return;
+  if(clear && blockIdx.x == 0 && threadIdx.x == 0)
+    *clear = 0u;
   __shared__ unsigned sh[256];
   sh[threadIdx.x] = 0;
   __syncthreads();
@@ -189,8 +206,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
 // Per digit: exclusive scan of its row of tile counts (coalesced, one
 // block per digit) and the row total in tot[digit].
 __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
-  unsigned * tot) {
+  unsigned * tot, const unsigned * gate) {
   chain_begin();
+  if(gate && *gate == 0u)
+    return;
   __shared__ unsigned wsum[32];
   const int d = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
   unsigned * row = hist + (size_t)d * nb;
@@ -237,8 +256,10 @@ __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
 #define RS_DYN_SMEM ((size_t)RS_TILE * 12)
 __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter(
   const unsigned long long * kin, const int * vin, unsigned long long * kout,
-  int * vout, int n, int shift, const unsigned * offs) {
+  int * vout, int n, int shift, const unsigned * offs, const unsigned * gate) {
   chain_begin();
+  if(gate && *gate == 0u)
+    return;
   extern __shared__ __align__(16) unsigned char rs_dyn[];
   unsigned long long * skey = (unsigned long long *)rs_dyn;
   int * sval = (int *)(rs_dyn + (size_t)RS_TILE * 8);
@@ -327,6 +348,39 @@ __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter
   }
 }
 
+// The keys are in order of key >> low: the first thread of each run that shares
+// a prefix orders it in place, ties as they are (the others see the same
+// prefixes meanwhile).  One read of the keys where there are no runs.
+__global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, int * vals,
+  int n, int low, unsigned * mark) {
+  chain_begin();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if(i + 1 >= n)
+    return;
+  const unsigned long long p = keys[i] >> low;
+  if(keys[i + 1] >> low != p || (i > 0 && keys[i - 1] >> low == p))
+    return;
+  int len = 2;
+  while(i + len < n && keys[i + len] >> low == p)
+    if(++len > RS_RUN_MAX) {
+      *mark = 1u;
+      return;
+    }
+  for(int j = i + 1; j < i + len; ++j) {
+    const unsigned long long k = keys[j];
+    const int v = vals[j];
+    int m = j;
+    for(; m > i && keys[m - 1] > k; --m) {
+      keys[m] = keys[m - 1];
+      vals[m] = vals[m - 1];
+    }
+    if(m < j) {
+      keys[m] = k;
+      vals[m] = v;
+    }
+  }
+}
+
 // ---- one-cluster sort --------------------------------------------------
 // Up to SC_MAX keys one launch sorts everything: a cluster of up to 16 blocks,
 // each with an equal share of the places.  A digit pass ranks a block's keys as
@@ -335,8 +389,8 @@ __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter
 // first so that they leave in runs of consecutive addresses, go to their
 // places through L2 (stores to the owner's shared memory instead moved 6 bytes
 // a clock and SM, three times slower).  Two cluster barriers a pass; no launch
-// between passes.  The multi-launch path below spends 24 launches whose tiles
-// fill a few SMs at these sizes: range, keys and sort of 2,250 / 31,000 /
+// between passes.  Eight passes of three launches each, whose tiles
+// fill a few SMs at these sizes, lose to it: range, keys and sort of 2,250 / 31,000 /
 // 132,651 keys take 33 / 44 / 76 us this way, 160 / 175 / 189 that way (at
 // 139,264 keys 78 against 188; beyond it a block's registers are full).
 // Latency bounds it: a pass of 8,300 keys a block is 33,000 cycles, 8,000 of
@@ -625,7 +679,7 @@ static int sc_blocks(int n) {
 
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
-  unsigned * hist, int bits) {
+  unsigned * hist, int bits, unsigned * mark) {
   if(const int c = sc_blocks(n)) {
     const int per = ((n + c - 1) / c + 3) & ~3;
     // prefix bits: at least 32 prefixes per key, in whole digits
@@ -659,20 +713,31 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int nb = (n + RS_TILE - 1) / RS_TILE;
   unsigned long long *ka = keys, *kb = keys_tmp;
   int *va = vals, *vb = vals_tmp;
-  for(int shift = 0; shift < 64; shift += 8) {
-    chain(L, k_radix_hist, nb, RS_THREADS, 0, ka, n, shift, hist);
-    chain(L, k_scan_rows, 256, 1024, 0, hist, nb, hist + (size_t)256 * nb);
-    chain(L, k_radix_scatter, nb, RS_THREADS, RS_DYN_SMEM, ka, va, kb, vb, n,
-      shift, hist);
-    *L.counter += 3;
-    unsigned long long * tk = ka;
-    ka = kb;
-    kb = tk;
-    int * tv = va;
-    va = vb;
-    vb = tv;
-  }
-  // eight passes: the result is back in (keys, vals)
+  // an even number of passes: the result is back in (keys, vals)
+  auto passes = [&](int from, int to, const unsigned * gate, unsigned * clear) {
+    for(int shift = from; shift < to; shift += 8) {
+      chain(L, k_radix_hist, nb, RS_THREADS, 0, ka, n, shift, hist, gate, clear);
+      chain(L, k_scan_rows, 256, 1024, 0, hist, nb, hist + (size_t)256 * nb, gate);
+      chain(L, k_radix_scatter, nb, RS_THREADS, RS_DYN_SMEM, ka, va, kb, vb, n,
+        shift, hist, gate);
+      *L.counter += 3;
+      unsigned long long * tk = ka;
+      ka = kb;
+      kb = tk;
+      int * tv = va;
+      va = vb;
+      vb = tv;
+      clear = nullptr;
+    }
+  };
+  int lg = 0;
+  while((1ll << lg) < n)
+    ++lg;
+  const int low = bits - (lg + 5 + 15) / 16 * 16;
+  passes(low, bits, nullptr, mark);
+  chain(L, k_prefix_runs, (n + 255) / 256, 256, 0, keys, vals, n, low, mark);
+  *L.counter += 1;
+  passes(0, 64, mark, nullptr);
   return cudaGetLastError();
 }
 
@@ -2155,7 +2220,8 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
      launch_keys(L, P, pp, range, (unsigned long long *)keys_out, perm_out) != cudaSuccess)
     return FSPH_ERR_CUDA;
   if(radix_sort_pairs(L, (unsigned long long *)keys_out, perm_out, ktmp, vtmp,
-       (int)n, hist, 63 / dimension * dimension) != cudaSuccess)
+       (int)n, hist, 63 / dimension * dimension,
+       (unsigned *)(range + RANGE_MARK)) != cudaSuccess)
     return FSPH_ERR_CUDA;
   return FSPH_OK;
 }
