@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, 
 // first so that they leave in runs of consecutive addresses, go to their
 // places through L2 (stores to the owner's shared memory instead moved 6 bytes
 // a clock and SM, three times slower).  Two cluster barriers a pass; no launch
-// between passes.  Eight passes of three launches each, whose tiles
-// fill a few SMs at these sizes, lose to it: range, keys and sort of 2,250 / 31,000 /
+// between passes.  Eight passes of three launches each (below), whose tiles
+// fill a few SMs at these sizes, lost to it: range, keys and sort of 2,250 / 31,000 /
 // 132,651 keys take 33 / 44 / 76 us this way, 160 / 175 / 189 that way (at
 // 139,264 keys 78 against 188; beyond it a block's registers are full).
 // Latency bounds it: a pass of 8,300 keys a block is 33,000 cycles, 8,000 of
