@@ -1305,7 +1305,7 @@ __device__ __forceinline__ int walk_start(const Tree & T, int g, const int4 & gl
 // walk_start of every group by a launch of its own, where there are many: in
 // the walk its chain of dependent loads (two a level) holds a whole warp, 40 us
 // of the Sedov 128^3 walk more than this launch; at 2,250 to 132,651 particles
-// the launch costs the 7 to 12 us that it does not save.
+// the launch costs 3 to 9 us that it does not save.
 #define WALK_START_LAUNCH (1 << 18)
 __global__ void __launch_bounds__(256) k_walk_start(Tree T, int dim, const float * qscale,
   const unsigned long long * rbits) {
