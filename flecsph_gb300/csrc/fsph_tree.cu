@@ -388,7 +388,8 @@ __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, 
 // distributed shared memory, and the keys, put in digit order in shared memory
 // first so that they leave in runs of consecutive addresses, go to their
 // places through L2 (stores to the owner's shared memory instead moved 6 bytes
-// a clock and SM, three times slower).  Two cluster barriers a pass; no launch
+// a clock and SM, three times slower).  Two cluster barriers a pass (and one
+// that has to be passed before a block first stores to another); no launch
 // between passes.  Eight passes of three launches each (below), whose tiles
 // fill a few SMs at these sizes, lost to it: range, keys and sort of 2,250 / 31,000 /
 // 132,651 keys take 33 / 44 / 76 us this way, 160 / 175 / 189 that way (at
@@ -440,6 +441,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
   int *vin = vals, *vout = vals_tmp;
   if(t == 0)
     aux[16] = 0;
+  // A block's shared memory may be touched by the others once it has started:
+  // every block arrives here, and waits before the first pass's exchange of
+  // counts, which the loads and ballots before it leave time for.
+  cl.barrier_arrive();
+  bool all_started = false;
   int first_shift = bits - prefix_bits;
   while(true) {
     for(int shift = first_shift; shift < bits; shift += 8) {
@@ -493,6 +499,10 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
       __syncthreads();
       // per digit: prefix over the warps (two threads a digit, half the warps
       // each); the digit's total goes to every block of the cluster
+      if(!all_started) {
+        cl.barrier_wait();
+        all_started = true;
+      }
       {
         const int d = t >> 1, part = t & 1;
         unsigned c[SC_WARPS / 2], sum = 0;
