@@ -281,7 +281,9 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_vsig(Particles P, Lists Ls,
 // Bound by the FP64 pipe.  Per pair of a uniform-h run 3D: ~60 operations, and
 // ~35 more in the branch of approaching pairs, which holds what only the
 // viscosity needs (its two divisions among them); recomputing every division
-// per pair (six and a root) took 130 and more.
+// per pair (six and a root) took 130 and more.  The other pairs' Pi, zero or
+// (pi_apart) a NaN, takes integer operations and a gather of c_s: 0.153 ->
+// 0.155 ms at 8k particles, 2.34 either way at 91k.
 template<int D, int K, bool VSIG>
 __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   PhysParams pp, Lists Ls, int kick, const DevTime * tm, const double * prho2,
@@ -304,6 +306,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   for(int d = 0; d < D; ++d)
     v12a[d] = VH[d][a];
   const double Prho2_a = prho2[a];
+  const bool part_a = pi_part(pp, P.f[F_ALPHA], a, rho_a, c_a);
   double acc[3] = {0, 0, 0};
   double vsig = 0.0;
   const int cnt = Ls.cnt[a];
@@ -333,21 +336,28 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
       const PairR r = pair_r(dist2);
       const double f = pair_g<D, K>(r, ph, pp);
       // mu and Pi are zero unless the pair approaches (viscosity.h:81-93)
-      double Pi = 0.0, appr = 0.0;
+      const double cn_b = CS[b], Prho2_b = prho2[b];
+      double Pi, appr;
       if(dotp < 0.0) {
         Pi = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + RHO[b]),
-          .5 * (c_a + CS[b]), ph.h, dotp, dist2);
+          .5 * (c_a + cn_b), ph.h, dotp, dist2);
         if(VSIG)
           appr = approach<D>(v12_ab, pos_ab, r);
       }
+      else {
+        // (a density that is a NaN shows in P / rho^2)
+        Pi = pi_apart(part_a, pi_part(pp, P.f[F_ALPHA], b,
+          nan64(Prho2_b) ? RHO[b] : 0.0, cn_b), dotp);
+        appr = nan64(dotp) ? dotp : 0.0;  // the pair drops out of the maximum
+      }
       if(VSIG && nonzero(dist2)) {
-        const double c_b = b >= a ? CS[b] : cs_old[b];
+        const double c_b = b >= a ? cn_b : cs_old[b];
         const double cand = (c_a < c_b ? c_b : c_a) - appr;
         vsig = vsig < cand ? cand : vsig;
       }
       // the self pair, coincident pairs and padding slots have x_ab = 0 and
       // f = 0: their terms vanish, as the reference's m_b = 0 makes them
-      const double s = -M[b] * (Prho2_a + prho2[b] + Pi);
+      const double s = -M[b] * (Prho2_a + Prho2_b + Pi);
       for(int d = 0; d < D; ++d)
         acc[d] += pos_ab[d] * f * s;
       if(pw)
@@ -385,11 +395,13 @@ __device__ __forceinline__ double2 pair_terms(const Particles & P, const PhysPar
     dotp += (v12a[d] - P.f[F_VHX + d][b]) * pos_ab[d];
   }
   ph.template set<false, true>(h_a, P.f[F_H][b], pp);
-  double2 t = make_double2(pair_g<D, K>(pair_r(dist2), ph, pp), 0.0);
-  if(dotp < 0.0)
-    t.y = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + P.f[F_RHO][b]),
-      .5 * (c_a + P.f[F_CS][b]), ph.h, dotp, dist2);
-  return t;
+  const double rho_b = P.f[F_RHO][b], c_b = P.f[F_CS][b];
+  const double Pi = dotp < 0.0
+    ? pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + rho_b), .5 * (c_a + c_b), ph.h,
+        dotp, dist2)
+    : pi_apart(pi_part(pp, P.f[F_ALPHA], a, rho_a, c_a),
+        pi_part(pp, P.f[F_ALPHA], b, rho_b, c_b), dotp);
+  return make_double2(pair_g<D, K>(pair_r(dist2), ph, pp), Pi);
 }
 
 // compute_dudt (default_physics.h:421-487).  KEPT: the pair terms of the

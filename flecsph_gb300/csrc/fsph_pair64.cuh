@@ -283,6 +283,29 @@ __device__ __forceinline__ double pair_pi(const PhysParams & pp, const double * 
   return visc_pi_pp(pp, ALPHA, a, b, rho_ab, c_ab, mu);
 }
 
+// Neither infinite nor NaN, on the integer pipe
+__device__ __forceinline__ bool finite64(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+__device__ __forceinline__ bool nan64(double x) {
+  return ((unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull) >
+         0x7ff0000000000000ull;
+}
+
+// Pi_ab of any other pair.  The reference forms it there too, with mu times
+// (dotp < 0): zero, but a NaN where the product v_ab . x_ab, a sound speed or
+// an alpha is not finite or a density is a NaN, and so the acceleration and
+// the energy rates carry it.  pi_part: what one particle has to do with that;
+// neither takes an FP64 operation.
+__device__ __forceinline__ bool pi_part(const PhysParams & pp, const double * ALPHA, int i,
+  double rho, double c) {
+  return finite64(c) && !nan64(rho) && (!pp.cullen || finite64(ALPHA[i]));
+}
+__device__ __forceinline__ double pi_apart(bool part_a, bool part_b, double dotp) {
+  return part_a && part_b && finite64(dotp) ? 0.0
+                                            : __longlong_as_double(0x7ff8000000000000ll);
+}
+
 // min(v_ab . x_ab / r_ab, 0), the approach speed of the signal speed
 // (default_physics.h:254-262)
 template<int D>
