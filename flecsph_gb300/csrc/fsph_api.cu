@@ -258,13 +258,6 @@ bool params_supported(const fsph_params * p, std::string * why) {
   return true;
 }
 
-// positions, velocities, thermodynamics or h changed: no derived record of
-// the state is current any more
-void records_stale(fsph_ctx * c) {
-  c->ahyd_ok = c->fv_ok = c->fdv_ok = c->vel_ok = false;
-  c->prho2_ok = c->pair64_ok = false;
-}
-
 fsph_status set_device(fsph_ctx * c) {
   CK(cudaSetDevice(c->device));
   return FSPH_OK;
@@ -630,7 +623,7 @@ static fsph_status upload_impl(fsph_ctx * c, const fsph_soa_view * v,
   if(!c || !v || v->n < 2 || v->n > c->cap || !v->x || !v->y ||
      (c->p.dimension == 3 && !v->z) || !v->m || !v->h || !v->id)
     return FSPH_ERR_ARG;
-  records_stale(c);
+  c->records_stale();
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -704,7 +697,7 @@ static fsph_status upload_fields_impl(fsph_ctx * c, const fsph_soa_view * v,
   cudaMemcpyKind kind) {
   if(!c || !v || !c->uploaded || v->n != c->n)
     return FSPH_ERR_ARG;
-  records_stale(c);
+  c->records_stale();
   fsph_status s = set_device(c);
   if(s)
     return s;
@@ -899,7 +892,7 @@ fsph_status fsph_update_iteration(fsph_ctx * c) { return update_iteration(c, fal
 static fsph_status update_iteration(fsph_ctx * c, bool range_known) {
   if(!c || !c->uploaded)
     return FSPH_ERR_STATE;
-  records_stale(c);
+  c->records_stale();
   c->grav_nodes_ok = false;
   fsph_status s = set_device(c);
   if(s)
@@ -1200,7 +1193,7 @@ static fsph_status elem(fsph_ctx * c, int op, int phase) {
   if(op != OP_KICK_V && op != OP_KICK_E && op != OP_KICK_U &&
      op != OP_SET_TOTAL_ENERGY && op != OP_DRAG_ACC && op != OP_DRAG_DEDT &&
      op != OP_DRAG_DUDT && op != OP_CHECK_NANS && op != OP_CHECK_NEGATIVITY)
-    records_stale(c);
+    c->records_stale();
   if(op == OP_KICK_V)
     c->fdv_ok = c->vel_ok = false;
   fsph_status s = set_device(c);
@@ -1213,7 +1206,7 @@ static fsph_status elem(fsph_ctx * c, int op, int phase) {
 }
 
 static fsph_status kick_drift(fsph_ctx * c, int op, bool with_range) {
-  records_stale(c);
+  c->records_stale();
   fsph_status s = set_device(c);
   if(s)
     return s;

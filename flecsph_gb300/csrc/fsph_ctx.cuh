@@ -99,6 +99,13 @@ struct fsph_ctx {
     bool sent[fsph::NF + 2] = {};  // NF fields, then id, key
   } io;
 
+  // positions, velocities, thermodynamics or h changed: no derived record of
+  // the state is current any more
+  void records_stale() {
+    ahyd_ok = fv_ok = fdv_ok = vel_ok = false;
+    prho2_ok = pair64_ok = false;
+  }
+
   // kernels are chained on the stream; in a captured graph, where the lanes of
   // an ensemble fill each other's gaps, it gained nothing (32 members: 14.2 ms
   // a run either way)

@@ -50,7 +50,11 @@ HostView view_of(const fsph_ctx * c) {
   return HostView{c->P, c->Palt, c->cs_new, c->n, c->tree_ok};
 }
 
+// The flags of the derived records (P / rho^2, pair terms, the pressure-only
+// acceleration and the rest) tell what the calls on the context left last, not
+// what a captured or replayed iteration does: none holds any more.
 void apply_view(fsph_ctx * c, const HostView & v) {
+  c->records_stale();
   c->P = v.P;
   c->Palt = v.Palt;
   c->cs_new = v.cs_new;
