@@ -3,6 +3,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cctype>
 #include <cmath>
 #include <cstdio>
@@ -256,6 +257,34 @@ bool params_supported(const fsph_params * p, std::string * why) {
     return false;
   }
   return true;
+}
+
+// The FP64 pair terms (16 B per list slot, 4 KB a particle at the default
+// capacity) only save the energy passes a second evaluation (91k Sedov: 0.56
+// against 2.19 ms a de/dt pass), so they must not crowd anything out: all contexts
+// of a device together hold at most 1/32 of its memory for them (9.3 GB: two
+// million particles), and a context takes them only where they are at most a
+// quarter of what is free.  The others evaluate.
+std::atomic<long long> pair64_held[64];
+
+bool pair64_reserve(fsph_ctx * c, size_t bytes) {
+  size_t mfree = 0, mtotal = 0;
+  if(c->device >= 64 || cudaMemGetInfo(&mfree, &mtotal) != cudaSuccess || bytes > mfree / 4)
+    return false;
+  std::atomic<long long> & held = pair64_held[c->device];
+  long long now = held.load();
+  do {
+    if(now + (long long)bytes > (long long)(mtotal / 32))
+      return false;
+  } while(!held.compare_exchange_weak(now, now + (long long)bytes));
+  c->pair64_bytes = bytes;
+  return true;
+}
+
+void pair64_give_back(fsph_ctx * c) {
+  if(c->pair64_bytes)
+    pair64_held[c->device] -= (long long)c->pair64_bytes;
+  c->pair64_bytes = 0;
 }
 
 fsph_status set_device(fsph_ctx * c) {
@@ -534,15 +563,11 @@ fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
     return fail(FSPH_ERR_OOM);
   }
   if(!c->mixed) {
-    // The pair terms (16 B per list slot) only save the energy passes a second
-    // evaluation: taken where they leave at least three quarters of the free
-    // memory to everything else (4 KB a particle at the default capacity)
     const size_t slots = Npad * (size_t)c->Ls.maxnb;
-    size_t mfree = 0, mtotal = 0;
-    if(cudaMemGetInfo(&mfree, &mtotal) == cudaSuccess &&
-       slots <= mfree / 4 / sizeof(double2) &&
+    if(pair64_reserve(c, slots * sizeof(double2)) &&
        dalloc(c, &c->pair64, slots) != cudaSuccess) {
       c->pair64 = nullptr;
+      pair64_give_back(c);
       cudaGetLastError();
     }
   }
@@ -567,6 +592,7 @@ void fsph_destroy(fsph_ctx * c) {
     cudaStreamSynchronize(c->io.stream);
   for(void * p : c->allocs)
     cudaFree(p);
+  pair64_give_back(c);
   if(c->let_buf)
     cudaFree(c->let_buf);
   for(auto & e : c->events)

@@ -273,7 +273,14 @@ void fsph_params_default(fsph_params * p);
 fsph_status fsph_params_set_external_force(fsph_params * p,
   const char * external_force_type);
 int32_t fsph_abi_version(void);
-/* Creates a context on `device` able to hold `capacity` particles. */
+/* Creates a context on `device` able to hold `capacity` particles.  Its
+ * device memory is taken here and freed by fsph_destroy: about 1 KB a particle
+ * and 4 bytes per list slot (max_neighbors, rounded up to a multiple of four;
+ * gravity over ranks adds a buffer of cell records on demand).
+ * With FSPH_PRECISION_FP64 the acceleration's pair terms take 16 bytes per
+ * slot more where all contexts of the device together then hold at most 1/32
+ * of its memory for them, and a quarter of the free memory suffices; otherwise
+ * the energy passes evaluate them again (the same results, slower). */
 fsph_ctx * fsph_create(const fsph_params * p, int32_t device, int64_t capacity,
   fsph_status * status);
 void fsph_destroy(fsph_ctx * ctx);
