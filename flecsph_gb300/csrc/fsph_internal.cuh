@@ -312,6 +312,7 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long> * mask, F app
 // and maximum), [8] blocks done (0 between passes), [9] the
 // key sort's mark.  range_part: RANGE_PART
 // words of scratch, free until the keys are sorted.
+#define RANGE_TICKET 8
 #define RANGE_MARK 9
 #define RANGE_WORDS 10
 #define RANGE_BLOCKS (152 * 8)

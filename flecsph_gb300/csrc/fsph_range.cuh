@@ -102,7 +102,7 @@ struct RangeAcc {
     }
     __syncthreads();
     if(t == 0)
-      s_final = atomicAdd((unsigned *)(range + 8), 1u) == gridDim.x - 1;
+      s_final = atomicAdd((unsigned *)(range + RANGE_TICKET), 1u) == gridDim.x - 1;
     __syncthreads();
     if(!s_final)
       return;
@@ -129,7 +129,7 @@ struct RangeAcc {
         range[t] = (t < 3 || t == 6) ? x : ~x;
     }
     if(t == 0)
-      *(unsigned *)(range + 8) = 0u;
+      *(unsigned *)(range + RANGE_TICKET) = 0u;
   }
 };
 

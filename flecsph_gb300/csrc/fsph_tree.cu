@@ -2223,9 +2223,12 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
   pp.dim = dimension;
   long long launches = 0;
   Launch L{(cudaStream_t)stream, &launches};
-  // every scratch word that is read is first written by these launches (the
-  // range's partial words share the keys' scratch), but the range's block
-  // counter: zero at load, and left zero by every call
+  // every scratch word that is read is first written by this call: the range's
+  // block counter here (calls that overlapped, which the caller must not make,
+  // could have left it at any value), the rest by the launches (the range's
+  // partial words share the keys' scratch)
+  if(cudaMemsetAsync(range + RANGE_TICKET, 0, sizeof(*range), L.stream) != cudaSuccess)
+    return FSPH_ERR_CUDA;
   if(launch_range(L, P, pp, range, ktmp) != cudaSuccess ||
      launch_keys(L, P, pp, range, (unsigned long long *)keys_out, perm_out) != cudaSuccess)
     return FSPH_ERR_CUDA;
