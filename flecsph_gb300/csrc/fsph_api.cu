@@ -953,7 +953,7 @@ static fsph_status update_iteration(fsph_ctx * c, bool range_known) {
   {
     Phase ph(c, FSPH_TIMER_SORT);
     CK(radix_sort_pairs(L, c->skeys, c->svals, c->skeys_tmp, c->svals_tmp, n,
-      c->hist, 63 / c->pp.dim * c->pp.dim, (unsigned *)(c->d_range + RANGE_MARK)));
+      c->hist, 63 / c->pp.dim * c->pp.dim, (unsigned *)(c->d_range + RANGE_SORT)));
     if(c->io.h2d_pending) {
       // fsph_step_io: input fields copied on the copy stream land first
       CK(cudaStreamWaitEvent(c->stream, c->io.ev[0], 0));

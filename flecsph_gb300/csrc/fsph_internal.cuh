@@ -309,11 +309,11 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long> * mask, F app
 
 // ---- fsph_tree.cu ----
 // Range words: [0..7] ordered encodings (x - h minima, x + h maxima, h minimum
-// and maximum), [8] blocks done (0 between passes), [9] the
-// key sort's mark.  range_part: RANGE_PART
-// words of scratch, free until the keys are sorted.
+// and maximum), [8] blocks done (0 between passes), [9] the key sort's two state
+// words.  range_part: RANGE_PART words of scratch, free until the keys are
+// sorted.
 #define RANGE_TICKET 8
-#define RANGE_MARK 9
+#define RANGE_SORT 9
 #define RANGE_WORDS 10
 #define RANGE_BLOCKS (152 * 8)
 #define RANGE_PART (8 * RANGE_BLOCKS)
@@ -321,11 +321,11 @@ cudaError_t launch_range(const Launch & L, const Particles & P, const PhysParams
   unsigned long long * range, unsigned long long * range_part);
 cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams & pp,
   const unsigned long long * range, unsigned long long * keys_out, int * idx_out);
-// `bits`: the data bits of the keys, below a constant marker bit; `mark`: a
-// word of scratch
+// `bits`: the data bits of the keys, below a constant marker bit; `state`: the
+// sort's two words, zero before the first one
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
-  unsigned * hist, int bits, unsigned * mark);
+  unsigned * hist, int bits, unsigned * state);
 size_t radix_hist_entries(int n);
 // the fields not in `skip`, id and key[i] in the order of perm
 cudaError_t launch_gather(const Launch & L, const Particles & src, const Particles & dst,

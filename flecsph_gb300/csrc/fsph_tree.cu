@@ -154,6 +154,14 @@ cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams 
 // keys that share a prefix in order; a run of more than RS_RUN_MAX of them
 // (particles crowded into a small part of the range) marks the sort, and the
 // eight passes over all bits follow, which return at once without the mark.
+// Such sets stay so from step to step, and four passes in vain are half a sort:
+// SORT_CROWDED keeps the mark for the next build, which then makes the eight
+// passes only, until no long run is left (k_crowded).  The word chooses between
+// two ways to the same order, so whatever set it belongs to does no harm.
+// A lattice with one particle 39 times its size away, sort and permute, every
+// build trying the prefix first -> this (ms): 132k (one cluster) 0.188 -> 0.136,
+// 2M 0.60 -> 0.50; beside one 3,000 times away 216k 0.190 -> 0.16, 1M 0.342 ->
+// 0.308, 2M 0.515 -> 0.47.
 // Sort with the permute, all bits -> prefix (ms): 216k 0.140 -> 0.103, 552k 0.178
 // -> 0.150, 1M 0.278 -> 0.228, 2M 0.480 -> 0.327, 4M star 0.884 -> 0.664, 19.7M
 // 3.59 -> 2.67.
@@ -170,6 +178,17 @@ cudaError_t launch_keys(const Launch & L, const Particles & P, const PhysParams 
 
 #define RS_RUN_MAX 24
 
+// The sort's two state words: [0] the passes over all bits are due in this sort
+// (set anew by each), [1] the last sort's keys were crowded.  The passes' part
+// in it: over the prefix or over all bits, and the first of each, which sets up
+// the words.
+#define SORT_CROWDED 1
+enum { SORT_PREFIX = 0, SORT_FULL = 1, SORT_FIRST = 2 };
+
+__device__ __forceinline__ bool sort_due(const unsigned * state, int part) {
+  return (part & SORT_FULL) ? state[0] != 0u : state[SORT_CROWDED] == 0u;
+}
+
 size_t radix_hist_entries(int n) {
   size_t nb = ((size_t)n + RS_TILE - 1) / RS_TILE;
   return 256 * nb + 256;  // [digit][tile] counts, then the 256 digit totals
@@ -177,12 +196,15 @@ size_t radix_hist_entries(int n) {
 
 __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
   const unsigned long long * keys, int n, int shift, unsigned * hist,
-  const unsigned * gate, unsigned * clear) {
+  unsigned * state, int part) {
   chain_begin();
-  if(gate && *gate == 0u)
+  const bool setup = (part & SORT_FIRST) && blockIdx.x == 0 && threadIdx.x == 0;
+  if(setup && !(part & SORT_FULL))
+    state[0] = state[SORT_CROWDED];
+  if(!sort_due(state, part))
     return;
-  if(clear && blockIdx.x == 0 && threadIdx.x == 0)
-    *clear = 0u;
+  if(setup && (part & SORT_FULL))
+    state[SORT_CROWDED] = 0u;
   __shared__ unsigned sh[256];
   sh[threadIdx.x] = 0;
   __syncthreads();
@@ -206,9 +228,9 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(
 // Per digit: exclusive scan of its row of tile counts (coalesced, one
 // block per digit) and the row total in tot[digit].
 __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
-  unsigned * tot, const unsigned * gate) {
+  unsigned * tot, const unsigned * state, int part) {
   chain_begin();
-  if(gate && *gate == 0u)
+  if(!sort_due(state, part))
     return;
   __shared__ unsigned wsum[32];
   const int d = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -256,9 +278,9 @@ __global__ void __launch_bounds__(1024) k_scan_rows(unsigned * hist, int nb,
 #define RS_DYN_SMEM ((size_t)RS_TILE * 12)
 __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter(
   const unsigned long long * kin, const int * vin, unsigned long long * kout,
-  int * vout, int n, int shift, const unsigned * offs, const unsigned * gate) {
+  int * vout, int n, int shift, const unsigned * offs, const unsigned * state, int part) {
   chain_begin();
-  if(gate && *gate == 0u)
+  if(!sort_due(state, part))
     return;
   extern __shared__ __align__(16) unsigned char rs_dyn[];
   unsigned long long * skey = (unsigned long long *)rs_dyn;
@@ -352,10 +374,10 @@ __global__ void __launch_bounds__(RS_THREADS, RS_SCATTER_BLOCKS) k_radix_scatter
 // a prefix orders it in place, ties as they are (the others see the same
 // prefixes meanwhile).  One read of the keys where there are no runs.
 __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, int * vals,
-  int n, int low, unsigned * mark) {
+  int n, int low, unsigned * state) {
   chain_begin();
   const int i = blockIdx.x * 256 + threadIdx.x;
-  if(i + 1 >= n)
+  if(i + 1 >= n || !sort_due(state, SORT_PREFIX))
     return;
   const unsigned long long p = keys[i] >> low;
   if(keys[i + 1] >> low != p || (i > 0 && keys[i - 1] >> low == p))
@@ -363,7 +385,7 @@ __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, 
   int len = 2;
   while(i + len < n && keys[i + len] >> low == p)
     if(++len > RS_RUN_MAX) {
-      *mark = 1u;
+      state[0] = 1u;
       return;
     }
   for(int j = i + 1; j < i + len; ++j) {
@@ -379,6 +401,23 @@ __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, 
       vals[m] = v;
     }
   }
+}
+
+// After the passes over all bits: are the keys still crowded, that is, would the
+// passes over the prefix leave a run that k_prefix_runs does not take?
+__global__ void __launch_bounds__(256) k_crowded(const unsigned long long * keys, int n,
+  int low, unsigned * state) {
+  chain_begin();
+  if(!sort_due(state, SORT_FULL))
+    return;
+  int found = 0;
+  for(int i = blockIdx.x * 256 + threadIdx.x; i + RS_RUN_MAX < n && !found;
+      i += gridDim.x * 256)
+    found = keys[i] >> low == keys[i + RS_RUN_MAX] >> low;
+  // few blocks, one store each: of 8,192 blocks the stores to one word alone
+  // took 0.1 ms
+  if(__syncthreads_or(found) && threadIdx.x == 0)
+    state[SORT_CROWDED] = 1u;
 }
 
 // ---- one-cluster sort --------------------------------------------------
@@ -401,7 +440,9 @@ __global__ void __launch_bounds__(256) k_prefix_runs(unsigned long long * keys, 
 // particles spread over the range apart (the prefix has at least 32 values per
 // particle); keys that share a prefix are adjacent then, in input order, and
 // the thread of the first sorts them by insertion.  A run longer than SC_RUN
-// (a clump in a wide range) makes the cluster go on with all eight passes.
+// (a clump in a wide range) makes the cluster go on with all eight passes, and
+// start with them in the next sort (SORT_CROWDED, as below, until no such run
+// is left).
 #define SC_THREADS 512
 #define SC_WARPS (SC_THREADS / 32)
 #define SC_ITEMS 17
@@ -420,7 +461,7 @@ __host__ __device__ constexpr size_t sc_smem(int per) {
 
 __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
   unsigned long long * keys, int * vals, unsigned long long * keys_tmp, int * vals_tmp,
-  int n, int per, int bits, int prefix_bits) {
+  int n, int per, int bits, int prefix_bits, unsigned * state) {
   chain_begin();
   extern __shared__ __align__(16) unsigned char sc_dyn[];
   unsigned long long * okey = (unsigned long long *)sc_dyn;
@@ -446,7 +487,13 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
   // counts, which the loads and ballots before it leave time for.
   cl.barrier_arrive();
   bool all_started = false;
-  int first_shift = bits - prefix_bits;
+  const int low = bits - prefix_bits;
+  // (every block has read the word before any passes the barrier after which
+  // it is written)
+  const bool crowded = state[SORT_CROWDED] != 0u;
+  int first_shift = crowded ? 0 : low;
+  if(crowded)
+    bits = 64;
   while(true) {
     for(int shift = first_shift; shift < bits; shift += 8) {
       // warp w owns the places [w * 32 * rounds, ...) of the block
@@ -603,6 +650,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
           cl.map_shared_rank(aux, b)[16] = 1;
       }
     cl.sync();
+    if(aux[16] && me == 0 && t == 0)
+      state[SORT_CROWDED] = 1u;
     if(!aux[16]) {
       // the first of a run puts it in order, the keys that begin no run and
       // belong to none are in place
@@ -639,6 +688,17 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
       keys[g0 + i] = __ldcg(kin + g0 + i);
       vals[g0 + i] = __ldcg(vin + g0 + i);
     }
+  if(crowded) {
+    // still so?
+    int found = 0;
+    for(int i = t; i < mine && g0 + i + SC_RUN < n && !found; i += SC_THREADS)
+      found = __ldcg(kin + g0 + i) >> low == __ldcg(kin + g0 + i + SC_RUN) >> low;
+    if(__syncthreads_or(found) && t == 0)
+      cl.map_shared_rank(aux, 0)[16] = 1;
+    cl.sync();
+    if(me == 0 && t == 0)
+      state[SORT_CROWDED] = aux[16];
+  }
 }
 
 // Blocks of the cluster for n keys, 0 where the sort takes several launches:
@@ -689,7 +749,7 @@ static int sc_blocks(int n) {
 
 cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   int * vals, unsigned long long * keys_tmp, int * vals_tmp, int n,
-  unsigned * hist, int bits, unsigned * mark) {
+  unsigned * hist, int bits, unsigned * state) {
   if(const int c = sc_blocks(n)) {
     const int per = ((n + c - 1) / c + 3) & ~3;
     // prefix bits: at least 32 prefixes per key, in whole digits
@@ -711,7 +771,7 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
     cfg.numAttrs = L.chained ? 2 : 1;
     *L.counter += 1;
     return cudaLaunchKernelEx(&cfg, k_sort_cluster, keys, vals, keys_tmp, vals_tmp, n, per,
-      bits, pb);
+      bits, pb, state);
   }
   static std::atomic<unsigned long long> attr_devices{0};
   cudaError_t ae = once_per_device(&attr_devices, []() {
@@ -724,12 +784,13 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
   unsigned long long *ka = keys, *kb = keys_tmp;
   int *va = vals, *vb = vals_tmp;
   // an even number of passes: the result is back in (keys, vals)
-  auto passes = [&](int from, int to, const unsigned * gate, unsigned * clear) {
+  auto passes = [&](int from, int to, int part) {
     for(int shift = from; shift < to; shift += 8) {
-      chain(L, k_radix_hist, nb, RS_THREADS, 0, ka, n, shift, hist, gate, clear);
-      chain(L, k_scan_rows, 256, 1024, 0, hist, nb, hist + (size_t)256 * nb, gate);
+      const int p = shift == from ? part | SORT_FIRST : part;
+      chain(L, k_radix_hist, nb, RS_THREADS, 0, ka, n, shift, hist, state, p);
+      chain(L, k_scan_rows, 256, 1024, 0, hist, nb, hist + (size_t)256 * nb, state, p);
       chain(L, k_radix_scatter, nb, RS_THREADS, RS_DYN_SMEM, ka, va, kb, vb, n,
-        shift, hist, gate);
+        shift, hist, state, p);
       *L.counter += 3;
       unsigned long long * tk = ka;
       ka = kb;
@@ -737,17 +798,17 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
       int * tv = va;
       va = vb;
       vb = tv;
-      clear = nullptr;
     }
   };
   int lg = 0;
   while((1ll << lg) < n)
     ++lg;
   const int low = bits - (lg + 5 + 15) / 16 * 16;
-  passes(low, bits, nullptr, mark);
-  chain(L, k_prefix_runs, (n + 255) / 256, 256, 0, keys, vals, n, low, mark);
-  *L.counter += 1;
-  passes(0, 64, mark, nullptr);
+  passes(low, bits, SORT_PREFIX);
+  chain(L, k_prefix_runs, (n + 255) / 256, 256, 0, keys, vals, n, low, state);
+  passes(0, 64, SORT_FULL);
+  chain(L, k_crowded, 152 * 2, 256, 0, keys, n, low, state);
+  *L.counter += 2;
   return cudaGetLastError();
 }
 
@@ -2226,7 +2287,8 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
   // every scratch word that is read is first written by this call: the range's
   // block counter here (calls that overlapped, which the caller must not make,
   // could have left it at any value), the rest by the launches (the range's
-  // partial words share the keys' scratch)
+  // partial words share the keys' scratch), but SORT_CROWDED, which may hold
+  // any value
   if(cudaMemsetAsync(range + RANGE_TICKET, 0, sizeof(*range), L.stream) != cudaSuccess)
     return FSPH_ERR_CUDA;
   if(launch_range(L, P, pp, range, ktmp) != cudaSuccess ||
@@ -2234,7 +2296,7 @@ extern "C" fsph_status fsph_sort_keys_noalloc(const double * x,
     return FSPH_ERR_CUDA;
   if(radix_sort_pairs(L, (unsigned long long *)keys_out, perm_out, ktmp, vtmp,
        (int)n, hist, 63 / dimension * dimension,
-       (unsigned *)(range + RANGE_MARK)) != cudaSuccess)
+       (unsigned *)(range + RANGE_SORT)) != cudaSuccess)
     return FSPH_ERR_CUDA;
   return FSPH_OK;
 }
