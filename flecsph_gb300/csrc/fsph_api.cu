@@ -957,15 +957,14 @@ static fsph_status update_iteration(fsph_ctx * c, bool range_known) {
     if(c->io.h2d_pending) {
       // fsph_step_io: input fields copied on the copy stream land first
       CK(cudaStreamWaitEvent(c->stream, c->io.ev[0], 0));
+      c->joined = true;
       c->io.h2d_pending = false;
-      L.chained = false;
     }
     // the mixed float-float path's {v, c_s} records come out of the permute
     float4 * vel = c->mixed && wendland(c->pp.kernel) ? c->K.vel : nullptr;
     CK(launch_permute(L, c->P, c->Palt, c->svals, c->skeys, c->permute_skip, c->d_range,
       c->K, c->T.ngroups, c->Ls.stat, vel, c->pp.dim));
     c->vel_ok = vel != nullptr;
-    L = c->L();
     Particles t = c->P;
     c->P = c->Palt;
     c->Palt = t;
@@ -1561,11 +1560,13 @@ fsph_status fsph_step_io(fsph_ctx * c, const fsph_soa_view * in, fsph_soa_view *
   c->io.active = false;
   if(c->io.h2d_pending) {  // the step stopped before the permute
     cudaStreamWaitEvent(c->stream, c->io.ev[0], 0);
+    c->joined = true;
     c->io.h2d_pending = false;
   }
   // the context's stream continues after the copies
   CK(cudaEventRecord(c->io.ev[7], c->io.stream));
   CK(cudaStreamWaitEvent(c->stream, c->io.ev[7], 0));
+  c->joined = true;
   if(s)
     return s;
   return fsph_sync(c);

@@ -76,6 +76,7 @@ struct fsph_ctx {
   bool prho2_ok = false;
   bool pair64_ok = false;
   bool uploaded = false;
+  bool joined = false;  // the stream waits for another one (Launch::joined)
   long long launches = 0;
   // timers
   bool timing = false;
@@ -114,6 +115,6 @@ struct fsph_ctx {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     const bool plain = cudaStreamIsCapturing(stream, &st) == cudaSuccess &&
                        st == cudaStreamCaptureStatusNone;
-    return fsph::Launch{stream, &launches, plain};
+    return fsph::Launch{stream, &launches, plain, &joined};
   }
 };

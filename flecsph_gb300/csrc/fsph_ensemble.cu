@@ -275,8 +275,10 @@ fsph_status lanes_wait_members(fsph_ensemble * e) {
 fsph_status members_wait_lanes(fsph_ensemble * e) {
   for(int l = 0; l < e->lanes; ++l)
     ECK(cudaEventRecord(e->lane_done[l], e->lane_stream[l]));
-  for(auto & mb : e->m)
+  for(auto & mb : e->m) {
     ECK(cudaStreamWaitEvent(mb.c->stream, e->lane_done[mb.lane], 0));
+    mb.c->joined = true;
+  }
   return FSPH_OK;
 }
 

@@ -239,6 +239,17 @@ struct Launch {
   cudaStream_t stream;
   long long * counter;  // launches issued
   bool chained = false; // may chain() overlap this launch with the one before
+  // set where the stream waits for another stream's event (null: it never
+  // does): the next launch does not overlap what came before
+  bool * joined = nullptr;
+  bool overlap() const {
+    if(!chained)
+      return false;
+    const bool first = joined && *joined;
+    if(first)
+      *joined = false;
+    return !first;
+  }
 };
 
 // The kernels of one iteration follow each other on one stream.  With chain()
@@ -247,8 +258,10 @@ struct Launch {
 // chain_begin() until all of that kernel has finished and its writes can be
 // seen.  chain_begin() is the first statement of every kernel launched so,
 // ahead of any access to memory and of any return: a kernel that ended before
-// its predecessor would let its successor start too early.  Work that is not a
-// chained kernel (copies, events, the other kernels) is ordered as ever.
+// its predecessor would let its successor start too early.  What griddepcontrol
+// waits for is the kernel before, so the first launch behind a wait for another
+// stream's event (Launch::joined) is a plain one; other work that is not a
+// chained kernel (copies, the other kernels) is ordered as ever.
 // Ten iterations, plain launches -> chained: 2k particles in 2D 2.83 -> 2.26 ms,
 // 32k in 3D by single calls 2.33 -> 2.04, 50k star 2.75 -> 2.67, 133k 3.66 -> 3.52,
 // 8k in FP64 2.38 -> 2.26, 2M 26.6 -> 26.2.  No block calls
@@ -267,7 +280,7 @@ inline cudaError_t chain(const Launch & L, void (*kernel)(P...), dim3 grid,
   cfg.dynamicSmemBytes = smem;
   cfg.stream = L.stream;
   cfg.attrs = at;
-  cfg.numAttrs = L.chained ? 1 : 0;
+  cfg.numAttrs = L.overlap() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 

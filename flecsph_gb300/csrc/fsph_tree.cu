@@ -768,7 +768,7 @@ cudaError_t radix_sort_pairs(const Launch & L, unsigned long long * keys,
     cfg.dynamicSmemBytes = sc_smem(per);
     cfg.stream = L.stream;
     cfg.attrs = at;
-    cfg.numAttrs = L.chained ? 2 : 1;
+    cfg.numAttrs = L.overlap() ? 2 : 1;
     *L.counter += 1;
     return cudaLaunchKernelEx(&cfg, k_sort_cluster, keys, vals, keys_tmp, vals_tmp, n, per,
       bits, pb, state);
