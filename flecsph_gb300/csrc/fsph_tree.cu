@@ -2097,8 +2097,10 @@ __global__ void __launch_bounds__(NB_WARPS * 32,
                   mask = __funnelshift_l(__float_as_uint(t[q]), mask, 1);
                 }
               }
-              if(slack <= mgc) {
-                // some pair lies inside the margin: candidate by candidate
+              if(slack <= mgc || !(rc < 1e18f)) {
+                // some pair lies inside the margin, or the squares may overflow
+                // and t be a NaN, which the slack does not show: candidate by
+                // candidate
                 mask = 0u;
                 for(int c = c0; c < c0 + 32 && c < ncand; ++c) {
                   const float dx = ax + cxs[c], dy = ay + cys[c], dz = az + czs[c];
