@@ -210,7 +210,9 @@ struct GravBuffers {
   float4 * gpk;        // 2 n
 };
 
-#define LIST_STAT_MAX (1 << 18)
+// Particles up to which the mixed pair passes choose their lanes by the list
+// statistics (SPLIT_MAX), so the walk keeps these no further
+#define LIST_STAT_MAX (1 << 17)
 // Neighbour lists, interleaved by warp in chunks of four slots:
 // [(i>>5)][slot/4][i&31][slot%4], so a lane reads four slots with one
 // 16-byte load and a warp reads 512 contiguous bytes.  maxnb is a multiple
@@ -220,8 +222,8 @@ struct GravBuffers {
 struct Lists {
   int * idx;
   int * cnt;
-  unsigned * stat;  // mixed path: longest list, all pairs (of runs whose pair
-                    // passes ask, up to LIST_STAT_MAX particles)
+  unsigned * stat;  // mixed path: longest list, all pairs (up to
+                    // LIST_STAT_MAX particles)
   int maxnb;
 };
 

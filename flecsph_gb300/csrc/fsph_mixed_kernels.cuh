@@ -282,7 +282,7 @@ __device__ __forceinline__ float vel_diff_dot(const float4 & h1a, const float4 &
 // costs the acceleration of one thread per particle 6 % (132k Sedov), so larger
 // runs, which would not take four lanes, do not have it.
 #ifndef SPLIT_MAX
-#define SPLIT_MAX (1 << 17)
+#define SPLIT_MAX LIST_STAT_MAX
 #endif
 #ifndef SPLIT_PAIRS
 #define SPLIT_PAIRS 24576ull
