@@ -702,7 +702,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_sort_cluster(
 }
 
 // Blocks of the cluster for n keys, 0 where the sort takes several launches:
-// about 1,024 keys a block (one round of ranking) until the cluster is full.
+// a key per thread (one round of ranking), twice the blocks with twice the keys,
+// until the cluster is full.
 // A cluster of 16 is beyond the portable 8: asked of the device once.
 static int sc_blocks(int n) {
   static std::atomic<unsigned long long> ready{0}, wide{0};
