@@ -52,7 +52,7 @@ sys.path.insert(0, ROOT)
 # Algorithmic work per particle and timer phase: the constants of
 # include/fsph_work.h (the one table both this file and the design notes
 # use), parsed from the header.
-HBM_PEAK = 6815.2  # GB/s, MEASURED_PEAKS.json hbm_gbs
+HBM_PEAK = 6782.8  # GB/s, MEASURED_PEAKS.json hbm_gbs
 # ncu dram__bytes_read.sum + dram__bytes_write.sum per particle of the
 # dominant kernel of a phase, from 96^3 Sedov captures (884,736 particles;
 # lists and records well above L2): the walk (459.4 MB,

@@ -4,8 +4,11 @@
 // One thread per particle walks its neighbour list (interleaved layout, so
 // a warp reads 32 consecutive slots per step).  Compiled with -fmad=false and
 // evaluated in the reference's operand order: with lists in the reference's
-// order the results are bit-identical to the reference on the CPU except
-// where libm and CUDA's pow/cbrt differ in the last bit.
+// order the results are those of the reference on the CPU, but for the last
+// bits in which libm's pow and cbrt differ from CUDA's, in which quotients and
+// roots from a reciprocal may (fsph_pair64.cuh: none has been seen to), and in
+// the fused signal speed pairs whose v . x and v . (x / r) round to different
+// signs.
 #include <cuda_runtime.h>
 
 #include "fsph_pair64.cuh"

@@ -1,9 +1,9 @@
 // fsph_mixed_kernels.cuh -- the mixed-precision neighbour-pair kernels
 // (density, acceleration, du/dt, de/dt) as templates over the dimension,
 // the smoothing kernel and the viscosity (Monaghan's constant alpha, or
-// Cullen & Dehnen's per-particle alpha).  fsph_mixed.cu instantiates the
-// constant-alpha kernels and fsph_mixed_cullen.cu the adaptive ones, so
-// the two sets compile in parallel.
+// Cullen & Dehnen's per-particle alpha).  fsph_mixed_pairs.cu instantiates
+// them, an object per viscosity and lane split, so that they compile side by
+// side.
 //
 // Pair arithmetic runs in FP32 on packed per-particle records; the density,
 // force and energy sums are Kahan-compensated; every per-particle quantity
@@ -268,7 +268,8 @@ __device__ __forceinline__ float vel_diff_dot(const float4 & h1a, const float4 &
 // two warps per scheduler, and a pass takes as long as its longest list.  Then
 // every particle gets four lanes: lane q evaluates slot q of each chunk of
 // four, and the terms are added in slot order, by the same operations as a
-// single thread would, so the sums round alike.  The per-particle work that
+// single thread would.  (The compiler may contract the two forms differently,
+// so last bits can differ: 2e-16 in the 50k star.)  The per-particle work that
 // follows a list (FP64 mostly) would waste three lanes of four: a block's
 // particles are handed to its first quarter of threads for it.
 //
