@@ -261,7 +261,7 @@ bool params_supported(const fsph_params * p, std::string * why) {
 
 // The FP64 pair terms (16 B per list slot, 4 KB a particle at the default
 // capacity) only save the energy passes a second evaluation (91k Sedov: 0.56
-// against 2.19 ms a de/dt pass), so they must not crowd anything out: all contexts
+// against 2.08 ms a de/dt pass), so they must not crowd anything out: all contexts
 // of a device together hold at most 1/32 of its memory for them (9.3 GB: two
 // million particles), and a context takes them only where they are at most a
 // quarter of what is free.  The others evaluate.
@@ -1018,8 +1018,10 @@ fsph_status fsph_compute_alpha(fsph_ctx * c) {
   Phase ph(c, FSPH_TIMER_DENSITY);
   if(c->mixed)
     CK(launch_alpha_mixed(L, c->P, c->pp, c->Ls, c->K, c->d_time));
-  else
-    CK(launch_alpha_cullen(L, c->P, c->pp, c->Ls, c->d_time));
+  else {
+    CK(launch_alpha_cullen(L, c->P, c->pp, c->Ls, c->d_time, c->prho2));
+    c->prho2_ok = true;
+  }
   return FSPH_OK;
 }
 
@@ -1077,7 +1079,7 @@ static bool wendland(int k) {
 // FP64 path: P / rho^2 as the state has it now
 static fsph_status prho2_current(fsph_ctx * c) {
   if(!c->prho2_ok)
-    CK(launch_prho2(c->L(), c->P, c->prho2));
+    CK(launch_prho2(c->L(), c->P, c->pp, c->prho2));
   c->prho2_ok = true;
   return FSPH_OK;
 }

@@ -66,10 +66,11 @@ struct fsph_ctx {
   // K.vel holds v and c_s of the current state (written by the permute of
   // update_iteration on the mixed path)
   bool vel_ok = false;
-  // FP64 path: P / rho^2 per particle (written by the density pass; prho2_ok
-  // while P and rho are unchanged since) and the pair terms the acceleration
-  // pass leaves for the energy passes (pair64_ok while positions, h, v_half,
-  // rho, c_s and alpha are; pair64 is null where it would take too much memory)
+  // FP64 path: P / rho^2 per particle (written by the density and the alpha
+  // pass; prho2_ok while P, rho, c_s and alpha are unchanged since) and the pair
+  // terms the acceleration pass leaves for the energy passes (pair64_ok while
+  // positions, h, v_half, rho, c_s and alpha are; pair64 is null where it would
+  // take too much memory)
   double * prho2 = nullptr;
   double2 * pair64 = nullptr;
   size_t pair64_bytes = 0;  // what of pair64_held (fsph_api.cu) is this one's

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
     cs);
   P.f[F_P][a] = Pa;
   cs_new[a] = cs;
-  prho2[a] = Pa / (rho_a * rho_a);
+  prho2[a] = kept_prho2(pp, Pa, rho_a, cs, P.f[F_ALPHA][a]);
   if(CULL) {
     div_v /= rho_a;
     const double div_v_p = P.f[F_DIVV][a];
@@ -115,22 +115,22 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_density(Particles P,
 }
 
 // P / rho^2 of every particle where the density pass's is out of date (a
-// caller changed P or rho in between).
-__global__ void __launch_bounds__(256) k_prho2(Particles P, double * prho2) {
+// caller changed P, rho, c_s or alpha in between).
+__global__ void __launch_bounds__(256) k_prho2(Particles P, PhysParams pp,
+  double * prho2) {
   chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i < P.n) {
-    const double rho = P.f[F_RHO][i];
-    prho2[i] = P.f[F_P][i] / (rho * rho);
-  }
+  if(i < P.n)
+    prho2[i] = kept_prho2(pp, P.f[F_P][i], P.f[F_RHO][i], P.f[F_CS][i], P.f[F_ALPHA][i]);
 }
 
 // viscosity::compute_alpha with A_trigger and compute_xi (viscosity.h:
 // 185-363): Cullen & Dehnen's adaptive alpha from the velocity divergence,
-// its rate and the traceless shear, in the reference's operand order.
+// its rate and the traceless shear, in the reference's operand order.  prho2 is
+// written anew, with the new alpha.
 template<int D, int K>
 __global__ void __launch_bounds__(PAIR_THREADS) k_alpha_cullen(Particles P,
-  PhysParams pp, Lists Ls, const DevTime * tm) {
+  PhysParams pp, Lists Ls, const DevTime * tm, double * prho2) {
   chain_begin();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if(a >= P.n)
@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_alpha_cullen(Particles P,
     alpha = alpha_a * exp(-dalphadt * tm->dt);
   }
   P.f[F_ALPHA][a] = alpha;
+  prho2[a] = kept_prho2(pp, P.f[F_P][a], rho_a, c_a, alpha);
 }
 
 // compute_signalspeed (default_physics.h:236-265).  The reference visits
@@ -284,9 +285,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_vsig(Particles P, Lists Ls,
 // Bound by the FP64 pipe.  Per pair of a uniform-h run 3D: ~60 operations, and
 // ~35 more in the branch of approaching pairs, which holds what only the
 // viscosity needs (its two divisions among them); recomputing every division
-// per pair (six and a root) took 130 and more.  The other pairs' Pi, zero or
-// (pi_apart) a NaN, takes integer operations and a gather of c_s: 0.153 ->
-// 0.155 ms at 8k particles, 2.34 either way at 91k.
+// per pair (six and a root) took 130 and more.
 template<int D, int K, bool VSIG>
 __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   PhysParams pp, Lists Ls, int kick, const DevTime * tm, const double * prho2,
@@ -309,7 +308,6 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
   for(int d = 0; d < D; ++d)
     v12a[d] = VH[d][a];
   const double Prho2_a = prho2[a];
-  const bool part_a = pi_part(pp, P.f[F_ALPHA], a, rho_a, c_a);
   double acc[3] = {0, 0, 0};
   double vsig = 0.0;
   const int cnt = Ls.cnt[a];
@@ -339,22 +337,17 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
       const PairR r = pair_r(dist2);
       const double f = pair_g<D, K>(r, ph, pp);
       // mu and Pi are zero unless the pair approaches (viscosity.h:81-93)
-      const double cn_b = CS[b], Prho2_b = prho2[b];
-      double Pi, appr;
+      const double Prho2_b = prho2[b];
+      double Pi = pi_apart(Prho2_a, Prho2_b, dotp);
+      double appr = nan64(dotp) ? dotp : 0.0;  // (drops out of the maximum)
       if(dotp < 0.0) {
         Pi = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + RHO[b]),
-          .5 * (c_a + cn_b), ph.h, dotp, dist2);
+          .5 * (c_a + CS[b]), ph.h, dotp, dist2);
         if(VSIG)
           appr = approach<D>(v12_ab, pos_ab, r);
       }
-      else {
-        // (a density that is a NaN shows in P / rho^2)
-        Pi = pi_apart(part_a, pi_part(pp, P.f[F_ALPHA], b,
-          nan64(Prho2_b) ? RHO[b] : 0.0, cn_b), dotp);
-        appr = nan64(dotp) ? dotp : 0.0;  // the pair drops out of the maximum
-      }
       if(VSIG && nonzero(dist2)) {
-        const double c_b = b >= a ? cn_b : cs_old[b];
+        const double c_b = b >= a ? CS[b] : cs_old[b];
         const double cand = (c_a < c_b ? c_b : c_a) - appr;
         vsig = vsig < cand ? cand : vsig;
       }
@@ -389,7 +382,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_accel(Particles P,
 template<int D, int K, bool KEPT>
 __device__ __forceinline__ double2 pair_terms(const Particles & P, const PhysParams & pp,
   PairH<D, K> & ph, const double2 * pr, int j, int a, int b, const double * pos_ab,
-  const double * v12a, double h_a, double rho_a, double c_a) {
+  const double * v12a, double h_a, double rho_a, double c_a, const double * prho2) {
   if(KEPT)
     return pr[(size_t)j * 32];
   double dist2 = 0.0, dotp = 0.0;
@@ -398,13 +391,12 @@ __device__ __forceinline__ double2 pair_terms(const Particles & P, const PhysPar
     dotp += (v12a[d] - P.f[F_VHX + d][b]) * pos_ab[d];
   }
   ph.template set<false, true>(h_a, P.f[F_H][b], pp);
-  const double rho_b = P.f[F_RHO][b], c_b = P.f[F_CS][b];
-  const double Pi = dotp < 0.0
-    ? pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + rho_b), .5 * (c_a + c_b), ph.h,
-        dotp, dist2)
-    : pi_apart(pi_part(pp, P.f[F_ALPHA], a, rho_a, c_a),
-        pi_part(pp, P.f[F_ALPHA], b, rho_b, c_b), dotp);
-  return make_double2(pair_g<D, K>(pair_r(dist2), ph, pp), Pi);
+  double2 t = make_double2(pair_g<D, K>(pair_r(dist2), ph, pp),
+    pi_apart(prho2[a], prho2[b], dotp));
+  if(dotp < 0.0)
+    t.y = pair_pi<D>(pp, P.f[F_ALPHA], a, b, .5 * (rho_a + P.f[F_RHO][b]),
+      .5 * (c_a + P.f[F_CS][b]), ph.h, dotp, dist2);
+  return t;
 }
 
 // compute_dudt (default_physics.h:421-487).  KEPT: the pair terms of the
@@ -444,7 +436,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_dudt(Particles P,
       for(int d = 0; d < D; ++d)
         pos_ab[d] = pa[d] - P.f[F_X + d][b];
       const double2 t = pair_terms<D, K, KEPT>(P, pp, ph, pr, j0 + u, a, b, pos_ab, v12a,
-        h_a, rho_a, c_a);
+        h_a, rho_a, c_a, prho2);
       double vdw = 0;
       for(int d = 0; d < D; ++d)
         vdw += (va[d] - P.f[F_VX + d][b]) * (pos_ab[d] * t.x);
@@ -489,7 +481,7 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_dedt(Particles P,
       for(int d = 0; d < D; ++d)
         pos_ab[d] = pa[d] - P.f[F_X + d][b];
       const double2 t = pair_terms<D, K, KEPT>(P, pp, ph, pr, j0 + u, a, b, pos_ab, v12a,
-        h_a, rho_a, c_a);
+        h_a, rho_a, c_a, prho2);
       double vad = 0, vbd = 0;
       for(int d = 0; d < D; ++d) {
         const double DiW = pos_ab[d] * t.x;
@@ -562,15 +554,16 @@ cudaError_t launch_density_fp64(const Launch & L, const Particles & P,
   return cudaGetLastError();
 }
 
-cudaError_t launch_prho2(const Launch & L, const Particles & P, double * prho2) {
-  chain(L, k_prho2, (P.n + 255) / 256, 256, 0, P, prho2);
+cudaError_t launch_prho2(const Launch & L, const Particles & P, const PhysParams & pp,
+  double * prho2) {
+  chain(L, k_prho2, (P.n + 255) / 256, 256, 0, P, pp, prho2);
   *L.counter += 1;
   return cudaGetLastError();
 }
 
 cudaError_t launch_alpha_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const DevTime * t) {
-  DISPATCH_DK(k_alpha_cullen, , P, pp, Ls, t);
+  const PhysParams & pp, const Lists & Ls, const DevTime * t, double * prho2) {
+  DISPATCH_DK(k_alpha_cullen, , P, pp, Ls, t, prho2);
   return cudaGetLastError();
 }
 

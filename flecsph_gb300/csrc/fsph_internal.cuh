@@ -414,17 +414,18 @@ cudaError_t launch_periodic(const Launch & L, Particles & P, Particles & Palt,
   const char ** why, unsigned skip);
 
 // ---- fsph_fp64.cu ----
-// prho2: P / rho^2 per particle, written by the density pass (or
-// launch_prho2).  pair: {grad W factor, Pi} of every list slot, written by the
+// prho2: P / rho^2 per particle, written by the density pass, the alpha
+// pass (or launch_prho2).  pair: {grad W factor, Pi} of every list slot, written by the
 // acceleration pass (null: not kept) and read by the energy passes (null:
 // evaluated there).  cs_old (acceleration): the sound speed before the density
 // pass if the signal speed is to ride along, else null.
 cudaError_t launch_density_fp64(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, double * cs_new, double * prho2,
   DevStatus * st, const DevTime * t);
-cudaError_t launch_prho2(const Launch & L, const Particles & P, double * prho2);
+cudaError_t launch_prho2(const Launch & L, const Particles & P, const PhysParams & pp,
+  double * prho2);
 cudaError_t launch_alpha_cullen(const Launch & L, const Particles & P,
-  const PhysParams & pp, const Lists & Ls, const DevTime * t);
+  const PhysParams & pp, const Lists & Ls, const DevTime * t, double * prho2);
 cudaError_t launch_vsig_fp64(const Launch & L, const Particles & P,
   const PhysParams & pp, const Lists & Ls, const double * cs_new);
 cudaError_t launch_repulsion(const Launch & L, const Particles & P,
