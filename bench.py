@@ -55,13 +55,13 @@ sys.path.insert(0, ROOT)
 HBM_PEAK = 6782.8  # GB/s, MEASURED_PEAKS.json hbm_gbs
 # ncu dram__bytes_read.sum + dram__bytes_write.sum per particle of the
 # dominant kernel of a phase, from 96^3 Sedov captures (884,736 particles;
-# lists and records well above L2): the walk (459.4 MB,
+# lists and records well above L2): the walk (474.9 MB,
 # profiles/k_neighbors_uni_sedov3d_96.md); the float-float
-# density and acceleration passes and the de/dt pass of the warm-up
-# iteration (567.6, 569.2 and 597.8 MB,
+# density and acceleration passes and the de/dt pass of a warm-up
+# iteration (567.9, 611.3 and 597.6 MB,
 # profiles/k_density_ff_accel_ff_dedt_ahyd_sedov3d_96.md)
-MEASURED_TRAFFIC_PER_PARTICLE = {"neighbors": 519.3, "density": 641.6, "accel": 643.3,
-                                 "energy": 675.7}
+MEASURED_TRAFFIC_PER_PARTICLE = {"neighbors": 536.7, "density": 641.9, "accel": 690.9,
+                                 "energy": 675.4}
 
 
 def read_work_header(path=os.path.join(ROOT, "include", "fsph_work.h")):

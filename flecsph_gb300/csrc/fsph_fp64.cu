@@ -6,8 +6,9 @@
 // evaluated in the reference's operand order: with lists in the reference's
 // order the results are those of the reference on the CPU, but for the last
 // bits in which libm's pow and cbrt differ from CUDA's, in which quotients and
-// roots from a reciprocal may (fsph_pair64.cuh: none has been seen to), and in
-// the fused signal speed pairs whose v . x and v . (x / r) round to different
+// roots from a reciprocal may (fsph_pair64.cuh: none has been seen to), in which
+// the order of three products in some kernels' gradients shows (there too), and
+// in the fused signal speed pairs whose v . x and v . (x / r) round to different
 // signs.
 #include <cuda_runtime.h>
 

@@ -18,7 +18,11 @@
 //     which a residual could underflow take the plain operators.
 //
 // Operand order otherwise follows kernels.h and viscosity.h of the reference,
-// as fsph_sphmath.cuh does.
+// as fsph_sphmath.cuh does, but for one thing: with the spline, Gaussian (not
+// super-Gaussian) and sinc kernels the reference multiplies x_ab in before it
+// divides by r, for every axis; here, as its other kernels do, f = (dW/dr) / r
+// is formed first and x_ab f after, three roundings either way (outputs differ
+// by some 4e-16).
 #pragma once
 
 #include "fsph_sphmath.cuh"

@@ -37,7 +37,8 @@ def _problem(dim, kernel, cullen):
 @pytest.mark.parametrize("dim,kernel", [(2, KERNEL_WENDLAND_C6), (3, KERNEL_WENDLAND_C6),
                                         (3, KERNEL_CUBIC_SPLINE)])
 @pytest.mark.parametrize("field,value", [("cs", np.nan), ("cs", np.inf), ("vhx", np.nan),
-                                         ("vhy", np.inf), ("alpha", np.nan)])
+                                         ("vhy", np.inf), ("alpha", np.nan),
+                                         ("alpha", np.inf), ("rho", np.nan)])
 def test_reaches_every_listing_particle(field, value, dim, kernel, cullen):
     from flecsph_gb300.sph import BodySystem
     if field == "alpha" and not cullen:
