@@ -1,6 +1,8 @@
 """Device memory of plain-FP64 contexts: what they hold beside the fields and
 lists (the pair terms of the acceleration pass) stays within 1/32 of the
 device's memory for all contexts together, and is given back."""
+import gc
+
 import pytest
 
 from flecsph_gb300.abi import PRECISION_FP64, Params
@@ -25,6 +27,7 @@ def _taken(p, n):
 
 
 def test_bounded_over_contexts_and_given_back():
+    gc.collect()  # contexts that other tests left
     total = _free()[1]
     limit = total // 32
     p = Params.defaults(dimension=3, precision_mode=PRECISION_FP64, max_neighbors=1024)
